@@ -180,6 +180,96 @@ def run(state):
     return {"o": o, "lse": lse, "dq": dq, "dk": dk, "dv": dv}
 
 
+def _f64(t):
+    return t.detach().to(torch.float64)
+
+
+def _rotate(x, cos, sin, sign=1.0):
+    """Rotary embedding (half split) of x [T, heads, 128] by sign times the angles."""
+    c, s = cos.unsqueeze(1), sign * sin.unsqueeze(1)
+    a, b = x[..., :64], x[..., 64:]
+    return torch.cat([a * c - b * s, b * c + a * s], dim=-1)
+
+
+def _attention(q, k, v, causal, do=None):
+    """Softmax attention of q [Tq, H, 128] on k, v [Tk, Hkv, 128], a head and some rows at a time; with ``do`` also the
+    gradients of q, k and v."""
+    Tq, H, hd = q.shape
+    G, rows = H // k.shape[1], max(128, (1 << 27) // k.shape[0])
+    o, lse = torch.empty_like(q), torch.empty(H, Tq, dtype=q.dtype, device=q.device)
+    dq, dk, dv = (torch.zeros_like(t) for t in (q, k, v))
+    for h in range(H):
+        kh, vh = k[:, h // G], v[:, h // G]
+        for r in range(0, Tq, rows):
+            sl = slice(r, min(Tq, r + rows))
+            n = sl.stop if causal else k.shape[0]
+            s = (q[sl, h] @ kh[:n].t()) / math.sqrt(hd)
+            if causal:
+                s[:, r:] += torch.full((n - r, n - r), float("-inf"), dtype=s.dtype, device=s.device).triu_(1)
+            lse[h, sl] = torch.logsumexp(s, 1)
+            p = s.sub_(lse[h, sl].unsqueeze(1)).exp_()
+            o[sl, h] = p @ vh[:n]
+            if do is not None:
+                dv[:n, h // G] += p.t() @ do[sl, h]
+                delta = (do[sl, h] * o[sl, h]).sum(1, keepdim=True)
+                ds = (do[sl, h] @ vh[:n].t()).sub_(delta).mul_(p).mul_(1.0 / math.sqrt(hd))
+                dq[sl, h] = ds @ kh[:n]
+                dk[:n, h // G] += ds.t() @ q[sl, h]
+    return o, lse, dq, dk, dv
+
+
+def _rms(x, w, eps):
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, in 64 bits.  A step has no such value here: after the optimizer's first
+    update of +-lr the sign of a gradient that is nearly zero decides, and its products are those of the other kinds."""
+    kind = case["kind"]
+    if kind == "step":
+        return None
+    state = prepare(case, seed)
+    if kind == "logits":
+        cfg, m = _config(case), state["model"]
+        if case["tokens"] > 8192:
+            return None
+        w = {k: _f64(t) for k, t in m.export_hf_state_dict().items()}
+        T, hd = case["tokens"], 128
+        ang = torch.arange(T, dtype=torch.float64, device=state["ids"].device).unsqueeze(1) / cfg.rope_theta ** (
+            torch.arange(0, hd, 2, dtype=torch.float64, device=state["ids"].device) / hd)
+        cos, sin = ang.cos(), ang.sin()
+        x = w["model.embed_tokens.weight"][state["ids"].reshape(-1)]
+        for i in range(cfg.num_hidden_layers):
+            p = "model.layers.%d." % i
+            h = _rms(x, w[p + "input_layernorm.weight"], cfg.rms_norm_eps)
+            q, k, v = ((h @ w[p + "self_attn.%s_proj.weight" % n].t()).view(T, -1, hd) for n in "qkv")
+            o = _attention(_rotate(q, cos, sin), _rotate(k, cos, sin), v, True)[0]
+            x = x + o.reshape(T, -1) @ w[p + "self_attn.o_proj.weight"].t()
+            h = _rms(x, w[p + "post_attention_layernorm.weight"], cfg.rms_norm_eps)
+            g, u = (h @ w[p + "mlp.%s_proj.weight" % n].t() for n in ("gate", "up"))
+            x = x + (g * torch.sigmoid(g) * u) @ w[p + "mlp.down_proj.weight"].t()
+        return (_rms(x, w["model.norm.weight"], cfg.rms_norm_eps) @ w["lm_head.weight"].t()).unsqueeze(0)
+    if kind == "mlp":
+        x, dy = _f64(state["x"]), _f64(state["dy"])
+        w1, w2 = (_f64(p) for p in state["mlp"].parameters())
+        g, u = (x @ w1.t()).chunk(2, dim=1)
+        sig = torch.sigmoid(g)
+        h, dh = g * sig * u, dy @ w2
+        dgu = torch.cat([dh * u * sig * (1 + g * (1 - sig)), dh * g * sig], dim=1)
+        return {"y": h @ w2.t(), "dx": dgu @ w1, "dw": [dgu.t() @ x, dy.t() @ h]}
+    if kind == "attention":
+        hq, hkv = state["hq"], state["hkv"]
+        T = case["tokens"]
+        q, k, v = _f64(state["qkv"]).view(T, -1, 128).split([hq, hkv, hkv], dim=1)
+        o, _, dq, dk, dv = _attention(q, k, v, True, _f64(state["do"]).view(T, hq, 128))
+        cos, sin = _f64(state["cos"]), _f64(state["sin"])
+        # the gradient goes back through the rotation that the projection's epilogue applied
+        d = torch.cat([_rotate(dq, cos, sin, -1.0), _rotate(dk, cos, sin, -1.0), dv], dim=1)
+        return {"o": o.reshape(T, -1), "dqkv": d.reshape(T, -1)}
+    o, lse, dq, dk, dv = _attention(*(_f64(state[n]) for n in ("q", "k", "v")), False, _f64(state["do"]))
+    return {"o": o, "lse": lse, "dq": dq, "dk": dk, "dv": dv}
+
+
 def work(case):
     """Products at two operations per multiply-add, causal halves not counted; a step's bytes are the optimizer's (fp32
     master and moments read and written, gradient and weight in bf16) and the activations' are left out: a step could keep
