@@ -21,6 +21,8 @@
 // Splitting dQ from dK/dV recomputes S and dP once more but needs no atomics and is deterministic.
 // Gradients are written with TMA stores through row-pitched tensor maps, so dq/dk/dv may be slices
 // of one packed [T, hq + 2 hkv, 128] gradient tensor.
+#include <limits.h>
+
 #include "ody_kernels.h"
 #include "sm100.cuh"
 
@@ -129,6 +131,12 @@ constexpr int KV_SMEM_TOTAL = KV_SMEM_TILES + 256 + 1024;
 // TMEM columns: S^T 0..127 (P^T, bf16, overwrites 0..63), dP^T 128..255 (dS^T overwrites 128..191), dV 256, dK 384
 constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
 
+// CTA order of the dK/dV grid.  Causal: the KV tiles of all heads that see the most query blocks (the first ones) come first,
+// so that no long CTA starts when the others are nearly done; without a mask all CTAs cost the same and consecutive ones
+// share their head's Q and dO in the L2.
+__device__ __forceinline__ int kv_tile_of(int cta, int tiles, int Hkv, int causal) { return causal ? cta / Hkv : cta % tiles; }
+__device__ __forceinline__ int kv_head_of(int cta, int tiles, int Hkv, int causal) { return causal ? cta % Hkv : cta / tiles; }
+
 // Optional redirection of an output: rows [d * rows, (d + 1) * rows) go to tensor map m[d] instead of the
 // kernel's own output map (another rank's buffer: the Ulysses head->sequence exchange of the gradient).
 struct SplitMaps {
@@ -158,7 +166,8 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x, kvh = blockIdx.y;
+  const int num_kv_tiles = (Tk + BIG - 1) / BIG;
+  const int kt = kv_tile_of(blockIdx.x, num_kv_tiles, Hkv, causal), kvh = kv_head_of(blockIdx.x, num_kv_tiles, Hkv, causal);
   const int kv0 = kt * BIG;
   const int G = H / Hkv;
   const int nq = (Tq + BLK - 1) / BLK;
@@ -232,7 +241,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const uint64_t q_mn0 = make_smem_desc(smem_u32(sQs), BLK_HALF, 1024), d_mn0 = make_smem_desc(smem_u32(sDs), BLK_HALF, 1024);
       const uint64_t ones_d = make_smem_desc_noswizzle(smem_u32(sOnes), 128, 256);
       const uint64_t stat_d0 = make_smem_desc_noswizzle(smem_u32(sStat), 128, 256);
-      const bool trace = dbg != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
+      const bool trace = dbg != nullptr && blockIdx.x == 0;
       // S^T(it) = K Q^T - lse / scale (per query column): waits for the Q block
       auto issue_s = [&](int it) -> bool {
         const int stage = it % STAGES;
@@ -318,7 +327,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int it = 0; it < total; ++it) {
       const uint32_t par = it & 1;
       const int qrow0 = (i0 + it % per_head) * BLK + hf * 64;
-      const bool strace = dbg != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 128 && it < 48;
+      const bool strace = dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 128 && it < 48;
       // ---- part 1: S^T -> P^T
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 2] = clock64();                             // S^T(it) complete
@@ -506,7 +515,8 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x, kvh = blockIdx.y;
+  const int num_kv_tiles = (Tk + BIG - 1) / BIG;
+  const int kt = kv_tile_of(blockIdx.x, num_kv_tiles, Hkv, causal), kvh = kv_head_of(blockIdx.x, num_kv_tiles, Hkv, causal);
   const int kv0 = kt * BIG;
   const int G = H / Hkv;
   const int nq = (Tq + BLK - 1) / BLK;
@@ -928,8 +938,9 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_q_tiles = (Tq + BIG - 1) / BIG;
-  const int qt = causal ? (num_q_tiles - 1 - (int)blockIdx.x) : (int)blockIdx.x;
-  const int head = blockIdx.y, kvh = head / (H / Hkv);
+  // CTA order as in the forward: causal, the tiles of all heads that attend to the most blocks first
+  const int qt = causal ? (num_q_tiles - 1 - (int)blockIdx.x / H) : (int)blockIdx.x % num_q_tiles;
+  const int head = causal ? (int)blockIdx.x % H : (int)blockIdx.x / num_q_tiles, kvh = head / (H / Hkv);
   const int q0 = qt * BIG;
   const int nk = (Tk + BLK - 1) / BLK;
   const int total = causal ? min(nk, (q0 + BIG) / BLK) : nk;
@@ -985,7 +996,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
       tc_fence_after();
       const uint64_t k_k0 = make_smem_desc(smem_u32(sKs), 16, 1024), v_k0 = make_smem_desc(smem_u32(sVs), 16, 1024);
       const uint64_t k_mn0 = make_smem_desc(smem_u32(sKs), BLK_HALF, 1024);
-      const bool trace = dbg != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
+      const bool trace = dbg != nullptr && blockIdx.x == 0;
       // S(it) = Q K^T, Q from TMEM
       auto issue_s = [&](int it) -> bool {
         const int stage = it % K_STAGES;
@@ -1075,7 +1086,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
     for (int it = 0; it < total; ++it) {
       const uint32_t par = it & 1;
       const int kvb0 = it * BLK + hf * 64;
-      const bool strace = dbg != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 128 && it < 48;
+      const bool strace = dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 128 && it < 48;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 4] = clock64();                             // S(it) complete
       uint32_t sv[64];
@@ -1269,7 +1280,9 @@ extern "C" int ody_flash_bwd_ex(const void* dO, const void* q, const void* k, co
   if ((r = make_tmap_3d_bf16(&tDQ, dq, HD, H, Tq, HD * 2, dq_row * 2, 64, 1, BIG))) return 790000 + r;
   if ((r = make_tmap_3d_bf16(&tDK, dk, HD, Hkv, Tk, HD * 2, dk_row * 2, 64, 1, BIG))) return 790000 + r;
   if ((r = make_tmap_3d_bf16(&tDV, dv, HD, Hkv, Tk, HD * 2, dv_row * 2, 64, 1, BIG))) return 790000 + r;
-  dim3 gkv((Tk + BIG - 1) / BIG, Hkv);
+  const int64_t ctas_kv = (int64_t)((Tk + BIG - 1) / BIG) * Hkv, ctas_q = (int64_t)((Tq + BIG - 1) / BIG) * H;
+  if (ctas_kv > INT_MAX || ctas_q > INT_MAX) return (int)cudaErrorInvalidValue;
+  const dim3 gkv((unsigned)ctas_kv), gq((unsigned)ctas_q);
   if (g_bwd_variant != 1) {
     float* dq_acc = (float*)(stat_tiles + (int64_t)H * (Tpad / BLK) * STAT_BYTES);
     cudaError_t e = cudaMemsetAsync(dq_acc, 0, (size_t)H * Tpad * HD * sizeof(float), st);
@@ -1286,7 +1299,6 @@ extern "C" int ody_flash_bwd_ex(const void* dO, const void* q, const void* k, co
   }
   flash_bwd_dkdv_kernel<<<gkv, NUM_THREADS, KV_SMEM_TOTAL, st>>>(tQ, tDO, tK, tV, tDK, tDV, stat_tiles, Tq, Tk,
                                                                  Tpad, H, Hkv, causal, scale, err, g_bwd_trace, sk, sv);
-  dim3 gq((Tq + BIG - 1) / BIG, H);
   flash_bwd_dq_kernel<<<gq, NUM_THREADS, Q_SMEM_TOTAL, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)dO, q_row, do_row, tK, tV, tDQ, lse2_pad, delta_pad, Tq, Tk, Tpad, H,
                                                              Hkv, causal, scale, err, sq, g_bwd_trace ? g_bwd_trace + 48 * 8 : nullptr);
   return (int)cudaGetLastError();

@@ -22,6 +22,8 @@
 //
 // q [Tq, H, 128], k/v [Tk, Hkv, 128] with arbitrary row pitch; out [Tq, H, 128] bf16; lse [H, Tq] fp32
 // (natural log).  causal requires Tq == Tk (row i sees keys 0..i).
+#include <limits.h>
+
 #include "ody_kernels.h"
 #include "sm100.cuh"
 #include "peer_comm.cuh"
@@ -103,8 +105,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_pairs = (Tq + CTA_ROWS - 1) / CTA_ROWS;
-  const int pair = causal ? (num_pairs - 1 - (int)blockIdx.x) : (int)blockIdx.x;    // heavy tiles first
-  const int head = blockIdx.y;
+  // Causal: the CTAs of all heads that attend to the most blocks come first, so that no long CTA starts when the others
+  // are nearly done (head by head, the last head's longest tile started last).  Without a mask all CTAs cost the same and
+  // consecutive ones share their head's K and V in the L2.
+  const int pair = causal ? (num_pairs - 1 - (int)blockIdx.x / H) : (int)blockIdx.x % num_pairs;
+  const int head = causal ? (int)blockIdx.x % H : (int)blockIdx.x / num_pairs;
   const int kv_head = head / (H / Hkv);
   const int q0 = pair * CTA_ROWS;
   const bool has_b = q0 + BM < Tq;
@@ -149,7 +154,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // ------------------------------------------------------------------ comm warps (PUSH only)
     if constexpr (PUSH) {
       reg_dec<REGS_COMM>();
-      const int cta = blockIdx.y * gridDim.x + blockIdx.x;
+      const int cta = blockIdx.x;
       if (cta < push_ctas) gc::comm_warps_main(pp, cta, push_ctas, 12 * 32, abort_flag, err);
     }
   } else if (warp < 4) {
@@ -261,7 +266,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const int nt = t == 0 ? nA : nB;
             if (j >= nt) continue;
             if (!mbar_wait(&bars->p_full[t], j & 1, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-            ODY_FWD_STAMP(blockIdx.x == 0 && blockIdx.y == 0, j, 10 + t * 2);
+            ODY_FWD_STAMP(blockIdx.x == 0, j, 10 + t * 2);
             if (!have_v) {
               if (!mbar_wait(&bars->v_full[s], ph, abort_flag, err, ODY_ERR_TIMEOUT_FULL)) { ok = false; break; }
               have_v = true;
@@ -274,7 +279,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 have_k1 = true;
               }
               issue_qk(t, j + 1);      // its commit on s_full[t] also covers the P V just issued
-              ODY_FWD_STAMP(blockIdx.x == 0 && blockIdx.y == 0, j, 11 + t * 2);
+              ODY_FWD_STAMP(blockIdx.x == 0, j, 11 + t * 2);
             } else {
               if (leader) umma_commit(&bars->o_done[t]);
             }
@@ -312,7 +317,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < nt; ++j) {
-      const bool tr = blockIdx.x == 0 && blockIdx.y == 0 && (threadIdx.x == 128 || threadIdx.x == 256);
+      const bool tr = blockIdx.x == 0 && (threadIdx.x == 128 || threadIdx.x == 256);
       ODY_FWD_STAMP(tr, j, t * 5 + 0);
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[t], j & 1, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (!ok) break;
@@ -542,12 +547,13 @@ extern "C" int ody_flash_fwd_ex(const void* q, const void* k, const void* v, voi
     }
     sm.rows = split_rows;
   }
-  dim3 grid((Tq + CTA_ROWS - 1) / CTA_ROWS, H);
+  const int64_t ctas = (int64_t)((Tq + CTA_ROWS - 1) / CTA_ROWS) * H;
+  if (ctas > INT_MAX) return (int)cudaErrorInvalidValue;
+  const dim3 grid((unsigned)ctas);
   gc::GatherParams pp;
   memset(&pp, 0, sizeof(pp));
   if (push != nullptr) {
     if ((r = gc::fill_gather(pp, push))) return r;
-    const int ctas = (int)(grid.x * grid.y);
     if (push->n_cta <= 0 || push->n_cta > ctas) return (int)cudaErrorInvalidValue;
     if (ks32)
       flash_fwd_kernel<true, true><<<grid, NUM_THREADS_PUSH, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, push->n_cta, sm);
