@@ -21,10 +21,9 @@
 // Splitting dQ from dK/dV recomputes S and dP once more but needs no atomics and is deterministic.
 // Gradients are written with TMA stores through row-pitched tensor maps, so dq/dk/dv may be slices
 // of one packed [T, hq + 2 hkv, 128] gradient tensor.
-#include <limits.h>
-
 #include "ody_kernels.h"
 #include "sm100.cuh"
+#include "attn_split.cuh"
 
 // Of every ODY_BWD_POLY_DEN column pairs, the first ODY_BWD_POLY_NUM take their exponentials on the FMA pipe
 // (exp2_poly2) instead of the special-function unit.  Measured on B200: any mix is a few percent slower than
@@ -137,6 +136,48 @@ constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
 __device__ __forceinline__ int kv_tile_of(int cta, int tiles, int Hkv, int causal) { return causal ? cta / Hkv : cta % tiles; }
 __device__ __forceinline__ int kv_head_of(int cta, int tiles, int Hkv, int causal) { return causal ? cta % Hkv : cta / tiles; }
 
+// 64 accumulator columns of this thread's TMEM lane, times mult, to a row of fp32 partials
+__device__ __forceinline__ void store_partial_row(uint32_t taddr, float mult, float* dst) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t o[16];
+    tmem_ld_32x16(taddr + c * 16, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      *reinterpret_cast<float4*>(dst + c * 16 + t * 4) =
+          make_float4(__uint_as_float(o[4 * t]) * mult, __uint_as_float(o[4 * t + 1]) * mult, __uint_as_float(o[4 * t + 2]) * mult,
+                      __uint_as_float(o[4 * t + 3]) * mult);
+  }
+}
+
+// Sum of the parts of split tiles, in order, rounded once.  One block per (tile, head, 16-row slice); part layout
+// [tile][max_parts][heads][n_out][128][128] fp32, out[i] [T, heads, 128] bf16 with row pitch ld[i].  Bound by memory.
+struct PartDests { __nv_bfloat16* out[2]; int64_t ld[2]; };
+template <int N_OUT>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ part, const PartDests d, int T, int heads,
+                                                        const SplitUnits units, const SplitPlan plan) {
+  const int tile = blockIdx.x, head = blockIdx.y;
+  const int n_parts = plan.parts(units(tile));
+  const int r = blockIdx.z * 16 + (threadIdx.x >> 4), c = (threadIdx.x & 15) * 8;
+  const int64_t row = (int64_t)tile * BIG + r;
+  if (n_parts == 1 || row >= T) return;
+#pragma unroll
+  for (int w = 0; w < N_OUT; ++w) {
+    const float* p = part + ((((int64_t)tile * plan.max_parts * heads + head) * N_OUT + w) * BIG + r) * HD + c;
+    const int64_t step = (int64_t)heads * N_OUT * BIG * HD;
+    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int z = 0; z < n_parts; ++z) {
+      const float4 x = *reinterpret_cast<const float4*>(p + z * step), y = *reinterpret_cast<const float4*>(p + z * step + 4);
+      a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+      a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+    }
+    *reinterpret_cast<uint4*>(d.out[w] + row * d.ld[w] + head * HD + c) =
+        make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
+  }
+}
+
 // Optional redirection of an output: rows [d * rows, (d + 1) * rows) go to tensor map m[d] instead of the
 // kernel's own output map (another rank's buffer: the Ulysses head->sequence exchange of the gradient).
 struct SplitMaps {
@@ -150,7 +191,8 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                       const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV,
                       const uint8_t* __restrict__ stat_tiles, int Tq, int Tk, int Tq_pad,
                       int H, int Hkv, int causal, float scale, int* __restrict__ err, long long* __restrict__ dbg,
-                      const __grid_constant__ SplitMaps dk_split, const __grid_constant__ SplitMaps dv_split) {
+                      const __grid_constant__ SplitMaps dk_split, const __grid_constant__ SplitMaps dv_split,
+                      const SplitPlan plan, float* __restrict__ part) {
 #ifndef ODY_ATTN_TRACE
   dbg = nullptr;   // the clock-stamp timeline is a development aid: compiled out of the product kernels
 #endif
@@ -167,13 +209,18 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_kv_tiles = (Tk + BIG - 1) / BIG;
-  const int kt = kv_tile_of(blockIdx.x, num_kv_tiles, Hkv, causal), kvh = kv_head_of(blockIdx.x, num_kv_tiles, Hkv, causal);
+  const int tile = blockIdx.x / plan.max_parts, z = blockIdx.x % plan.max_parts;
+  const int kt = kv_tile_of(tile, num_kv_tiles, Hkv, causal), kvh = kv_head_of(tile, num_kv_tiles, Hkv, causal);
   const int kv0 = kt * BIG;
   const int G = H / Hkv;
   const int nq = (Tq + BLK - 1) / BLK;
   const int i0 = causal ? min(nq, kv0 / BLK) : 0;          // first query block that sees this KV tile
   const int per_head = nq - i0;
-  const int total = per_head * G;
+  // this CTA's share [u0, u0 + total) of the tile's (head, query block) list
+  const int n_parts = plan.parts(per_head * G);
+  if (z >= n_parts) return;
+  const int u0 = plan.begin(z);
+  const int total = plan.end(z, per_head * G) - u0;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->kv_full, 1);
@@ -211,8 +258,8 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int it = 0; it < total; ++it) {
         const int stage = it % STAGES;
         const uint32_t phase = (it / STAGES) & 1;
-        const int head = kvh * G + it / per_head;
-        const int qrow = (i0 + it % per_head) * BLK;
+        const int head = kvh * G + (u0 + it) / per_head;
+        const int qrow = (i0 + (u0 + it) % per_head) * BLK;
         // the Q ring is released by dK, the dO ring (earlier) by dV
         if (!mbar_wait(&bars->q_empty[stage], phase ^ 1, abort_flag, err, ODY_ERR_TIMEOUT_EMPTY)) break;
         uint8_t* sQ = sQs + stage * BLK_BYTES;
@@ -326,7 +373,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     bool ok = true;
     for (int it = 0; it < total; ++it) {
       const uint32_t par = it & 1;
-      const int qrow0 = (i0 + it % per_head) * BLK + hf * 64;
+      const int qrow0 = (i0 + (u0 + it) % per_head) * BLK + hf * 64;
       const bool strace = dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 128 && it < 48;
       // ---- part 1: S^T -> P^T
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
@@ -409,6 +456,16 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_done, 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
     if (ok) {
       tc_fence_after();
+      if (n_parts > 1) {
+        // partial sums of a split tile: fp32 rows [dV | dK][128][128] of this part
+        float* prow = part + (((int64_t)(kt * plan.max_parts + z) * Hkv + kvh) * 2 * BIG + r) * HD + hf * 64;
+#pragma unroll 1
+        for (int which = 0; which < 2; ++which) {
+          const uint32_t col = (which == 0 ? COL_DV : COL_DK) + hf * 64;
+          const float mult = which == 0 ? 1.f : scale;
+          store_partial_row(tmem + col + lane_off, mult, prow + which * BIG * HD);
+        }
+      } else {
       // dV -> sV region, dK -> sK region (both dead now), bf16, swizzled for the TMA store; this warp converts
       // output columns [hf * 64, hf * 64 + 64), which is exactly one 64-column half of the staging tile
 #pragma unroll 1
@@ -436,10 +493,11 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       }
       fence_proxy_async_smem();
+      }
     }
     tc_fence_before();
     named_barrier(1, 256);
-    if (ok && warp == 4 && lane == 0 && !*abort_flag) {
+    if (ok && n_parts == 1 && warp == 4 && lane == 0 && !*abort_flag) {
       const int d = dk_split.rows > 0 ? kv0 / dk_split.rows : 0;
       const int row = dk_split.rows > 0 ? kv0 - d * dk_split.rows : kv0;
       const CUtensorMap* mV = dk_split.rows > 0 ? &dv_split.m[d] : &tmDV;
@@ -924,7 +982,8 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const __grid_constant__ CUtensorMap tmDQ, const float* __restrict__ lse2_pad,
                     const float* __restrict__ delta_pad, int Tq, int Tk, int Tq_pad, int H, int Hkv, int causal,
-                    float scale, int* __restrict__ err, const __grid_constant__ SplitMaps dq_split, long long* __restrict__ dbg) {
+                    float scale, int* __restrict__ err, const __grid_constant__ SplitMaps dq_split, const SplitPlan plan,
+                    float* __restrict__ part, long long* __restrict__ dbg) {
 #ifndef ODY_ATTN_TRACE
   dbg = nullptr;   // the clock-stamp timeline is a development aid: compiled out of the product kernels
 #endif
@@ -939,11 +998,17 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_q_tiles = (Tq + BIG - 1) / BIG;
   // CTA order as in the forward: causal, the tiles of all heads that attend to the most blocks first
-  const int qt = causal ? (num_q_tiles - 1 - (int)blockIdx.x / H) : (int)blockIdx.x % num_q_tiles;
-  const int head = causal ? (int)blockIdx.x % H : (int)blockIdx.x / num_q_tiles, kvh = head / (H / Hkv);
+  const int tile = blockIdx.x / plan.max_parts, z = blockIdx.x % plan.max_parts;
+  const int qt = causal ? (num_q_tiles - 1 - tile / H) : tile % num_q_tiles;
+  const int head = causal ? tile % H : tile / num_q_tiles, kvh = head / (H / Hkv);
   const int q0 = qt * BIG;
   const int nk = (Tk + BLK - 1) / BLK;
-  const int total = causal ? min(nk, (q0 + BIG) / BLK) : nk;
+  // this CTA's share [b0, b0 + total) of the KV blocks the tile sees
+  const int seen = causal ? min(nk, (q0 + BIG) / BLK) : nk;
+  const int n_parts = plan.parts(seen);
+  if (z >= n_parts) return;
+  const int b0 = plan.begin(z);
+  const int total = plan.end(z, seen) - b0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < K_STAGES; ++s) {
@@ -976,13 +1041,13 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
         if (!mbar_wait(&bars->k_empty[stage], phase ^ 1, abort_flag, err, ODY_ERR_TIMEOUT_EMPTY)) break;
         uint8_t* sK = sKs + stage * BLK_BYTES;
         mbar_expect_tx(&bars->k_full[stage], BLK_BYTES);
-        tma_load_3d(sK, &tmK, 0, kvh, it * BLK, &bars->k_full[stage]);
-        tma_load_3d(sK + BLK_HALF, &tmK, 64, kvh, it * BLK, &bars->k_full[stage]);
+        tma_load_3d(sK, &tmK, 0, kvh, (b0 + it) * BLK, &bars->k_full[stage]);
+        tma_load_3d(sK + BLK_HALF, &tmK, 64, kvh, (b0 + it) * BLK, &bars->k_full[stage]);
         if (!mbar_wait(&bars->v_empty[stage], phase ^ 1, abort_flag, err, ODY_ERR_TIMEOUT_EMPTY)) break;
         uint8_t* sV = sVs + stage * BLK_BYTES;
         mbar_expect_tx(&bars->v_full[stage], BLK_BYTES);
-        tma_load_3d(sV, &tmV, 0, kvh, it * BLK, &bars->v_full[stage]);
-        tma_load_3d(sV + BLK_HALF, &tmV, 64, kvh, it * BLK, &bars->v_full[stage]);
+        tma_load_3d(sV, &tmV, 0, kvh, (b0 + it) * BLK, &bars->v_full[stage]);
+        tma_load_3d(sV + BLK_HALF, &tmV, 64, kvh, (b0 + it) * BLK, &bars->v_full[stage]);
       }
     }
    } else if (warp == 1) {
@@ -1085,7 +1150,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
     bool ok = true;
     for (int it = 0; it < total; ++it) {
       const uint32_t par = it & 1;
-      const int kvb0 = it * BLK + hf * 64;
+      const int kvb0 = (b0 + it) * BLK + hf * 64;
       const bool strace = dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 128 && it < 48;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 4] = clock64();                             // S(it) complete
@@ -1145,7 +1210,11 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
       if (strace) dbg[it * 8 + 7] = clock64();                             // dS published
     }
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_done, 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
-    if (ok) {
+    if (ok && n_parts > 1) {
+      tc_fence_after();
+      store_partial_row(tmem + COL_DQ + hf * 64 + lane_off, scale,
+                        part + (((int64_t)(qt * plan.max_parts + z) * H + head) * BIG + r) * HD + hf * 64);
+    } else if (ok) {
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -1167,7 +1236,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
     }
     tc_fence_before();
     named_barrier(1, 256);
-    if (ok && warp == 4 && lane == 0 && !*abort_flag) {
+    if (ok && n_parts == 1 && warp == 4 && lane == 0 && !*abort_flag) {
       const int d = dq_split.rows > 0 ? q0 / dq_split.rows : 0;
       const int row = dq_split.rows > 0 ? q0 - d * dq_split.rows : q0;
       const CUtensorMap* mQ = dq_split.rows > 0 ? &dq_split.m[d] : &tmDQ;
@@ -1200,6 +1269,30 @@ extern "C" int ody_flash_bwd_set_variant(int v) {
   return 0;
 }
 
+// Plans of the two split-pair grids (attn_split.cuh).  Block and CTA times measured at 8192 tokens x 32 heads.
+static void bwd_plans(int Tq, int Tk, int H, int Hkv, int causal, ody::SplitUnits* ukv, ody::SplitPlan* pkv, ody::SplitUnits* uq,
+                      ody::SplitPlan* pq) {
+  using namespace ody;
+  using namespace ody::bwd;
+  const int nq = (Tq + BLK - 1) / BLK, nk = (Tk + BLK - 1) / BLK;
+  *ukv = SplitUnits{causal ? 1 : 0, nq, H / Hkv, 1};
+  *uq = SplitUnits{causal ? 2 : 0, nk, 1, 1};
+  *pkv = split_plan(*ukv, nk, Hkv, 1.3, 3.0, 2 * BIG * HD * 4);
+  *pq = split_plan(*uq, nq, H, 1.1, 3.0, BIG * HD * 4);
+}
+
+extern "C" int64_t ody_flash_bwd_split_bytes(int Tq, int Tk, int H, int Hkv, int causal) {
+  using namespace ody;
+  using namespace ody::bwd;
+  if (Tq <= 0 || Tk <= 0 || H <= 0 || Hkv <= 0 || H % Hkv || g_bwd_variant != 1) return 0;
+  SplitUnits ukv, uq;
+  SplitPlan pkv, pq;
+  bwd_plans(Tq, Tk, H, Hkv, causal, &ukv, &pkv, &uq, &pq);
+  const int64_t kv = pkv.max_parts > 1 ? (int64_t)((Tk + BIG - 1) / BIG) * Hkv * pkv.max_parts * 2 * BIG * HD * 4 : 0;
+  const int64_t dq = pq.max_parts > 1 ? (int64_t)((Tq + BIG - 1) / BIG) * H * pq.max_parts * BIG * HD * 4 : 0;
+  return kv > dq ? kv : dq;      // the two kernels run one after the other
+}
+
 extern "C" int64_t ody_flash_bwd_workspace_bytes(int Tq, int H) {
   const int64_t Tpad = ((int64_t)Tq + 127) / 128 * 128;
   // -delta and exp2-domain -lse (padded), the statistics tiles, and the fp32 dQ accumulator of the fused kernel
@@ -1224,6 +1317,18 @@ extern "C" int ody_flash_bwd_ex(const void* dO, const void* q, const void* k, co
                                 int64_t q_row, int64_t k_row, int64_t v_row, int64_t o_row, int64_t dq_row, int64_t dk_row,
                                 int64_t dv_row, int causal, float scale, void* const* dq_split, void* const* dk_split,
                                 void* const* dv_split, int n_split, int split_rows, int* err, cudaStream_t st) {
+  return ody_flash_bwd_parts(dO, q, k, v, o, lse, dq, dk, dv, workspace, Tq, Tk, H, Hkv, do_row, q_row, k_row, v_row, o_row, dq_row,
+                             dk_row, dv_row, causal, scale, dq_split, dk_split, dv_split, n_split, split_rows, nullptr, 0, err, st);
+}
+
+// With `parts` (16-byte aligned, at least ody_flash_bwd_split_bytes of these sizes) small grids split the streamed dimension
+// (attn_split.cuh); not together with n_split > 0.
+extern "C" int ody_flash_bwd_parts(const void* dO, const void* q, const void* k, const void* v, const void* o, const float* lse,
+                                   void* dq, void* dk, void* dv, void* workspace, int Tq, int Tk, int H, int Hkv, int64_t do_row,
+                                   int64_t q_row, int64_t k_row, int64_t v_row, int64_t o_row, int64_t dq_row, int64_t dk_row,
+                                   int64_t dv_row, int causal, float scale, void* const* dq_split, void* const* dk_split,
+                                   void* const* dv_split, int n_split, int split_rows, void* parts, int64_t parts_bytes, int* err,
+                                   cudaStream_t st) {
   using namespace ody;
   using namespace ody::bwd;
   SplitMaps sq, sk, sv;
@@ -1280,7 +1385,14 @@ extern "C" int ody_flash_bwd_ex(const void* dO, const void* q, const void* k, co
   if ((r = make_tmap_3d_bf16(&tDQ, dq, HD, H, Tq, HD * 2, dq_row * 2, 64, 1, BIG))) return 790000 + r;
   if ((r = make_tmap_3d_bf16(&tDK, dk, HD, Hkv, Tk, HD * 2, dk_row * 2, 64, 1, BIG))) return 790000 + r;
   if ((r = make_tmap_3d_bf16(&tDV, dv, HD, Hkv, Tk, HD * 2, dv_row * 2, 64, 1, BIG))) return 790000 + r;
-  const int64_t ctas_kv = (int64_t)((Tk + BIG - 1) / BIG) * Hkv, ctas_q = (int64_t)((Tq + BIG - 1) / BIG) * H;
+  SplitUnits ukv, uq;
+  SplitPlan pkv, pq;
+  bwd_plans(Tq, Tk, H, Hkv, causal, &ukv, &pkv, &uq, &pq);
+  if (parts == nullptr || ((uintptr_t)parts & 15) || n_split > 0 || g_bwd_variant != 1 ||
+      parts_bytes < ody_flash_bwd_split_bytes(Tq, Tk, H, Hkv, causal))
+    pkv = pq = SplitPlan();
+  const int kv_tiles = (Tk + BIG - 1) / BIG, q_tiles = (Tq + BIG - 1) / BIG;
+  const int64_t ctas_kv = (int64_t)kv_tiles * Hkv * pkv.max_parts, ctas_q = (int64_t)q_tiles * H * pq.max_parts;
   if (ctas_kv > INT_MAX || ctas_q > INT_MAX) return (int)cudaErrorInvalidValue;
   const dim3 gkv((unsigned)ctas_kv), gq((unsigned)ctas_q);
   if (g_bwd_variant != 1) {
@@ -1298,8 +1410,16 @@ extern "C" int ody_flash_bwd_ex(const void* dO, const void* q, const void* k, co
     return (int)cudaGetLastError();
   }
   flash_bwd_dkdv_kernel<<<gkv, NUM_THREADS, KV_SMEM_TOTAL, st>>>(tQ, tDO, tK, tV, tDK, tDV, stat_tiles, Tq, Tk,
-                                                                 Tpad, H, Hkv, causal, scale, err, g_bwd_trace, sk, sv);
+                                                                 Tpad, H, Hkv, causal, scale, err, g_bwd_trace, sk, sv, pkv, (float*)parts);
+  if (pkv.max_parts > 1) {
+    const PartDests d = {{(__nv_bfloat16*)dv, (__nv_bfloat16*)dk}, {dv_row, dk_row}};
+    sum_parts_kernel<2><<<dim3(kv_tiles, Hkv, BIG / 16), 256, 0, st>>>((const float*)parts, d, Tk, Hkv, ukv, pkv);
+  }
   flash_bwd_dq_kernel<<<gq, NUM_THREADS, Q_SMEM_TOTAL, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)dO, q_row, do_row, tK, tV, tDQ, lse2_pad, delta_pad, Tq, Tk, Tpad, H,
-                                                             Hkv, causal, scale, err, sq, g_bwd_trace ? g_bwd_trace + 48 * 8 : nullptr);
+                                                             Hkv, causal, scale, err, sq, pq, (float*)parts, g_bwd_trace ? g_bwd_trace + 48 * 8 : nullptr);
+  if (pq.max_parts > 1) {
+    const PartDests d = {{(__nv_bfloat16*)dq, nullptr}, {dq_row, 0}};
+    sum_parts_kernel<1><<<dim3(q_tiles, H, BIG / 16), 256, 0, st>>>((const float*)parts, d, Tq, H, uq, pq);
+  }
   return (int)cudaGetLastError();
 }

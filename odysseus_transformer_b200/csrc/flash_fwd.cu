@@ -22,11 +22,10 @@
 //
 // q [Tq, H, 128], k/v [Tk, Hkv, 128] with arbitrary row pitch; out [Tq, H, 128] bf16; lse [H, Tq] fp32
 // (natural log).  causal requires Tq == Tk (row i sees keys 0..i).
-#include <limits.h>
-
 #include "ody_kernels.h"
 #include "sm100.cuh"
 #include "peer_comm.cuh"
+#include "attn_split.cuh"
 
 // KS32: Q and K sit in shared memory as eight [128 rows x 32 B] slices (32-byte swizzle) instead of two
 // [128 rows x 128 B] halves (128-byte swizzle), so that each Q K^T instruction reads two contiguous 4 KB blocks.
@@ -94,7 +93,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                  float* __restrict__ lse, int Tq, int Tk, int H, int Hkv, int causal, float scale,
                  int* __restrict__ err, const __grid_constant__ gc::GatherParams pp,
-                 int push_ctas, const __grid_constant__ SplitMaps osplit) {
+                 int push_ctas, const __grid_constant__ SplitMaps osplit, const SplitPlan plan,
+                 float* __restrict__ part, float2* __restrict__ part_ml) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;                               // tile t at sQ + t * TILE_BYTES (reused as output staging)
@@ -108,15 +108,22 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // Causal: the CTAs of all heads that attend to the most blocks come first, so that no long CTA starts when the others
   // are nearly done (head by head, the last head's longest tile started last).  Without a mask all CTAs cost the same and
   // consecutive ones share their head's K and V in the L2.
-  const int pair = causal ? (num_pairs - 1 - (int)blockIdx.x / H) : (int)blockIdx.x % num_pairs;
-  const int head = causal ? (int)blockIdx.x % H : (int)blockIdx.x / num_pairs;
+  const int cta_tile = PUSH ? blockIdx.x : blockIdx.x / plan.max_parts, z = PUSH ? 0 : blockIdx.x % plan.max_parts;
+  const int pair = causal ? (num_pairs - 1 - cta_tile / H) : cta_tile % num_pairs;
+  const int head = causal ? cta_tile % H : cta_tile / num_pairs;
   const int kv_head = head / (H / Hkv);
   const int q0 = pair * CTA_ROWS;
   const bool has_b = q0 + BM < Tq;
   const int kv_blocks = (Tk + BN - 1) / BN;
   // blocks each tile attends to: causal tile A ends on its diagonal block q0 / 128, tile B one block later
-  const int nA = causal ? (q0 / BN + 1) : kv_blocks;
-  const int nB = has_b ? (causal ? nA + 1 : kv_blocks) : 0;
+  const int allA = causal ? (q0 / BN + 1) : kv_blocks;
+  const int allB = has_b ? (causal ? allA + 1 : kv_blocks) : 0;
+  // this CTA's share [b0, b1) of those blocks: tile A's are divided, tile B's one more goes with the last part
+  const int n_parts = PUSH ? 1 : plan.parts(allA);
+  if (z >= n_parts) return;
+  const int b0 = plan.begin(z);
+  const int b1 = z == n_parts - 1 ? INT_MAX : plan.end(z, allA);
+  const int nA = min(allA, b1) - b0, nB = has_b ? min(allB, b1) - b0 : 0;
   const int nblk = nA > nB ? nA : nB;
 
   if (threadIdx.x == 0) {
@@ -180,12 +187,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const int s = j & 1;
           const uint32_t ph = (j >> 1) & 1;
           if (!mbar_wait(&bars->k_empty[s], ph ^ 1, abort_flag, err, ODY_ERR_TIMEOUT_EMPTY)) break;
-          load_kmajor(sK + s * TILE_BYTES, &tmK, kv_head, j * BN, &bars->k_full[s]);
+          load_kmajor(sK + s * TILE_BYTES, &tmK, kv_head, (b0 + j) * BN, &bars->k_full[s]);
           ++issued_k;
           if (!mbar_wait(&bars->v_empty[s], ph ^ 1, abort_flag, err, ODY_ERR_TIMEOUT_EMPTY)) break;
           mbar_expect_tx(&bars->v_full[s], TILE_BYTES);
-          tma_load_3d(sV + s * TILE_BYTES, &tmV, 0, kv_head, j * BN, &bars->v_full[s]);
-          tma_load_3d(sV + s * TILE_BYTES + HALF_BYTES, &tmV, 64, kv_head, j * BN, &bars->v_full[s]);
+          tma_load_3d(sV + s * TILE_BYTES, &tmV, 0, kv_head, (b0 + j) * BN, &bars->v_full[s]);
+          tma_load_3d(sV + s * TILE_BYTES + HALF_BYTES, &tmV, 64, kv_head, (b0 + j) * BN, &bars->v_full[s]);
           ++issued_v;
         }
         if (*abort_flag) {
@@ -330,8 +337,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tmem_ld_32x32(col_s + 96, sv + 96);
       tmem_ld_wait();
       ODY_FWD_STAMP(tr, j, t * 5 + 2);
-      const int kv0 = j * BN;
-      if (j == diag) {
+      const int kv0 = (b0 + j) * BN;
+      if (b0 + j == diag) {
 #pragma unroll
         for (int c = 0; c < 128; ++c)
           if (c > r) sv[c] = 0xff800000u;               // -inf
@@ -419,7 +426,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // epilogue: O / l -> bf16 -> swizzled smem (this tile's Q is dead by now) -> TMA store; lse
     if (ok && nt > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t], 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
     uint8_t* stage = sQ + t * TILE_BYTES;
-    if (ok && nt > 0) {
+    if (!PUSH && n_parts > 1) {
+      if (ok && nt > 0) {
+        // a part of a split tile: O as accumulated, fp32, and this row's maximum in use and sum; merge_parts_kernel does the rest
+        tc_fence_after();
+        const int64_t row = ((int64_t)(pair * plan.max_parts + z) * H + head) * CTA_ROWS + t * BM + r;
+        part_ml[row] = make_float2(m_used, l);
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c) {
+          uint32_t o[16];
+          tmem_ld_32x16(col_o + c * 16, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(part + row * HD + c * 16 + i * 4) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+        }
+      }
+    } else if (ok && nt > 0) {
       tc_fence_after();
       const float inv_l = 1.f / l;
 #pragma unroll
@@ -443,7 +466,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     tc_fence_before();
     const bool all_ok = named_barrier_and(1 + t, 128, ok);
-    if (all_ok && nt > 0 && q == 0 && lane == 0 && !*abort_flag) {
+    if (all_ok && nt > 0 && n_parts == 1 && q == 0 && lane == 0 && !*abort_flag) {
       tma_store_3d(&tmO, stage, 0, head, qt0);
       tma_store_3d(&tmO, stage + HALF_BYTES, 64, head, qt0);
       if (osplit.rows > 0) {
@@ -462,6 +485,37 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+}
+
+// Parts of split tiles -> output rows and log-sum-exp.  One block per (pair, head, 16-row slice), eight columns per thread;
+// parts are taken in order.  Bound by memory.
+__global__ void __launch_bounds__(256) merge_parts_kernel(const float* __restrict__ part, const float2* __restrict__ part_ml,
+                                                          __nv_bfloat16* __restrict__ o, float* __restrict__ lse, int Tq, int H,
+                                                          int64_t o_row, const SplitUnits units, const SplitPlan plan) {
+  const int pair = blockIdx.x, head = blockIdx.y;
+  const int n_parts = plan.parts(units(pair));
+  const int r = blockIdx.z * 16 + (threadIdx.x >> 4), c = (threadIdx.x & 15) * 8;
+  const int row = pair * CTA_ROWS + r;
+  if (n_parts == 1 || row >= Tq) return;
+  const int64_t base = ((int64_t)pair * plan.max_parts * H + head) * CTA_ROWS + r, step = (int64_t)H * CTA_ROWS;
+  float m = -INFINITY;
+  for (int z = 0; z < n_parts; ++z) m = fmaxf(m, part_ml[base + z * step].x);
+  float l = 0.f, a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int z = 0; z < n_parts; ++z) {
+    const float2 ml = part_ml[base + z * step];
+    const float w = exp2f(ml.x - m);
+    const float* p = part + (base + z * step) * HD + c;
+    const float4 x = *reinterpret_cast<const float4*>(p), y = *reinterpret_cast<const float4*>(p + 4);
+    l += w * ml.y;
+    a[0] += w * x.x; a[1] += w * x.y; a[2] += w * x.z; a[3] += w * x.w;
+    a[4] += w * y.x; a[5] += w * y.y; a[6] += w * y.z; a[7] += w * y.w;
+  }
+  const float inv_l = 1.f / l;
+  *reinterpret_cast<uint4*>(o + (int64_t)row * o_row + head * HD + c) =
+      make_uint4(pack_bf16(a[0] * inv_l, a[1] * inv_l), pack_bf16(a[2] * inv_l, a[3] * inv_l), pack_bf16(a[4] * inv_l, a[5] * inv_l),
+                 pack_bf16(a[6] * inv_l, a[7] * inv_l));
+  if (c == 0) lse[(int64_t)head * Tq + row] = (m + log2f(l)) * 0.6931471805599453f;
 }
 
 }  // namespace fwd
@@ -509,12 +563,40 @@ extern "C" int ody_flash_fwd_push(const void* q, const void* k, const void* v, v
   return ody_flash_fwd_ex(q, k, v, o, lse, Tq, Tk, H, Hkv, q_row, k_row, v_row, o_row, causal, scale, push, nullptr, 0, 0, 0, err, st);
 }
 
-// Full form: optional push (ring) and optional split of the output rows over n_split extra destinations
-// o_split[d] ([split_rows, H, 128], row pitch split_row elements; may be peer memory), split_rows % 128 == 0.
+// Plan of the forward grid when its streamed dimension may be split (attn_split.cuh): 1.9 us per pair of 128 x 128 blocks
+static ody::SplitPlan fwd_plan(int Tq, int Tk, int H, int causal, ody::SplitUnits* u) {
+  using namespace ody;
+  using namespace ody::fwd;
+  *u = SplitUnits{causal ? 2 : 0, (Tk + BN - 1) / BN, 1, 2};
+  return split_plan(*u, (Tq + CTA_ROWS - 1) / CTA_ROWS, H, 1.9, 3.0, (int64_t)CTA_ROWS * (HD + 2) * 4);
+}
+
+// Scratch of the split form for these sizes: fp32 rows of all parts, then their (maximum, sum) pairs.
+extern "C" int64_t ody_flash_fwd_split_bytes(int Tq, int Tk, int H, int causal) {
+  using namespace ody;
+  using namespace ody::fwd;
+  if (Tq <= 0 || Tk <= 0 || H <= 0) return 0;
+  SplitUnits u;
+  const SplitPlan p = fwd_plan(Tq, Tk, H, causal, &u);
+  return p.max_parts > 1 ? (int64_t)((Tq + CTA_ROWS - 1) / CTA_ROWS) * H * p.max_parts * CTA_ROWS * (HD + 2) * 4 : 0;
+}
+
 extern "C" int ody_flash_fwd_ex(const void* q, const void* k, const void* v, void* o, float* lse, int Tq, int Tk, int H,
                                 int Hkv, int64_t q_row, int64_t k_row, int64_t v_row, int64_t o_row, int causal, float scale,
                                 const OdyGatherDesc* push, void* const* o_split, int n_split, int split_rows,
                                 int64_t split_row, int* err, cudaStream_t st) {
+  return ody_flash_fwd_parts(q, k, v, o, lse, Tq, Tk, H, Hkv, q_row, k_row, v_row, o_row, causal, scale, push, o_split, n_split,
+                             split_rows, split_row, nullptr, 0, err, st);
+}
+
+// Full form: optional push (ring) and optional split of the output rows over n_split extra destinations
+// o_split[d] ([split_rows, H, 128], row pitch split_row elements; may be peer memory), split_rows % 128 == 0.
+// With `parts` (16-byte aligned, at least ody_flash_fwd_split_bytes of these sizes) a small grid splits the keys over more CTAs
+// (attn_split.cuh); not together with a push or extra destinations.
+extern "C" int ody_flash_fwd_parts(const void* q, const void* k, const void* v, void* o, float* lse, int Tq, int Tk, int H,
+                                   int Hkv, int64_t q_row, int64_t k_row, int64_t v_row, int64_t o_row, int causal, float scale,
+                                   const OdyGatherDesc* push, void* const* o_split, int n_split, int split_rows,
+                                   int64_t split_row, void* parts, int64_t parts_bytes, int* err, cudaStream_t st) {
   using namespace ody;
   using namespace ody::fwd;
   if (Tq <= 0 || Tk <= 0 || H <= 0 || Hkv <= 0 || H % Hkv) return (int)cudaErrorInvalidValue;
@@ -547,7 +629,15 @@ extern "C" int ody_flash_fwd_ex(const void* q, const void* k, const void* v, voi
     }
     sm.rows = split_rows;
   }
-  const int64_t ctas = (int64_t)((Tq + CTA_ROWS - 1) / CTA_ROWS) * H;
+  SplitUnits units;
+  SplitPlan plan = fwd_plan(Tq, Tk, H, causal, &units);
+  if (parts == nullptr || ((uintptr_t)parts & 15) || push != nullptr || n_split > 0 ||
+      parts_bytes < ody_flash_fwd_split_bytes(Tq, Tk, H, causal))
+    plan = SplitPlan();
+  const int pairs = (Tq + CTA_ROWS - 1) / CTA_ROWS;
+  const int64_t ctas = (int64_t)pairs * H * plan.max_parts;
+  float* part = (float*)parts;
+  float2* part_ml = (float2*)(part + (plan.max_parts > 1 ? ctas * CTA_ROWS * HD : 0));
   if (ctas > INT_MAX) return (int)cudaErrorInvalidValue;
   const dim3 grid((unsigned)ctas);
   gc::GatherParams pp;
@@ -556,13 +646,15 @@ extern "C" int ody_flash_fwd_ex(const void* q, const void* k, const void* v, voi
     if ((r = gc::fill_gather(pp, push))) return r;
     if (push->n_cta <= 0 || push->n_cta > ctas) return (int)cudaErrorInvalidValue;
     if (ks32)
-      flash_fwd_kernel<true, true><<<grid, NUM_THREADS_PUSH, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, push->n_cta, sm);
+      flash_fwd_kernel<true, true><<<grid, NUM_THREADS_PUSH, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, push->n_cta, sm, plan, part, part_ml);
     else
-      flash_fwd_kernel<true, false><<<grid, NUM_THREADS_PUSH, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, push->n_cta, sm);
+      flash_fwd_kernel<true, false><<<grid, NUM_THREADS_PUSH, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, push->n_cta, sm, plan, part, part_ml);
   } else if (ks32) {
-    flash_fwd_kernel<false, true><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm);
+    flash_fwd_kernel<false, true><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm, plan, part, part_ml);
   } else {
-    flash_fwd_kernel<false, false><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm);
+    flash_fwd_kernel<false, false><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm, plan, part, part_ml);
   }
+  if (plan.max_parts > 1)
+    merge_parts_kernel<<<dim3(pairs, H, CTA_ROWS / 16), 256, 0, st>>>(part, part_ml, (__nv_bfloat16*)o, lse, Tq, H, o_row, units, plan);
   return (int)cudaGetLastError();
 }

@@ -111,6 +111,14 @@ int ody_flash_bwd_ex(const void* dO, const void* q, const void* k, const void* v
                      int64_t k_row, int64_t v_row, int64_t o_row, int64_t dq_row, int64_t dk_row, int64_t dv_row, int causal,
                      float scale, void* const* dq_split, void* const* dk_split, void* const* dv_split, int n_split,
                      int split_rows, int* err, cudaStream_t stream);
+// the same with scratch for the partial sums of small grids, whose streamed dimension is then split over more CTAs:
+// parts: ody_flash_bwd_split_bytes(...) bytes, 16-byte aligned (0 bytes: these sizes are not split)
+int64_t ody_flash_bwd_split_bytes(int Tq, int Tk, int H, int Hkv, int causal);
+int ody_flash_bwd_parts(const void* dO, const void* q, const void* k, const void* v, const void* o, const float* lse, void* dq,
+                        void* dk, void* dv, void* workspace, int Tq, int Tk, int H, int Hkv, int64_t do_row, int64_t q_row,
+                        int64_t k_row, int64_t v_row, int64_t o_row, int64_t dq_row, int64_t dk_row, int64_t dv_row, int causal,
+                        float scale, void* const* dq_split, void* const* dk_split, void* const* dv_split, int n_split,
+                        int split_rows, void* parts, int64_t parts_bytes, int* err, cudaStream_t stream);
 
 // ---- GEMM fused with an all-gather of one operand and/or a reduce-scatter of the result over peer memory
 // (gemm_comm.cu).  Descriptions are plain data; pointers in *_peer[p] address rank p's symmetric memory.
@@ -163,6 +171,13 @@ int ody_flash_fwd_ex(const void* q, const void* k, const void* v, void* o, float
                      int64_t q_row, int64_t k_row, int64_t v_row, int64_t o_row, int causal, float scale,
                      const OdyGatherDesc* push, void* const* o_split, int n_split, int split_rows, int64_t split_row, int* err,
                      cudaStream_t stream);
+// the same with scratch for the partial results of small grids, whose keys are then split over more CTAs:
+// parts: ody_flash_fwd_split_bytes(...) bytes, 16-byte aligned (0 bytes: these sizes are not split)
+int64_t ody_flash_fwd_split_bytes(int Tq, int Tk, int H, int causal);
+int ody_flash_fwd_parts(const void* q, const void* k, const void* v, void* o, float* lse, int Tq, int Tk, int H, int Hkv,
+                        int64_t q_row, int64_t k_row, int64_t v_row, int64_t o_row, int causal, float scale,
+                        const OdyGatherDesc* push, void* const* o_split, int n_split, int split_rows, int64_t split_row,
+                        void* parts, int64_t parts_bytes, int* err, cudaStream_t stream);
 int ody_flash_set_peer_wait_limit(long long cycles);
 int ody_flash_set_push_order(int unit_major);
 // schedule of the comm warps' pushes on the current device: 0 destination by destination (default), 1 every unit to all

@@ -481,3 +481,41 @@ def test_attention_bwd_packed_outputs(lib, bwd_variant):
     ref = torch.cat([dqr, dkr, dvr], dim=1)
     assert torch.isfinite(dqkv.float()).all()
     assert ((dqkv.float() - ref).norm() / ref.norm()).item() < 2e-2
+
+
+# Sizes whose grids leave SMs idle, so that the streamed dimension is split over more CTAs (csrc/attn_split.cuh): grouped
+# queries on one kv head, few heads, few query rows on many keys and the reverse, lengths next to a block edge.
+SPLIT_CASES = [
+    (1531, 1531, 8, 2, True), (2600, 2600, 4, 1, True), (1025, 1025, 4, 4, True), (3073, 3073, 2, 2, True),
+    (300, 8000, 2, 2, False), (8000, 257, 4, 1, False), (129, 4097, 1, 1, False), (4096, 4096, 1, 1, True),
+]
+
+
+@pytest.mark.parametrize("Tq,Tk,H,Hkv,causal", SPLIT_CASES)
+def test_attention_split_grids(lib, Tq, Tk, H, Hkv, causal):
+    """Split grids against fp32 PyTorch, with strided operands and gradients, and twice the same bits."""
+    from odysseus_transformer_b200.ops import torch_ref as R
+    torch.manual_seed(Tq + 5 * Tk + H)
+    q = _rand(Tq, H + 1, 128)[:, 1:]
+    kv = _rand(Tk, 2 * Hkv, 128)
+    k, v = kv[:, :Hkv], kv[:, Hkv:]
+    do = _rand(Tq, H, 128)
+    scale = 1.0 / math.sqrt(128)
+    o, lse = lib.attn_fwd(q, k, v, causal, scale)
+    _check_status(lib)
+    orf, lser = R.attn_fwd(q, k, v, causal, scale)
+    torch.testing.assert_close(lse, lser, rtol=1e-3, atol=2e-3)
+    torch.testing.assert_close(o.float(), orf.float(), rtol=2e-2, atol=2e-2)
+    dqb = torch.full((Tq, H + 1, 128), 7.0, device="cuda", dtype=torch.bfloat16)
+    dkv = torch.full_like(kv, float("nan"))
+    got = lib.attn_bwd(do, q, k, v, orf.to(torch.bfloat16), lser, causal, scale, dqb[:, 1:], dkv[:, :Hkv], dkv[:, Hkv:])
+    _check_status(lib)
+    assert (dqb[:, 0] == 7.0).all()
+    ref = R.attn_bwd(do, q, k, v, orf.to(torch.bfloat16), lser, causal, scale)
+    for name, a, b in zip(("dq", "dk", "dv"), got, ref):
+        rel = ((a.float() - b).norm() / b.norm()).item()
+        assert rel < 2e-2, f"{name}: rel err {rel}"
+    o2, lse2 = lib.attn_fwd(q, k, v, causal, scale)
+    again = lib.attn_bwd(do, q, k, v, orf.to(torch.bfloat16), lser, causal, scale, None, None, None)
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)
+    assert all(torch.equal(a, b) for a, b in zip(got, again))
