@@ -15,8 +15,8 @@
 //            would leave the tensor core half idle.  S^T / dP^T are single buffered; the issue order
 //            dV(i), S^T(i+1), dK(i), dP^T(i+1) keeps the in-order tensor pipe busy while the softmax warps
 //            work on the other matrix.  Query heads sharing the kv head are looped inside.
-//   dq     : one CTA per (128-row query tile, head).  Q and dO stay in shared memory; 128-row blocks of K
-//            and V stream.  S = Q K^T, dP = dO V^T (double buffered), dS (bf16 in TMEM) and dQ += dS K.
+//   dq     : one CTA per (128-row query tile, head).  Q and dO stay in TMEM; 128-row blocks of K and V stream.
+//            S = Q K^T, dP = dO V^T, dS (bf16 in TMEM) and dQ += dS K, each in two independent 64-key halves.
 //
 // Splitting dQ from dK/dV recomputes S and dP once more but needs no atomics and is deterministic.
 // Gradients are written with TMA stores through row-pitched tensor maps, so dq/dk/dv may be slices
@@ -958,14 +958,22 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* 
 
 // ------------------------------------------------------------------------------------------- dQ
 // Q and dO of the tile are the A operands of every S = Q K^T and dP = dO V^T of the kernel, so they live in TMEM (bf16,
-// 64 columns each, written once by the softmax warps straight from global memory) and all 24 MMAs of a block are of the
+// 64 columns each, written once by the softmax warps straight from global memory) and all MMAs of a block are of the
 // TS kind: only the streamed K / V block is read from shared memory, which is what bounds the rate of SS instructions.
+//
+// A block is worked on in two 64-key halves, one per softmax warpgroup, with barriers of their own all the way: S_h, dP_h and
+// dS_h of a half depend only on that half.  The kernel is bound by the softmax warps (exponentials of one special-function
+// unit per scheduler, then dS): with one barrier per block the two warps of a scheduler computed exponentials at the same
+// time and dS at the same time, so the unit idled during dS; the halves drift apart and one warp's exponentials run under
+// the other's dS.  It costs twice the instructions for S and dP (64 keys each), which the pipe has room for.  Backward of
+// 8192 tokens x 32 heads 1785 -> 1689 us, 32768 x 4 3093 -> 2896, 12288 x 32 (8 kv heads) 3720 -> 3434.
 constexpr int K_STAGES = 3;
+constexpr int HALF = BLK / 2;                    // keys per softmax warpgroup
 struct BarsQ {
   uint64_t k_full[K_STAGES], k_empty[K_STAGES];
   uint64_t v_full[K_STAGES], v_empty[K_STAGES];
   uint64_t a_ready;                              // Q and dO are in TMEM
-  uint64_t s_full, s_free, dp_full, ds_full;     // one completion per block each: parity = block & 1
+  uint64_t s_full[2], s_free[2], dp_full[2], ds_full[2];   // [64-key half]: one completion per block each, parity = block & 1
   uint64_t acc_done, drain;
   uint32_t tmem_base;
   int abort_flag;
@@ -974,7 +982,7 @@ struct BarsQ {
 // load of K(i+1) could only start when dQ(i-1) had finished and the MMA thread waited ~700 cycles per block for it.
 constexpr int Q_SMEM_TILES = BIG_BYTES + 2 * K_STAGES * BLK_BYTES;       // dQ staging + K ring + V ring
 constexpr int Q_SMEM_TOTAL = Q_SMEM_TILES + 256 + 1024;
-// TMEM columns: S 0..127, dP 128..255 (dS, bf16, overwrites its first 64 columns), dQ 256..383, Q 384..447, dO 448..511
+// TMEM columns: S 0..127, dP 128..255 (dS, bf16, overwrites the first 32 columns of each 64-key half), dQ 256..383, Q 384..447, dO 448..511
 constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DQ = 256, COL_QA = 384, COL_DOA = 448;
 
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -1016,10 +1024,12 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
       mbar_init(&bars->v_full[s], 1); mbar_init(&bars->v_empty[s], 1);
     }
     mbar_init(&bars->a_ready, 256);
-    mbar_init(&bars->s_full, 1);
-    mbar_init(&bars->s_free, 256);
-    mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->ds_full, 256);
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(&bars->s_full[h], 1);
+      mbar_init(&bars->s_free[h], 128);
+      mbar_init(&bars->dp_full[h], 1);
+      mbar_init(&bars->ds_full[h], 128);
+    }
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->drain, 1);
     bars->abort_flag = 0;
@@ -1055,60 +1065,62 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
       // every lane runs the control flow, so the compiler keeps descriptors and loop state in uniform registers;
       // one elected lane issues the tcgen05 instructions (see the note on the issue rate in flash_fwd.cu)
       const bool leader = elect_one();
-      constexpr uint32_t IDESC_S = make_idesc_bf16(BIG, BLK, 0, 0);
+      constexpr uint32_t IDESC_S = make_idesc_bf16(BIG, HALF, 0, 0);
       constexpr uint32_t IDESC_ACC = make_idesc_bf16(BIG, HD, 0, 1);
       bool ok = mbar_wait(&bars->a_ready, 0, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       const uint64_t k_k0 = make_smem_desc(smem_u32(sKs), 16, 1024), v_k0 = make_smem_desc(smem_u32(sVs), 16, 1024);
       const uint64_t k_mn0 = make_smem_desc(smem_u32(sKs), BLK_HALF, 1024);
       const bool trace = dbg != nullptr && blockIdx.x == 0;
-      // S(it) = Q K^T, Q from TMEM
-      auto issue_s = [&](int it) -> bool {
+      // S_h(it) = Q K_h^T over the 64 keys of half h, Q from TMEM
+      auto issue_s = [&](int it, int h) -> bool {
         const int stage = it % K_STAGES;
         if (!mbar_wait(&bars->k_full[stage], (it / K_STAGES) & 1, abort_flag, err, ODY_ERR_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        const uint64_t kd = desc_advance(k_k0, stage * BLK_BYTES);
+        const uint64_t kd = desc_advance(k_k0, stage * BLK_BYTES + h * HALF * 128);
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk)
-          if (leader) umma_ts(tmem + COL_S, tmem + COL_QA + kk * 8, desc_advance(kd, (kk >> 2) * BLK_HALF + (kk & 3) * 32), IDESC_S, kk > 0 ? 1u : 0u);
-        if (leader) umma_commit(&bars->s_full);
+          if (leader) umma_ts(tmem + COL_S + h * HALF, tmem + COL_QA + kk * 8, desc_advance(kd, (kk >> 2) * BLK_HALF + (kk & 3) * 32), IDESC_S, kk > 0 ? 1u : 0u);
+        if (leader) umma_commit(&bars->s_full[h]);
         return true;
       };
-      // dP(it) = dO V^T, dO from TMEM
-      auto issue_dp = [&](int it) -> bool {
+      // dP_h(it) = dO V_h^T, dO from TMEM
+      auto issue_dp = [&](int it, int h) -> bool {
         const int stage = it % K_STAGES;
         if (!mbar_wait(&bars->v_full[stage], (it / K_STAGES) & 1, abort_flag, err, ODY_ERR_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        const uint64_t vd = desc_advance(v_k0, stage * BLK_BYTES);
+        const uint64_t vd = desc_advance(v_k0, stage * BLK_BYTES + h * HALF * 128);
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk)
-          if (leader) umma_ts(tmem + COL_DP, tmem + COL_DOA + kk * 8, desc_advance(vd, (kk >> 2) * BLK_HALF + (kk & 3) * 32), IDESC_S, kk > 0 ? 1u : 0u);
-        if (leader) umma_commit(&bars->v_empty[stage]);
-        if (leader) umma_commit(&bars->dp_full);
+          if (leader) umma_ts(tmem + COL_DP + h * HALF, tmem + COL_DOA + kk * 8, desc_advance(vd, (kk >> 2) * BLK_HALF + (kk & 3) * 32), IDESC_S, kk > 0 ? 1u : 0u);
+        if (h == 1 && leader) umma_commit(&bars->v_empty[stage]);
+        if (leader) umma_commit(&bars->dp_full[h]);
         return true;
       };
-      if (ok && total > 0) ok = issue_s(0) && issue_dp(0);
+      if (ok && total > 0) ok = issue_s(0, 0) && issue_dp(0, 0) && issue_s(0, 1) && issue_dp(0, 1);
       for (int it = 0; it < total && ok; ++it) {
         const uint32_t par = it & 1;
-        if (trace && it < 48) dbg[it * 8 + 0] = clock64();                 // loop start
-        if (it + 1 < total) {
-          // S(it+1) overwrites S(it): the softmax warps must hold S(it) in registers
-          if (!mbar_wait(&bars->s_free, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-          if (trace && it < 48) dbg[it * 8 + 1] = clock64();               // S(it) freed
-          if (!issue_s(it + 1)) { ok = false; break; }
-          if (trace && it < 48) dbg[it * 8 + 2] = clock64();               // S(it+1) issued
-        }
-        if (!mbar_wait(&bars->ds_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-        if (trace && it < 48) dbg[it * 8 + 3] = clock64();                 // dS(it) seen
-        tc_fence_after();
         const uint64_t kmn = desc_advance(k_mn0, (it % K_STAGES) * BLK_BYTES);
-        const uint32_t acc0 = it > 0 ? 1u : 0u;
 #pragma unroll
-        for (int kk = 0; kk < BLK / 16; ++kk)   // dQ += dS K
-          if (leader) umma_ts(tmem + COL_DQ, tmem + COL_DP + kk * 8, desc_advance(kmn, kk * 2048), IDESC_ACC, kk > 0 ? 1u : acc0);
-        if (leader) umma_commit(&bars->k_empty[it % K_STAGES]);
-        // dP(it+1) overwrites dS(it), which the in-order pipe has consumed with dQ(it) by then
-        if (it + 1 < total && !issue_dp(it + 1)) { ok = false; break; }
+        for (int h = 0; h < 2; ++h) {
+          if (trace && it < 48 && h == 0) dbg[it * 8 + 0] = clock64();                 // loop start
+          if (it + 1 < total) {
+            // S_h(it+1) overwrites S_h(it): the softmax warps must hold it in registers
+            if (!mbar_wait(&bars->s_free[h], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+            if (trace && it < 48 && h == 0) dbg[it * 8 + 1] = clock64();               // S(it) freed
+            if (!issue_s(it + 1, h)) { ok = false; break; }
+            if (trace && it < 48 && h == 0) dbg[it * 8 + 2] = clock64();               // S(it+1) issued
+          }
+          if (!mbar_wait(&bars->ds_full[h], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+          if (trace && it < 48 && h == 0) dbg[it * 8 + 3] = clock64();                 // dS(it) seen
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < HALF / 16; ++kk)   // dQ += dS_h K_h
+            if (leader) umma_ts(tmem + COL_DQ, tmem + COL_DP + h * HALF + kk * 8, desc_advance(kmn, (h * (HALF / 16) + kk) * 2048), IDESC_ACC, (it | h | kk) > 0 ? 1u : 0u);
+          if (h == 1 && leader) umma_commit(&bars->k_empty[it % K_STAGES]);
+          // dP_h(it+1) overwrites dS_h(it), which the in-order pipe has consumed with dQ by then
+          if (it + 1 < total && !issue_dp(it + 1, h)) { ok = false; break; }
+        }
       }
       if (ok) {
         if (leader) umma_commit(&bars->acc_done);
@@ -1152,7 +1164,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
       const uint32_t par = it & 1;
       const int kvb0 = (b0 + it) * BLK + hf * 64;
       const bool strace = dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 128 && it < 48;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[hf], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 4] = clock64();                             // S(it) complete
       uint32_t sv[64];
       if (ok) {
@@ -1161,7 +1173,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
         tmem_ld_32x32(tmem + COL_S + hf * 64 + 32 + lane_off, sv + 32);
         tmem_ld_wait();
         tc_fence_before();
-        mbar_arrive(&bars->s_free);                       // S(it) is in registers
+        mbar_arrive(&bars->s_free[hf]);                       // S(it) is in registers
       }
       const bool diag = causal && (kvb0 + 63 > q0);
       const bool tail = kvb0 + 64 > Tk;
@@ -1183,7 +1195,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
         sv[2 * c + 1] = __float_as_uint(p1);
       }
       if (strace) dbg[it * 8 + 5] = clock64();                             // P computed (as far as the compiler kept it here)
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_full[hf], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 6] = clock64();                             // dP(it) complete
       uint32_t dp[64];
       if (ok) {
@@ -1192,8 +1204,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
         tmem_ld_32x32(tmem + COL_DP + hf * 64 + 32 + lane_off, dp + 32);
         tmem_ld_wait();
       }
-      // dS overwrites dP's first 64 columns: both warps of the quarter have loaded; they also agree on leaving
-      if (!named_barrier_and(4 + q, 64, ok)) { ok = false; break; }
+      if (!ok) break;
       uint32_t ds[32];
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
@@ -1202,11 +1213,11 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
         upk2(mul2(pk2u(sv[2 * c], sv[2 * c + 1]), add2(pk2u(dp[2 * c], dp[2 * c + 1]), ndelta_2)), d0, d1);
         ds[c] = pack_bf16(d0, d1);
       }
-      tmem_st_32x16(tmem + COL_DP + hf * 32 + lane_off, ds);
-      tmem_st_32x16(tmem + COL_DP + hf * 32 + 16 + lane_off, ds + 16);
+      tmem_st_32x16(tmem + COL_DP + hf * HALF + lane_off, ds);
+      tmem_st_32x16(tmem + COL_DP + hf * HALF + 16 + lane_off, ds + 16);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars->ds_full);
+      mbar_arrive(&bars->ds_full[hf]);
       if (strace) dbg[it * 8 + 7] = clock64();                             // dS published
     }
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_done, 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
