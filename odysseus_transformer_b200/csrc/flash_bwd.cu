@@ -74,45 +74,57 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
 // equal, so the operand does not depend on which half the hardware takes as k = 0..7).  Tile 0 carries -lse / scale
 // (so that (S^T + c) * scale * log2 e = s * scale * log2 e - lse * log2 e), tile 1 carries -delta.  Layout: 8-row groups
 // of 256 bytes; inside a group the first 16-byte halves of the 8 rows, then the second halves.
-__global__ void prep_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
+// One warp per 8 rows of a head: half a warp reads a row (16 bytes per lane), all eight rows of dO and O are in flight before
+// the first is used, and the statistics leave as whole 128-byte lines - lane = (tile, half, row) stores one 16-byte piece.
+// (One warp per row, 8 bytes per lane and four 16-byte stores by one lane, took 113 us at 12288 x 32 heads; this 50.)
+__global__ void __launch_bounds__(256) prep_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
                             const float* __restrict__ lse, float* __restrict__ delta_pad, float* __restrict__ lse2_pad,
                             uint8_t* __restrict__ stat_tiles, float inv_scale,
                             int T, int Tpad, int H, int64_t do_row, int64_t o_row) {
-  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp_global >= Tpad * H) return;
-  const int t = warp_global / H, h = warp_global % H;
-  float s = 0.f, l2 = 0.f, l1 = 0.f;
-  if (t < T) {
-    const uint2 a = *reinterpret_cast<const uint2*>(dO + (int64_t)t * do_row + h * HD + lane * 4);
-    const uint2 b = *reinterpret_cast<const uint2*>(O + (int64_t)t * o_row + h * HD + lane * 4);
-    const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
+  if (wg >= (int64_t)(Tpad / 8) * H) return;
+  const int h = (int)(wg % H), t0 = (int)(wg / H) * 8;
+  const int sub = lane >> 4, c = (lane & 15) * 8;
+  uint4 a[4], b[4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(b2[i]);
-      s += x.x * y.x + x.y * y.y;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    l1 = lse[(int64_t)h * T + t];
-    l2 = l1 * LOG2E;
-  }
-  if (lane == 0) {
-    delta_pad[(int64_t)h * Tpad + t] = -s;
-    lse2_pad[(int64_t)h * Tpad + t] = -l2;
-    const int blk = t / BLK, row = t % BLK;
-    uint8_t* tile = stat_tiles + ((int64_t)h * (Tpad / BLK) + blk) * STAT_BYTES + (row >> 3) * 256 + (row & 7) * 16;
-    const float c[2] = {-0.5f * l1 * inv_scale, -0.5f * s};
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-      const __nv_bfloat16 hi = __float2bfloat16_rn(c[w]);
-      const __nv_bfloat16 lo = __float2bfloat16_rn(c[w] - __bfloat162float(hi));
-      const uint4 v = make_uint4((uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(lo) << 16), 0u, 0u, 0u);
-      *reinterpret_cast<uint4*>(tile + w * STAT_TILE) = v;
-      *reinterpret_cast<uint4*>(tile + w * STAT_TILE + 128) = v;
+  for (int i = 0; i < 4; ++i) {
+    const int t = t0 + 2 * i + sub;
+    a[i] = b[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (t < T) {
+      a[i] = *reinterpret_cast<const uint4*>(dO + (int64_t)t * do_row + h * HD + c);
+      b[i] = *reinterpret_cast<const uint4*>(O + (int64_t)t * o_row + h * HD + c);
     }
   }
+  const int row = lane & 7;                        // the row whose statistics this lane writes
+  const float l1 = t0 + row < T ? lse[(int64_t)h * T + t0 + row] : 0.f;
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a[i]);
+    const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b[i]);
+    float d = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 x = __bfloat1622float2(a2[j]), y = __bfloat1622float2(b2[j]);
+      d += x.x * y.x + x.y * y.y;
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);      // within the half warp
+    const float even = __shfl_sync(0xffffffffu, d, 0), odd = __shfl_sync(0xffffffffu, d, 16);
+    if ((row >> 1) == i) s = (row & 1) ? odd : even;
+  }
+  const int w = lane >> 4, half = (lane >> 3) & 1;
+  if (lane < 8) {
+    delta_pad[(int64_t)h * Tpad + t0 + row] = -s;
+    lse2_pad[(int64_t)h * Tpad + t0 + row] = -(l1 * LOG2E);
+  }
+  const float v = w == 0 ? -0.5f * l1 * inv_scale : -0.5f * s;
+  const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+  const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(hi));
+  uint8_t* tile = stat_tiles + ((int64_t)h * (Tpad / BLK) + t0 / BLK) * STAT_BYTES + ((t0 % BLK) >> 3) * 256;
+  *reinterpret_cast<uint4*>(tile + w * STAT_TILE + half * 128 + row * 16) =
+      make_uint4((uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(lo) << 16), 0u, 0u, 0u);
 }
 
 // ------------------------------------------------------------------------------------------- dK / dV
@@ -1381,7 +1393,7 @@ extern "C" int ody_flash_bwd_parts(const void* dO, const void* q, const void* k,
   float* lse2_pad = delta_pad + (int64_t)H * Tpad;
   uint8_t* stat_tiles = (uint8_t*)(lse2_pad + (int64_t)H * Tpad);
   {
-    const int64_t warps = (int64_t)Tpad * H;
+    const int64_t warps = (int64_t)(Tpad / 8) * H;
     const int threads = 256;
     const int64_t blocks = (warps * 32 + threads - 1) / threads;
     prep_kernel<<<(unsigned)blocks, threads, 0, st>>>((const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, delta_pad,
