@@ -242,6 +242,21 @@ std::vector<at::Tensor> ce_fwd(const at::Tensor& logits, const at::Tensor& targe
   return {loss, lse};
 }
 
+// loss per row, and the gradient (times scale) written over the logits
+at::Tensor ce_grad_(at::Tensor logits, const at::Tensor& targets, const at::Tensor& scale, int64_t ignore_index) {
+  check_bf16(logits, "logits");
+  ody_req(logits.is_contiguous() && logits.dim() == 2 && targets.scalar_type() == at::kLong && targets.is_contiguous() &&
+          targets.numel() == logits.size(0) && targets.get_device() == logits.get_device(), "ce_grad_: logits [T, V], targets [T] int64");
+  ody_req(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.numel() >= 1 && scale.get_device() == logits.get_device(),
+          "ce_grad_: scale must be a float32 CUDA tensor on the logits' device");
+  c10::cuda::CUDAGuard guard(logits.device());
+  auto loss = at::empty({logits.size(0)}, logits.options().dtype(at::kFloat));
+  ODY_CHECK(ody_ce_grad(logits.data_ptr(), targets.data_ptr<int64_t>(), loss.data_ptr<float>(), scale.data_ptr<float>(),
+                        logits.size(0), logits.size(1), ignore_index, cur_stream()), "ce_grad");
+  ++g_launches;
+  return loss;
+}
+
 void ce_bwd_(at::Tensor logits, const at::Tensor& targets, const at::Tensor& lse, const at::Tensor& scale,
              int64_t ignore_index) {
   check_bf16(logits, "logits");
@@ -254,6 +269,18 @@ void ce_bwd_(at::Tensor logits, const at::Tensor& targets, const at::Tensor& lse
                          lse.data_ptr<float>() + r0, scale.data_ptr<float>(), n, V, ignore_index, cur_stream()), "ce_bwd");
     ++g_launches;
   }
+}
+
+// dst = src * scale[0] (one pass, scale on the device); dst and src contiguous, of one size
+void scale_into_(at::Tensor dst, const at::Tensor& src, const at::Tensor& scale) {
+  check_bf16(dst, "dst"); check_bf16(src, "src");
+  ody_req(dst.is_contiguous() && src.is_contiguous() && dst.numel() == src.numel() && dst.numel() % 8 == 0 &&
+          dst.get_device() == src.get_device(), "scale_into_: contiguous tensors of one size, a multiple of 8");
+  ody_req(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.numel() >= 1 && scale.get_device() == src.get_device(),
+          "scale_into_: scale must be a float32 CUDA tensor on the same device");
+  c10::cuda::CUDAGuard guard(src.device());
+  ODY_CHECK(ody_scale(dst.data_ptr(), src.data_ptr(), scale.data_ptr<float>(), src.numel(), cur_stream()), "scale_into");
+  ++g_launches;
 }
 
 // ------------------------------------------------------------------------------------------- AdamW
@@ -383,6 +410,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("ce_fwd", &ce_fwd);
   m.def("ce_bwd_", &ce_bwd_);
+  m.def("ce_grad_", &ce_grad_);
+  m.def("scale_into_", &scale_into_);
   m.def("adamw_step", &adamw_step, py::arg("master"), py::arg("m"), py::arg("v"), py::arg("grad"), py::arg("param"),
         py::arg("lr"), py::arg("beta1"), py::arg("beta2"), py::arg("eps"), py::arg("weight_decay"), py::arg("step"),
         py::arg("grad_scale"), py::arg("guard") = py::none());

@@ -37,10 +37,17 @@ int ody_swiglu_bwd(const void* dh, const void* gu, void* dgu, int64_t T, int64_t
 // (softmax - onehot) * scale[0]  (scale on device), rows with target == ignore_index get 0.
 int ody_ce_fwd(const void* logits, const int64_t* targets, float* loss, float* lse, int64_t T, int64_t V,
                int64_t ignore_index, cudaStream_t stream);
+// ce_fwd and ce_bwd in one kernel: loss [T], logits overwritten by their gradient
+int ody_ce_grad(void* logits, const int64_t* targets, float* loss, const float* scale, int64_t T, int64_t V,
+                int64_t ignore_index, cudaStream_t stream);
 int ody_ce_bwd(void* logits, const int64_t* targets, const float* lse, const float* scale, int64_t T, int64_t V,
                int64_t ignore_index, cudaStream_t stream);
 
 // ---- AdamW on flat shards: fp32 master / m / v, bf16 grad in, bf16 param out.  guard (device, may be null):
+// dst = src * scale[0] over n bf16 values (n % 8 == 0; dst may be src)
+int ody_scale(void* dst, const void* src, const float* scale, int64_t n, cudaStream_t stream);
+// dst = src * scale[0] over n bf16 values (n % 8 == 0; dst may be src)
+int ody_scale(void* dst, const void* src, const float* scale, int64_t n, cudaStream_t stream);
 // when *guard != 0 at run time the kernel changes nothing (a failed step must not reach the master weights).
 int ody_adamw(float* master, float* m, float* v, const void* grad, void* param, int64_t n, float lr, float beta1,
               float beta2, float eps, float weight_decay, int step, float grad_scale, const float* guard,

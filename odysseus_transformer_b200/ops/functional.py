@@ -417,6 +417,16 @@ def cross_entropy_sum(logits: torch.Tensor, targets: torch.Tensor, scale: float 
     return _CrossEntropySum.apply(logits, targets, scale, ignore_index)
 
 
+def _scaled(g: torch.Tensor, scale: torch.Tensor, out: Optional[torch.Tensor]) -> torch.Tensor:
+    """``g * scale`` for a one-element device tensor ``scale``, into ``out`` when given."""
+    if (native.use_native(g) and g.is_contiguous() and g.numel() % 8 == 0 and g.data_ptr() % 16 == 0 and scale.is_cuda
+            and (out is None or (out.is_contiguous() and out.dtype == g.dtype and out.data_ptr() % 16 == 0))):
+        out = torch.empty_like(g) if out is None else out
+        native.lib().scale_into_(out, g, scale.detach().float().reshape(1))
+        return out
+    return torch.mul(g, scale.to(g.dtype)) if out is None else torch.mul(g, scale.to(g.dtype), out=out)
+
+
 class _ChunkedLinearCrossEntropy(Function):
     """lm_head + cross-entropy over row chunks, gradients computed in the same pass.
 
@@ -441,16 +451,17 @@ class _ChunkedLinearCrossEntropy(Function):
         for r0 in range(0, t, chunk_rows):
             hc, tc = h[r0:r0 + chunk_rows], targets[r0:r0 + chunk_rows]
             logits = gemm_nt(hc, full)
-            if use_native:
+            grads = need_dh or need_dw
+            if use_native and grads:
+                loss = native.lib().ce_grad_(logits, tc, scale_t, ignore_index)      # loss and gradient in one pass
+            elif use_native:
                 loss, lse = native.lib().ce_fwd(logits, tc, ignore_index)
             else:
                 loss, lse = R.cross_entropy_fwd(logits, tc, ignore_index)
             total += loss.sum()
-            if not (need_dh or need_dw):
+            if not grads:
                 continue
-            if use_native:
-                native.lib().ce_bwd_(logits, tc, lse, scale_t, ignore_index)
-            else:
+            if not use_native:
                 R.cross_entropy_bwd_(logits, tc, lse, scale_t[0], ignore_index)
             if need_dh:
                 gemm_nn(logits, full, out=dh[r0:r0 + chunk_rows])
@@ -470,9 +481,17 @@ class _ChunkedLinearCrossEntropy(Function):
         saved = list(ctx.saved_tensors)
         dh = saved.pop(0) if ctx.have[0] else None
         dw = saved.pop(0) if ctx.have[1] else None
+        gw = None
         if dh is not None:
-            dh = dh * dloss.to(dh.dtype)
-        gw = deliver_grad(ctx.w, dw * dloss.to(dw.dtype)) if dw is not None else None
+            dh = _scaled(dh, dloss, None)
+        if dw is not None:
+            w = ctx.w
+            mg = getattr(w, "main_grad", None)
+            if mg is not None and mg.dtype == dw.dtype and not getattr(w, "_grad_written", False):
+                _scaled(dw, dloss, mg)                     # scaled on its way to the optimizer: one pass over [V/n, d]
+                w._grad_written = True
+            else:
+                gw = deliver_grad(w, _scaled(dw, dloss, None))
         return dh, gw, None, None, None, None, None
 
 

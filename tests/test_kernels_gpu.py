@@ -519,3 +519,35 @@ def test_attention_split_grids(lib, Tq, Tk, H, Hkv, causal):
     again = lib.attn_bwd(do, q, k, v, orf.to(torch.bfloat16), lser, causal, scale, None, None, None)
     assert torch.equal(o, o2) and torch.equal(lse, lse2)
     assert all(torch.equal(a, b) for a, b in zip(got, again))
+
+
+@pytest.mark.parametrize("T,V,ignore", [(37, 32000, True), (5, 128256, False), (64, 8, True), (3, 8200, False)])
+def test_cross_entropy_grad_in_one_pass(lib, T, V, ignore):
+    """Loss and gradient of the one-pass kernel against the two kernels it replaces where the scale is known up front."""
+    torch.manual_seed(V + T)
+    logits = _rand(T, V, scale=3.0)
+    tg = torch.randint(V, (T,), device="cuda")
+    if ignore:
+        tg[::5] = -100
+    scale = torch.full((1,), 0.37, device="cuda")
+    loss, lse = lib.ce_fwd(logits, tg, -100)
+    want = logits.clone()
+    lib.ce_bwd_(want, tg, lse, scale, -100)
+    got = logits.clone()
+    loss1 = lib.ce_grad_(got, tg, scale, -100)
+    torch.cuda.synchronize()
+    torch.testing.assert_close(loss1, loss, rtol=1e-5, atol=1e-5)      # sums of fp32 exponentials in another order
+    torch.testing.assert_close(got.float(), want.float(), rtol=1e-2, atol=1e-6)
+
+
+def test_scale_into(lib):
+    src = _rand(123, 72)
+    scale = torch.full((1,), 0.3, device="cuda")
+    want = (src.float() * 0.3).to(torch.bfloat16)
+    dst = torch.full_like(src, float("nan"))
+    lib.scale_into_(dst, src, scale)
+    assert torch.equal(dst, want)
+    lib.scale_into_(src, src, scale)
+    assert torch.equal(src, want)
+    with pytest.raises(RuntimeError):
+        lib.scale_into_(dst[:, :64], src[:, :64], scale)
