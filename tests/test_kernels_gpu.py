@@ -551,3 +551,19 @@ def test_scale_into(lib):
     assert torch.equal(src, want)
     with pytest.raises(RuntimeError):
         lib.scale_into_(dst[:, :64], src[:, :64], scale)
+
+
+@pytest.mark.parametrize("T,V,d", [(1, 8, 8), (777, 50, 1024), (300, 32000, 136), (2048, 100000, 64)])
+def test_embedding_grad(lib, T, V, d):
+    """Rows that several tokens share are summed in bf16, as index_add into a bf16 gradient does: each of k additions may
+    round by half a bf16 step (2^-9) of the partial sum."""
+    torch.manual_seed(T + V)
+    dy, ids = _rand(T, d), torch.randint(V, (T,), device="cuda")
+    dw = torch.full((V, d), float("nan"), device="cuda", dtype=torch.bfloat16)
+    lib.embedding_grad_(dy, ids, dw)
+    torch.cuda.synchronize()
+    want = torch.zeros(V, d, device="cuda").index_add_(0, ids, dy.float())
+    size = torch.zeros(V, d, device="cuda").index_add_(0, ids, dy.float().abs())
+    k = torch.bincount(ids, minlength=V).view(V, 1)
+    assert ((dw.float() - want).abs() <= k * 2.0 ** -9 * size + 1e-30).all()
+    assert torch.equal(dw[k.view(-1) == 0], torch.zeros_like(dw[k.view(-1) == 0]))
