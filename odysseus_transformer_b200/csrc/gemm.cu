@@ -62,11 +62,15 @@ __device__ __forceinline__ bool epi_all_ok(bool ok) {
 
 // ROPE: the epilogue rotates the q / k heads of a packed projection (RopeEpi, sm100.cuh); a separate instance, so that
 // the plain one keeps its register allocation
-template <int LAYOUT, bool ROPE>
+//
+// SPLIT: `splits` CTAs share a tile's k-blocks; each writes its fp32 accumulator to part [splits][M][N] and
+// splitk_sum_kernel does what the epilogue would have done.
+template <int LAYOUT, bool ROPE, bool SPLIT = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __nv_bfloat16* __restrict__ c_in, int M, int N, int K,
-                 int64_t ldc, int accumulate, int mn3d, const RopeEpi rp, int* __restrict__ err) {
+                 int64_t ldc, int accumulate, int mn3d, const RopeEpi rp, int* __restrict__ err,
+                 float* __restrict__ part = nullptr, int splits = 1) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   GemmBars* bars = (GemmBars*)(smem + SMEM_TILES);
@@ -75,8 +79,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
+  const int num_items = tiles_m * tiles_n * (SPLIT ? splits : 1);      // item = tile * splits + which share of its k-blocks
   const int kblocks = (K + BK - 1) / BK;
+  auto kb_begin = [&](int item) { return SPLIT ? (int)((int64_t)kblocks * (item % splits) / splits) : 0; };
+  auto kb_end = [&](int item) { return SPLIT ? (int)((int64_t)kblocks * (item % splits + 1) / splits) : kblocks; };
   constexpr bool A_MN = (LAYOUT == 2), B_MN = (LAYOUT != 0);
   constexpr uint32_t IDESC = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
 
@@ -112,11 +118,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t phase = 0;
       int issued = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
         int tm, tn;
-        tile_coords(tile, tiles_m, tiles_n, tm, tn);
+        tile_coords(SPLIT ? item / splits : item, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * BM, n0 = tn * BN;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        const int kb1 = kb_end(item);
+        for (int kb = kb_begin(item); kb < kb1; ++kb) {
           if (!mbar_wait(&bars->empty[stage], phase ^ 1, abort_flag, err, ODY_ERR_TIMEOUT_EMPTY)) { ok = false; break; }
           uint8_t* sA = smem + stage * STAGE_BYTES;
           uint8_t* sB = sA + A_BYTES;
@@ -165,17 +172,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t s0 = smem_u32(smem);
       const uint64_t adesc0 = A_MN ? make_smem_desc(s0, 8192, 1024) : make_smem_desc(s0, 16, 1024);
       const uint64_t bdesc0 = B_MN ? make_smem_desc(s0 + A_BYTES, 8192, 1024) : make_smem_desc(s0 + A_BYTES, 16, 1024);
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++local_tile) {
+        const int kb0 = kb_begin(item), kb1 = kb_end(item);
         const int buf = local_tile & 1;
         const uint32_t acc_phase = (local_tile >> 1) & 1;
         if (!mbar_wait(&bars->tmem_empty[buf], acc_phase ^ 1, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&bars->full[stage], phase, abort_flag, err, ODY_ERR_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint64_t a0 = desc_advance(adesc0, stage * STAGE_BYTES), b0 = desc_advance(bdesc0, stage * STAGE_BYTES);
-          if (leader) umma_ss(d_tmem, a0, b0, IDESC, kb > 0 ? 1u : 0u);
+          if (leader) umma_ss(d_tmem, a0, b0, IDESC, kb > kb0 ? 1u : 0u);
 #pragma unroll
           for (int kk = 1; kk < BK / UMMA_K; ++kk)
             if (leader) umma_ss(d_tmem, desc_advance(a0, kk * (A_MN ? 2048 : 32)), desc_advance(b0, kk * (B_MN ? 2048 : 32)), IDESC, 1u);
@@ -196,9 +204,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int r = q * 32 + lane;                 // row inside the tile
     const bool store_thread = (warp == 2 && lane == 0);
     int local_tile = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local_tile) {
+    for (int item = blockIdx.x; item < num_items; item += gridDim.x, ++local_tile) {
       int tm, tn;
-      tile_coords(tile, tiles_m, tiles_n, tm, tn);
+      tile_coords(SPLIT ? item / splits : item, tiles_m, tiles_n, tm, tn);
       const int m0 = tm * BM, n0 = tn * BN;
       const int buf = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
@@ -208,8 +216,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll 1
       for (int c = 0; c < BN / EPI_COLS; ++c) {
         uint8_t* sbuf = epi + (c & 1) * EPI_BYTES;
-        if (store_thread) tma_store_wait_read<1>();
-        named_barrier(1, 128);
+        if (!SPLIT) {
+          if (store_thread) tma_store_wait_read<1>();
+          named_barrier(1, 128);
+        }
         const uint32_t taddr = tmem_base + buf * BN + c * EPI_COLS + ((uint32_t)(q * 32) << 16);
         uint32_t v[64];
         tmem_ld_32x32(taddr, v);
@@ -228,6 +238,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (c == BN / EPI_COLS - 1) {
           tc_fence_before();
           mbar_arrive(&bars->tmem_empty[buf]);
+        }
+        if constexpr (SPLIT) {
+          if (row < M) {
+            float* dst = part + ((int64_t)(item % splits) * M + row) * N + col0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (col0 + j * 4 < N)
+                *reinterpret_cast<uint4*>(dst + j * 4) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          }
+          continue;
         }
         if (accumulate && row < M) {
           const __nv_bfloat16* cp = c_in + (int64_t)row * ldc + col0;
@@ -273,15 +293,64 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// C = sum over the shares of a split product, in order, then what the GEMM epilogue does: rotary embedding of the q / k heads,
+// plus what C accumulates onto or the residual, one rounding.  Eight columns per thread; bound by the partials' reads (L2).
+__global__ void __launch_bounds__(256) splitk_sum_kernel(const float* __restrict__ part, int splits, int M, int N,
+                                                         const __nv_bfloat16* c_in, int64_t ld_in, int accumulate, const RopeEpi rp,
+                                                         __nv_bfloat16* C, int64_t ldc) {
+  const int vpr = N / 8;
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (int64_t)M * vpr) return;
+  const int row = (int)(i / vpr), col = (int)(i % vpr) * 8;
+  auto sum8 = [&](int c, float* a) {
+    const float* p = part + (int64_t)row * N + c;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] = 0.f;
+#pragma unroll 4
+    for (int z = 0; z < splits; ++z) {
+      const float4 x = *reinterpret_cast<const float4*>(p + (int64_t)z * M * N), y = *reinterpret_cast<const float4*>(p + (int64_t)z * M * N + 4);
+      a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+      a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+    }
+  };
+  float a[8];
+  sum8(col, a);
+  if (rope_epi_wants(rp, col & ~63)) {
+    // the other half of this head, 64 columns away
+    const bool hi = (col & 64) != 0;
+    float w[8];
+    sum8(hi ? col - 64 : col + 64, w);
+    const float* cs = rp.cos + (int64_t)row * 64 + (col & 63);
+    const float* sn = rp.sin + (int64_t)row * 64 + (col & 63);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] = a[e] * cs[e] + (hi ? 1.f : -1.f) * w[e] * sn[e];
+  }
+  if (accumulate) {
+    const uint4 old = *reinterpret_cast<const uint4*>(c_in + (int64_t)row * ld_in + col);
+    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&old);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float2 f = __bfloat1622float2(o2[t]);
+      a[2 * t] += f.x;
+      a[2 * t + 1] += f.y;
+    }
+  }
+  uint4 o;
+  __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) p2[t] = __floats2bfloat162_rn(a[2 * t], a[2 * t + 1]);
+  *reinterpret_cast<uint4*>(C + (int64_t)row * ldc + col) = o;
+}
+
 static int g_num_sms = 0;
 
-template <int LAYOUT, bool ROPE>
+template <int LAYOUT, bool ROPE, bool SPLIT = false>
 static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                        int64_t ldc, int accumulate, const void* c_in, int64_t ld_in, const RopeEpi& rp, int* err,
-                       cudaStream_t st) {
+                       cudaStream_t st, float* part = nullptr, int splits = 1) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<LAYOUT, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<LAYOUT, ROPE, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
@@ -303,10 +372,14 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (r) return 710000 + r;
   r = make_tmap_2d_bf16(&tC, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc * 2, EPI_COLS, BM);
   if (r) return 720000 + r;
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * splits;
   const int grid = tiles < g_num_sms ? tiles : g_num_sms;
-  gemm_bf16_kernel<LAYOUT, ROPE><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tA, tB, tC, (const __nv_bfloat16*)c_in, M, N, K, ld_in,
-                                                                  accumulate, mn3d, rp, err);
+  gemm_bf16_kernel<LAYOUT, ROPE, SPLIT><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tA, tB, tC, (const __nv_bfloat16*)c_in, M, N, K, ld_in,
+                                                                  accumulate, mn3d, rp, err,
+                                                                  part, splits);
+  if (SPLIT)
+    splitk_sum_kernel<<<(unsigned)(((int64_t)M * (N / 8) + 255) / 256), 256, 0, st>>>(part, splits, M, N, (const __nv_bfloat16*)c_in, ld_in,
+                                                                                      accumulate, rp, (__nv_bfloat16*)C, ldc);
   return (int)cudaGetLastError();
 }
 
@@ -349,6 +422,64 @@ extern "C" int ody_gemm_resolve_epilogue(const OdyEpilogue* epi, const void* C, 
   }
   (void)M;
   return 0;
+}
+
+// CTAs that share a tile's k-blocks (1: none).  A product with few output tiles and a long K leaves most SMs idle and the
+// others in a long chain (512 x 1024 from K = 32000, the gradient of a small model's last hidden state: 16 tiles of 500
+// k-blocks).  Estimates in us: 0.3 per 64-deep k-block of a 128 x 256 tile, operands at 6 TB/s, and for a split one
+// more launch and its partials written and read in the L2; a split has to promise a sixth.
+static int gemm_splits(int M, int N, int K) {
+  const int sms = 148;
+  if (g_gemm_variant != 0 || (N % 8)) return 1;
+  const int64_t tiles = (int64_t)((M + 127) / 128) * ((N + 255) / 256), kblocks = (K + 63) / 64;
+  if (tiles > sms / 2 || kblocks < 8) return 1;
+  const double mem = ((double)M * K + (double)N * K) * 2.0 / 6.0e6;
+  double best = 0.3 * kblocks > mem ? 0.3 * kblocks : mem;
+  best *= 0.85;
+  int splits = 1;
+  for (int s = 2; s <= sms / tiles && s <= 32 && s * 4 <= kblocks; ++s) {
+    double t = 0.3 * ((kblocks + s - 1) / s);
+    t = (t > mem ? t : mem) + 3.0 + (double)s * M * N * 8.0 / 6.0e6;
+    if (t < best) { best = t; splits = s; }
+  }
+  return splits;
+}
+
+// Scratch ody_gemm_bf16_ws can use for this product; 0: it is not split.
+extern "C" int64_t ody_gemm_split_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int s = gemm_splits(M, N, K);
+  return s > 1 ? (int64_t)s * M * N * 4 : 0;
+}
+
+template <int LAYOUT>
+static int gemm_split(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+                      int accumulate, const void* c_in, int64_t ld_in, const ody::RopeEpi& rp, int* err, cudaStream_t st, float* ws,
+                      int splits) {
+  return ody::launch_gemm<LAYOUT, false, true>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, ws, splits);
+}
+
+// ody_gemm_bf16_ex with scratch (16-byte aligned, ody_gemm_split_bytes of the sizes): products with few tiles split K.
+extern "C" int ody_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
+                                int64_t ldc, int layout, int accumulate, const OdyEpilogue* epi, void* ws, int64_t ws_bytes,
+                                int* err, cudaStream_t st) {
+  const int64_t need = ody_gemm_split_bytes(M, N, K);
+  if (need == 0 || ws == nullptr || ws_bytes < need || ((uintptr_t)ws & 15))
+    return ody_gemm_bf16_ex(A, B, C, M, N, K, lda, ldb, ldc, layout, accumulate, epi, err, st);
+  if ((lda % 8) || (ldb % 8) || (ldc % 8) || (N % 8) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15))
+    return (int)cudaErrorInvalidValue;
+  const void* c_in;
+  int64_t ld_in;
+  ody::RopeEpi rp;
+  if (int r = ody_gemm_resolve_epilogue(epi, C, M, N, ldc, &accumulate, &c_in, &ld_in, &rp)) return r;
+  if (rp.cos != nullptr && layout != 0) return (int)cudaErrorInvalidValue;
+  const int splits = gemm_splits(M, N, K);
+  switch (layout) {
+    case 0: return gemm_split<0>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
+    case 1: return gemm_split<1>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
+    case 2: return gemm_split<2>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
+  }
+  return (int)cudaErrorInvalidValue;
 }
 
 extern "C" int ody_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,

@@ -87,6 +87,11 @@ typedef struct OdyEpilogue {
 } OdyEpilogue;
 int ody_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
                      int layout, int accumulate, const OdyEpilogue* epilogue, int* err, cudaStream_t stream);
+// the same with scratch: products with few output tiles and a long K split it over more CTAs (0 bytes: not split)
+int64_t ody_gemm_split_bytes(int M, int N, int K);
+int ody_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+                     int layout, int accumulate, const OdyEpilogue* epilogue, void* ws, int64_t ws_bytes, int* err,
+                     cudaStream_t stream);
 int ody_gemm_bf16_2cta_ex(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
                           int layout, int accumulate, const OdyEpilogue* epilogue, int* err, cudaStream_t stream);
 

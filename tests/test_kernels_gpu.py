@@ -567,3 +567,55 @@ def test_embedding_grad(lib, T, V, d):
     k = torch.bincount(ids, minlength=V).view(V, 1)
     assert ((dw.float() - want).abs() <= k * 2.0 ** -9 * size + 1e-30).all()
     assert torch.equal(dw[k.view(-1) == 0], torch.zeros_like(dw[k.view(-1) == 0]))
+
+
+# Few output tiles and a long K (the split of csrc/gemm.cu): one tile, ragged edges, the smallest and largest number of shares
+SPLITK_SHAPES = [(128, 256, 2048), (512, 1024, 32000), (8, 8, 65536), (130, 264, 1000), (1, 4096, 11008), (2000, 72, 8200),
+                 (128, 1024, 2816)]
+
+
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K", SPLITK_SHAPES)
+def test_gemm_split_k(lib, layout, M, N, K):
+    """Against fp32 and against the unsplit kernel; accumulating onto C, with a residual, into a strided output."""
+    torch.manual_seed(M + N + K + layout)
+    K = K // 8 * 8
+    if layout == 2:
+        M = max(8, M // 8 * 8)
+    a = _rand(M, K) if layout != 2 else _rand(K, M)
+    b = _rand(N, K) if layout == 0 else _rand(K, N)
+    ref = (a.float() if layout != 2 else a.float().t()) @ (b.float().t() if layout == 0 else b.float())
+    c = lib.gemm(a, b, None, layout, False)
+    lib.gemm_set_variant(1)
+    c1 = lib.gemm(a, b, None, layout, False)
+    lib.gemm_set_variant(0)
+    _check_status(lib)
+    assert ((c.float() - ref).norm() / ref.norm()).item() <= 1.05 * ((c1.float() - ref).norm() / ref.norm()).item() + 1e-5
+    wide = _rand(M, 2 * N)
+    want = wide.float().clone()
+    want[:, N:] += ref
+    lib.gemm(a, b, wide[:, N:], layout, True)
+    _check_status(lib)
+    assert ((wide.float() - want).norm() / want.norm()).item() < 5e-3
+    res = _rand(M, N)
+    if layout == 0:
+        y = lib.gemm(a, b, None, 0, False, None, res)
+        _check_status(lib)
+        assert ((y.float() - (ref + res.float())).norm() / (ref + res.float()).norm()).item() < 5e-3
+
+
+@pytest.mark.parametrize("M", [1, 128, 300])
+def test_gemm_split_k_rope(lib, M):
+    """The rotary epilogue done by the summing kernel equals the one of the unsplit kernel up to the sum's rounding."""
+    from odysseus_transformer_b200.ops import torch_ref as R
+    torch.manual_seed(M)
+    N, K = 768, 4096
+    a, b = _rand(M, K), _rand(N, K)
+    cos, sin = R.rope_tables(torch.randint(0, 9999, (M,), device="cuda"), 128, 10000.0)
+    rope = (cos, sin, 256, 384)
+    y = lib.gemm(a, b, None, 0, False, rope, None)
+    lib.gemm_set_variant(1)
+    y1 = lib.gemm(a, b, None, 0, False, rope, None)
+    lib.gemm_set_variant(0)
+    _check_status(lib)
+    assert ((y.float() - y1.float()).norm() / y1.float().norm()).item() < 2e-3
