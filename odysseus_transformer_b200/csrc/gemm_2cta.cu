@@ -282,8 +282,29 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const uint32_t empty0 = map_to_cta(&bars->tmem_empty[buf], 0);
 #pragma unroll 1
       for (int c = 0; c < BN / EPI_COLS; ++c) {
+        if (ROPE && rope_epi_wants(rp, n0 + c * EPI_COLS)) {
+          // both halves of a head at once; its high half is the next chunk
+          const int row = m0 + r, col0 = n0 + c * EPI_COLS;
+          if (store_thread) tma_store_wait_read<0>();
+          named_barrier(1, 128);
+          rope_epi_head(rp, row, row < M, tmem_base + buf * BN + c * EPI_COLS + ((uint32_t)(q * 32) << 16), epi, epi + EPI_BYTES, r,
+                        accumulate && row < M && col0 < N ? c_in + (int64_t)row * ldc + col0 : nullptr);
+          if (c == BN / EPI_COLS - 2) {
+            tc_fence_before();
+            mbar_arrive_cluster(empty0);
+          }
+          fence_proxy_async_smem();
+          named_barrier(1, 128);
+          if (store_thread && col0 < N && m0 < M) {
+            tma_store_2d(&tmC, epi, col0, m0);
+            tma_store_2d(&tmC, epi + EPI_BYTES, col0 + EPI_COLS, m0);
+            tma_store_commit();
+          }
+          ++c;
+          continue;
+        }
         uint8_t* sbuf = epi + (c & 1) * EPI_BYTES;
-        if (store_thread) tma_store_wait_read<1>();
+        if (store_thread) tma_store_wait_read<ROPE ? 0 : 1>();     // a rotated head leaves both tiles in one group
         named_barrier(1, 128);
         const uint32_t taddr = tmem_base + buf * BN + c * EPI_COLS + ((uint32_t)(q * 32) << 16);
         uint32_t v[64];
@@ -291,15 +312,6 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         tmem_ld_32x32(taddr + 32, v + 32);
         tmem_ld_wait();
         const int row = m0 + r, col0 = n0 + c * EPI_COLS;
-        if (ROPE && rope_epi_wants(rp, col0)) {
-          // the other half of this head, still in the accumulator (read before the buffer is handed back below)
-          uint32_t w[64];
-          const uint32_t paddr = (c & 1) ? taddr - EPI_COLS : taddr + EPI_COLS;
-          tmem_ld_32x32(paddr, w);
-          tmem_ld_32x32(paddr + 32, w + 32);
-          tmem_ld_wait();
-          if (row < M) rope_epi_apply(rp, row, c & 1, v, w);
-        }
         if (c == BN / EPI_COLS - 1) {
           tc_fence_before();
           mbar_arrive_cluster(empty0);            // this thread's rows of the accumulator are in registers
