@@ -17,8 +17,31 @@ from typing import NamedTuple, Optional, Tuple
 
 import torch
 from torch.autograd import Function
+from torch.autograd import forward_ad as _forward_ad
 
 from . import native, torch_ref as R
+
+# ----------------------------------------------------------------------------- calling autograd functions
+
+
+class _NoBackward:
+    """Stands in for an autograd function's ``ctx`` where no backward can follow."""
+
+    needs_input_grad = (False,) * 16
+
+    def save_for_backward(self, *tensors):
+        pass
+
+
+def call(fn, *args):
+    """``fn.apply(*args)``, without autograd's wrapping when gradients are off: evaluation of a short prompt is bound by the
+    host, and the wrapping was a third of a call's time there (logits of 128 tokens, two layers).  Whatever else looks at
+    ``apply`` - functorch transforms, forward-mode levels, tracing, compilation - still gets it."""
+    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling()):
+        return fn.apply(*args)
+    return fn.forward(_NoBackward(), *args)
+
 
 # ----------------------------------------------------------------------------- GEMM primitives
 
@@ -155,7 +178,7 @@ class _Linear(Function):
 
 def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """y = x @ w^T with w [out, in] (no bias: Llama has none)."""
-    return _Linear.apply(x, w)
+    return call(_Linear, x, w)
 
 
 # ----------------------------------------------------------------------------- RMSNorm
@@ -183,7 +206,7 @@ class _RMSNorm(Function):
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
-    return _RMSNorm.apply(x, w, eps)
+    return call(_RMSNorm, x, w, eps)
 
 
 class _AddRMSNorm(Function):
@@ -212,7 +235,7 @@ class _AddRMSNorm(Function):
 
 
 def add_rmsnorm(x: torch.Tensor, delta: torch.Tensor, w: torch.Tensor, eps: float):
-    return _AddRMSNorm.apply(x, delta, w, eps)
+    return call(_AddRMSNorm, x, delta, w, eps)
 
 
 class _RMSNormKeep(Function):
@@ -243,7 +266,7 @@ class _RMSNormKeep(Function):
 
 def rmsnorm_keep(s: torch.Tensor, w: torch.Tensor, eps: float):
     """(s, rmsnorm(s)); see ``_RMSNormKeep``."""
-    return _RMSNormKeep.apply(s, w, eps)
+    return call(_RMSNormKeep, s, w, eps)
 
 
 # Work folded into GEMM epilogues by the model blocks: "rope" - the q|k|v projection rotates q and k; "residual" - the
@@ -291,7 +314,7 @@ class _RoPE(Function):
 
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     """Rotate-half RoPE on [T, H, hd] (HF convention, reference decoder/odysseus.py:210-213)."""
-    return _RoPE.apply(x, cos, sin)
+    return call(_RoPE, x, cos, sin)
 
 
 # ----------------------------------------------------------------------------- SwiGLU
@@ -316,7 +339,7 @@ class _SwiGLU(Function):
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """[T, 2i] = [gate | up] -> silu(gate) * up (reference decoder/odysseus.py:293-295)."""
-    return _SwiGLU.apply(gate_up)
+    return call(_SwiGLU, gate_up)
 
 
 # ----------------------------------------------------------------------------- attention
@@ -378,7 +401,7 @@ class _Attention(Function):
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = True,
               scale: Optional[float] = None) -> torch.Tensor:
     """Softmax attention, q [T,H,hd], k/v [T,Hkv,hd] (GQA when Hkv < H)."""
-    return _Attention.apply(q, k, v, causal, scale)
+    return call(_Attention, q, k, v, causal, scale)
 
 
 # ----------------------------------------------------------------------------- cross-entropy
@@ -535,4 +558,4 @@ class _Embedding(Function):
 
 
 def embedding(ids: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    return _Embedding.apply(ids, w)
+    return call(_Embedding, ids, w)

@@ -271,4 +271,4 @@ def packed_rope_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
     epilogue (``parallel.linear.ag_linear(..., rope=...)``); the forward rotation is skipped, the backward one is not."""
     hd = qkv.shape[1] // (hq + 2 * hkv)
     scale = scale if scale is not None else 1.0 / math.sqrt(hd)
-    return _PackedRopeAttention.apply(qkv, cos, sin, hq, hkv, ring_group, scale, pre_rotated)
+    return F.call(_PackedRopeAttention, qkv, cos, sin, hq, hkv, ring_group, scale, pre_rotated)

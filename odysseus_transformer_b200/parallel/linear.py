@@ -201,7 +201,7 @@ def ag_linear(x: torch.Tensor, w: torch.Tensor, group, rope=None) -> torch.Tenso
     from ..ops import fused_comm
     if fused_comm.enabled(x, group):
         return fused_comm.ag_linear(x, w, group, rope)
-    return _AGLinear.apply(x, w, group, rope)
+    return F.call(_AGLinear, x, w, group, rope)
 
 
 # ----------------------------------------------------------------------------- GEMM -> RS (row parallel)
@@ -239,7 +239,7 @@ def linear_rs(x: torch.Tensor, w: torch.Tensor, group, residual: Optional[torch.
     from ..ops import fused_comm
     if fused_comm.enabled(x, group):
         return fused_comm.linear_rs(x, w, group, residual)
-    return _LinearRS.apply(x, w, group, residual)
+    return F.call(_LinearRS, x, w, group, residual)
 
 
 # ----------------------------------------------------------------------------- ZeRO-3 linear
@@ -377,7 +377,7 @@ def zero3_linear(x: torch.Tensor, w_shard: torch.Tensor, group, sched: Optional[
     from ..ops import fused_comm
     if fused_comm.enabled(x, group):
         return fused_comm.zero3_linear(x, w_shard, group, sched, idx, rope, residual)
-    return _Zero3Linear.apply(x, w_shard, group, sched, idx, rope, residual)
+    return F.call(_Zero3Linear, x, w_shard, group, sched, idx, rope, residual)
 
 
 class _Zero3Embedding(Function):

@@ -106,7 +106,9 @@ class Trainer:
         with self._phase("forward"):
             loss = self.model(local_input_ids, local_position_ids, labels=local_target_ids,
                               global_tokens=self.global_tokens)
-        with self._phase("backward"):
+        # in this thread: handing the graph to autograd's device thread costs a wake-up per hand-over and nothing runs beside
+        # it (512 tokens of a small model: 1612 -> 1425 us a step)
+        with self._phase("backward"), torch.autograd.set_multithreading_enabled(False):
             loss.backward()
         # [loss, kernel status] summed over the ranks in one collective, before the optimizer looks at it
         dev = self.ctx.device
