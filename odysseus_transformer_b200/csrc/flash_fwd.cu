@@ -22,6 +22,8 @@
 //
 // q [Tq, H, 128], k/v [Tk, Hkv, 128] with arbitrary row pitch; out [Tq, H, 128] bf16; lse [H, Tq] fp32
 // (natural log).  causal requires Tq == Tk (row i sees keys 0..i).
+#include <type_traits>
+
 #include "ody_kernels.h"
 #include "sm100.cuh"
 #include "peer_comm.cuh"
@@ -323,11 +325,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const float sl2 = scale * 1.4426950408889634f;
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < nt; ++j) {
+    // Only a tile's last block can hold masked keys (the diagonal, the end of the keys): all others run an instance without
+    // the masks (8192 tokens x 32 heads 494 -> 486 us, 32768 x 4 913 -> 896).
+    auto block = [&](int j, auto masked) -> bool {
       const bool tr = blockIdx.x == 0 && (threadIdx.x == 128 || threadIdx.x == 256);
       ODY_FWD_STAMP(tr, j, t * 5 + 0);
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[t], j & 1, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
-      if (!ok) break;
+      if (!ok) return false;
       ODY_FWD_STAMP(tr, j, t * 5 + 1);
       tc_fence_after();
       uint32_t sv[128];
@@ -337,16 +341,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tmem_ld_32x32(col_s + 96, sv + 96);
       tmem_ld_wait();
       ODY_FWD_STAMP(tr, j, t * 5 + 2);
-      const int kv0 = (b0 + j) * BN;
-      if (b0 + j == diag) {
+      if constexpr (decltype(masked)::value) {
+        const int kv0 = (b0 + j) * BN;
+        if (b0 + j == diag) {
 #pragma unroll
-        for (int c = 0; c < 128; ++c)
-          if (c > r) sv[c] = 0xff800000u;               // -inf
-      }
-      if (kv0 + BN > Tk) {
+          for (int c = 0; c < 128; ++c)
+            if (c > r) sv[c] = 0xff800000u;               // -inf
+        }
+        if (kv0 + BN > Tk) {
 #pragma unroll
-        for (int c = 0; c < 128; ++c)
-          if (kv0 + c >= Tk) sv[c] = 0xff800000u;
+          for (int c = 0; c < 128; ++c)
+            if (kv0 + c >= Tk) sv[c] = 0xff800000u;
+        }
       }
       // One pass over the 128 scores: exponentials against the maximum in use (packed pairs, x = s * scale * log2(e) - m),
       // P back over S in four 32-column pieces, the row sum, and - on the side, off the dependent chain - the row maximum
@@ -422,7 +428,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_before();
       mbar_arrive(&bars->p_full[t]);
       ODY_FWD_STAMP(tr, j, t * 5 + 4);
-    }
+      return true;
+    };
+    for (int j = 0; j + 1 < nt; ++j)
+      if (!block(j, std::false_type())) break;
+    if (ok && nt > 0) block(nt - 1, std::true_type());
     // epilogue: O / l -> bf16 -> swizzled smem (this tile's Q is dead by now) -> TMA store; lse
     if (ok && nt > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t], 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
     uint8_t* stage = sQ + t * TILE_BYTES;
