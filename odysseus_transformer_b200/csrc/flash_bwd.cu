@@ -197,14 +197,13 @@ struct SplitMaps {
   int rows;     // 0 = unused
 };
 
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
-                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                      const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV,
-                      const uint8_t* __restrict__ stat_tiles, int Tq, int Tk, int Tq_pad,
-                      int H, int Hkv, int causal, float scale, int* __restrict__ err, long long* __restrict__ dbg,
-                      const __grid_constant__ SplitMaps dk_split, const __grid_constant__ SplitMaps dv_split,
-                      const SplitPlan plan, float* __restrict__ part) {
+// One CTA of the dK/dV grid (flash_bwd_pair_kernel below runs it)
+__device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, const CUtensorMap& tmDO, const CUtensorMap& tmK,
+                                         const CUtensorMap& tmV, const CUtensorMap& tmDK, const CUtensorMap& tmDV,
+                                         const uint8_t* __restrict__ stat_tiles, int Tq, int Tk, int Tq_pad,
+                                         int H, int Hkv, int causal, float scale, int* __restrict__ err, long long* __restrict__ dbg,
+                                         const SplitMaps& dk_split, const SplitMaps& dv_split, const SplitPlan plan,
+                                         float* __restrict__ part) {
 #ifndef ODY_ATTN_TRACE
   dbg = nullptr;   // the clock-stamp timeline is a development aid: compiled out of the product kernels
 #endif
@@ -221,7 +220,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_kv_tiles = (Tk + BIG - 1) / BIG;
-  const int tile = blockIdx.x / plan.max_parts, z = blockIdx.x % plan.max_parts;
+  const int tile = cta / plan.max_parts, z = cta % plan.max_parts;
   const int kt = kv_tile_of(tile, num_kv_tiles, Hkv, causal), kvh = kv_head_of(tile, num_kv_tiles, Hkv, causal);
   const int kv0 = kt * BIG;
   const int G = H / Hkv;
@@ -300,7 +299,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const uint64_t q_mn0 = make_smem_desc(smem_u32(sQs), BLK_HALF, 1024), d_mn0 = make_smem_desc(smem_u32(sDs), BLK_HALF, 1024);
       const uint64_t ones_d = make_smem_desc_noswizzle(smem_u32(sOnes), 128, 256);
       const uint64_t stat_d0 = make_smem_desc_noswizzle(smem_u32(sStat), 128, 256);
-      const bool trace = dbg != nullptr && blockIdx.x == 0;
+      const bool trace = dbg != nullptr && cta == 0;
       // S^T(it) = K Q^T - lse / scale (per query column): waits for the Q block
       auto issue_s = [&](int it) -> bool {
         const int stage = it % STAGES;
@@ -386,7 +385,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int it = 0; it < total; ++it) {
       const uint32_t par = it & 1;
       const int qrow0 = (i0 + (u0 + it) % per_head) * BLK + hf * 64;
-      const bool strace = dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 128 && it < 48;
+      const bool strace = dbg != nullptr && cta == 0 && threadIdx.x == 128 && it < 48;
       // ---- part 1: S^T -> P^T
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 2] = clock64();                             // S^T(it) complete
@@ -997,13 +996,13 @@ constexpr int Q_SMEM_TOTAL = Q_SMEM_TILES + 256 + 1024;
 // TMEM columns: S 0..127, dP 128..255 (dS, bf16, overwrites the first 32 columns of each 64-key half), dQ 256..383, Q 384..447, dO 448..511
 constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DQ = 256, COL_QA = 384, COL_DOA = 448;
 
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* __restrict__ dog, int64_t q_row, int64_t do_row,
-                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                    const __grid_constant__ CUtensorMap tmDQ, const float* __restrict__ lse2_pad,
-                    const float* __restrict__ delta_pad, int Tq, int Tk, int Tq_pad, int H, int Hkv, int causal,
-                    float scale, int* __restrict__ err, const __grid_constant__ SplitMaps dq_split, const SplitPlan plan,
-                    float* __restrict__ part, long long* __restrict__ dbg) {
+// One CTA of the dQ grid
+__device__ __forceinline__ void dq_cta(const int cta, const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* __restrict__ dog,
+                                       int64_t q_row, int64_t do_row, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                                       const CUtensorMap& tmDQ, const float* __restrict__ lse2_pad,
+                                       const float* __restrict__ delta_pad, int Tq, int Tk, int Tq_pad, int H, int Hkv, int causal,
+                                       float scale, int* __restrict__ err, const SplitMaps& dq_split, const SplitPlan plan,
+                                       float* __restrict__ part, long long* __restrict__ dbg) {
 #ifndef ODY_ATTN_TRACE
   dbg = nullptr;   // the clock-stamp timeline is a development aid: compiled out of the product kernels
 #endif
@@ -1018,7 +1017,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_q_tiles = (Tq + BIG - 1) / BIG;
   // CTA order as in the forward: causal, the tiles of all heads that attend to the most blocks first
-  const int tile = blockIdx.x / plan.max_parts, z = blockIdx.x % plan.max_parts;
+  const int tile = cta / plan.max_parts, z = cta % plan.max_parts;
   const int qt = causal ? (num_q_tiles - 1 - tile / H) : tile % num_q_tiles;
   const int head = causal ? tile % H : tile / num_q_tiles, kvh = head / (H / Hkv);
   const int q0 = qt * BIG;
@@ -1083,7 +1082,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
       tc_fence_after();
       const uint64_t k_k0 = make_smem_desc(smem_u32(sKs), 16, 1024), v_k0 = make_smem_desc(smem_u32(sVs), 16, 1024);
       const uint64_t k_mn0 = make_smem_desc(smem_u32(sKs), BLK_HALF, 1024);
-      const bool trace = dbg != nullptr && blockIdx.x == 0;
+      const bool trace = dbg != nullptr && cta == 0;
       // S_h(it) = Q K_h^T over the 64 keys of half h, Q from TMEM
       auto issue_s = [&](int it, int h) -> bool {
         const int stage = it % K_STAGES;
@@ -1175,7 +1174,7 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
     for (int it = 0; it < total; ++it) {
       const uint32_t par = it & 1;
       const int kvb0 = (b0 + it) * BLK + hf * 64;
-      const bool strace = dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 128 && it < 48;
+      const bool strace = dbg != nullptr && cta == 0 && threadIdx.x == 128 && it < 48;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[hf], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 4] = clock64();                             // S(it) complete
       uint32_t sv[64];
@@ -1274,6 +1273,35 @@ flash_bwd_dq_kernel(const __nv_bfloat16* __restrict__ qg, const __nv_bfloat16* _
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
+// Both grids in one launch: CTAs 0 .. n_kv - 1 are the dK/dV grid, the others the dQ grid.  They share nothing but their inputs;
+// in one launch the dQ CTAs fill the SMs that the dK/dV grid's last wave leaves idle (4096 queries on 8192 keys, 32 heads on 8:
+// 512 dK/dV CTAs are 3.5 waves), and a small problem runs both side by side.  Backward of that case 1635 -> 1537 us, 2048
+// tokens x 32 heads 177 -> 173, 32768 x 4 2906 -> 2885, 8192 x 32 (many waves) unchanged.
+struct PairArgs {
+  CUtensorMap tmQ, tmDO, tmK, tmV, tmDK, tmDV, tmDQ;
+  SplitMaps dk_split, dv_split, dq_split;
+  SplitPlan kv_plan, q_plan;
+  const uint8_t* stat_tiles;
+  const float *lse2_pad, *delta_pad;
+  const __nv_bfloat16 *q, *dO;
+  int64_t q_row, do_row;
+  float *kv_part, *q_part;
+  long long* dbg;
+  int* err;
+  int n_kv, Tq, Tk, Tq_pad, H, Hkv, causal;
+  float scale;
+};
+constexpr int PAIR_SMEM_TOTAL = KV_SMEM_TOTAL > Q_SMEM_TOTAL ? KV_SMEM_TOTAL : Q_SMEM_TOTAL;
+__global__ void __launch_bounds__(NUM_THREADS, 1) flash_bwd_pair_kernel(const __grid_constant__ PairArgs a) {
+  if ((int)blockIdx.x < a.n_kv)
+    dkdv_cta(blockIdx.x, a.tmQ, a.tmDO, a.tmK, a.tmV, a.tmDK, a.tmDV, a.stat_tiles, a.Tq, a.Tk, a.Tq_pad, a.H, a.Hkv, a.causal,
+             a.scale, a.err, a.dbg, a.dk_split, a.dv_split, a.kv_plan, a.kv_part);
+  else
+    dq_cta((int)blockIdx.x - a.n_kv, a.q, a.dO, a.q_row, a.do_row, a.tmK, a.tmV, a.tmDQ, a.lse2_pad, a.delta_pad, a.Tq, a.Tk,
+           a.Tq_pad, a.H, a.Hkv, a.causal, a.scale, a.err, a.dq_split, a.q_plan, a.q_part,
+           a.dbg != nullptr ? a.dbg + 48 * 8 : nullptr);
+}
+
 }  // namespace bwd
 }  // namespace ody
 
@@ -1304,6 +1332,15 @@ static void bwd_plans(int Tq, int Tk, int H, int Hkv, int causal, ody::SplitUnit
   *pq = split_plan(*uq, nq, H, 1.1, 3.0, BIG * HD * 4);
 }
 
+static int64_t kv_part_bytes(const ody::SplitPlan& p, int Tk, int Hkv) {
+  using namespace ody::bwd;
+  return p.max_parts > 1 ? (int64_t)((Tk + BIG - 1) / BIG) * Hkv * p.max_parts * 2 * BIG * HD * 4 : 0;
+}
+static int64_t q_part_bytes(const ody::SplitPlan& p, int Tq, int H) {
+  using namespace ody::bwd;
+  return p.max_parts > 1 ? (int64_t)((Tq + BIG - 1) / BIG) * H * p.max_parts * BIG * HD * 4 : 0;
+}
+
 extern "C" int64_t ody_flash_bwd_split_bytes(int Tq, int Tk, int H, int Hkv, int causal) {
   using namespace ody;
   using namespace ody::bwd;
@@ -1311,9 +1348,7 @@ extern "C" int64_t ody_flash_bwd_split_bytes(int Tq, int Tk, int H, int Hkv, int
   SplitUnits ukv, uq;
   SplitPlan pkv, pq;
   bwd_plans(Tq, Tk, H, Hkv, causal, &ukv, &pkv, &uq, &pq);
-  const int64_t kv = pkv.max_parts > 1 ? (int64_t)((Tk + BIG - 1) / BIG) * Hkv * pkv.max_parts * 2 * BIG * HD * 4 : 0;
-  const int64_t dq = pq.max_parts > 1 ? (int64_t)((Tq + BIG - 1) / BIG) * H * pq.max_parts * BIG * HD * 4 : 0;
-  return kv > dq ? kv : dq;      // the two kernels run one after the other
+  return kv_part_bytes(pkv, Tk, Hkv) + q_part_bytes(pq, Tq, H);
 }
 
 extern "C" int64_t ody_flash_bwd_workspace_bytes(int Tq, int H) {
@@ -1380,9 +1415,7 @@ extern "C" int ody_flash_bwd_parts(const void* dO, const void* q, const void* k,
     return (int)cudaErrorInvalidValue;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(flash_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM_TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM_TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(flash_bwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_TOTAL);
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(flash_bwd_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM_TOTAL);
     if (e != cudaSuccess) return (int)e;
@@ -1416,13 +1449,13 @@ extern "C" int ody_flash_bwd_parts(const void* dO, const void* q, const void* k,
     pkv = pq = SplitPlan();
   const int kv_tiles = (Tk + BIG - 1) / BIG, q_tiles = (Tq + BIG - 1) / BIG;
   const int64_t ctas_kv = (int64_t)kv_tiles * Hkv * pkv.max_parts, ctas_q = (int64_t)q_tiles * H * pq.max_parts;
-  if (ctas_kv > INT_MAX || ctas_q > INT_MAX) return (int)cudaErrorInvalidValue;
-  const dim3 gkv((unsigned)ctas_kv), gq((unsigned)ctas_q);
+  if (ctas_kv + ctas_q > INT_MAX) return (int)cudaErrorInvalidValue;
+  const int64_t kv_bytes = kv_part_bytes(pkv, Tk, Hkv);
   if (g_bwd_variant != 1) {
     float* dq_acc = (float*)(stat_tiles + (int64_t)H * (Tpad / BLK) * STAT_BYTES);
     cudaError_t e = cudaMemsetAsync(dq_acc, 0, (size_t)H * Tpad * HD * sizeof(float), st);
     if (e != cudaSuccess) return (int)e;
-    flash_bwd_fused_kernel<<<gkv, NUM_THREADS, F_SMEM_TOTAL, st>>>(tQ, tDO, tK, tV, tDK, tDV, stat_tiles, dq_acc, Tq, Tk, Tpad, H, Hkv,
+    flash_bwd_fused_kernel<<<dim3((unsigned)ctas_kv), NUM_THREADS, F_SMEM_TOTAL, st>>>(tQ, tDO, tK, tV, tDK, tDV, stat_tiles, dq_acc, Tq, Tk, Tpad, H, Hkv,
                                                                    causal, scale, err, sk, sv);
     DqDests dd;
     memset(&dd, 0, sizeof(dd));
@@ -1432,17 +1465,25 @@ extern "C" int ody_flash_bwd_parts(const void* dO, const void* q, const void* k,
                                                                         dq_row, Tq, Tpad, H, scale);
     return (int)cudaGetLastError();
   }
-  flash_bwd_dkdv_kernel<<<gkv, NUM_THREADS, KV_SMEM_TOTAL, st>>>(tQ, tDO, tK, tV, tDK, tDV, stat_tiles, Tq, Tk,
-                                                                 Tpad, H, Hkv, causal, scale, err, g_bwd_trace, sk, sv, pkv, (float*)parts);
+  PairArgs pa;
+  memset(&pa, 0, sizeof(pa));
+  pa.tmQ = tQ; pa.tmDO = tDO; pa.tmK = tK; pa.tmV = tV; pa.tmDK = tDK; pa.tmDV = tDV; pa.tmDQ = tDQ;
+  pa.dk_split = sk; pa.dv_split = sv; pa.dq_split = sq;
+  pa.kv_plan = pkv; pa.q_plan = pq;
+  pa.stat_tiles = stat_tiles; pa.lse2_pad = lse2_pad; pa.delta_pad = delta_pad;
+  pa.q = (const __nv_bfloat16*)q; pa.dO = (const __nv_bfloat16*)dO; pa.q_row = q_row; pa.do_row = do_row;
+  pa.kv_part = (float*)parts;
+  pa.q_part = (float*)((uint8_t*)parts + kv_bytes);
+  pa.dbg = g_bwd_trace; pa.err = err;
+  pa.n_kv = (int)ctas_kv; pa.Tq = Tq; pa.Tk = Tk; pa.Tq_pad = Tpad; pa.H = H; pa.Hkv = Hkv; pa.causal = causal; pa.scale = scale;
+  flash_bwd_pair_kernel<<<(unsigned)(ctas_kv + ctas_q), NUM_THREADS, PAIR_SMEM_TOTAL, st>>>(pa);
   if (pkv.max_parts > 1) {
     const PartDests d = {{(__nv_bfloat16*)dv, (__nv_bfloat16*)dk}, {dv_row, dk_row}};
-    sum_parts_kernel<2><<<dim3(kv_tiles, Hkv, BIG / 16), 256, 0, st>>>((const float*)parts, d, Tk, Hkv, ukv, pkv);
+    sum_parts_kernel<2><<<dim3(kv_tiles, Hkv, BIG / 16), 256, 0, st>>>(pa.kv_part, d, Tk, Hkv, ukv, pkv);
   }
-  flash_bwd_dq_kernel<<<gq, NUM_THREADS, Q_SMEM_TOTAL, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)dO, q_row, do_row, tK, tV, tDQ, lse2_pad, delta_pad, Tq, Tk, Tpad, H,
-                                                             Hkv, causal, scale, err, sq, pq, (float*)parts, g_bwd_trace ? g_bwd_trace + 48 * 8 : nullptr);
   if (pq.max_parts > 1) {
     const PartDests d = {{(__nv_bfloat16*)dq, nullptr}, {dq_row, 0}};
-    sum_parts_kernel<1><<<dim3(q_tiles, H, BIG / 16), 256, 0, st>>>((const float*)parts, d, Tq, H, uq, pq);
+    sum_parts_kernel<1><<<dim3(q_tiles, H, BIG / 16), 256, 0, st>>>(pa.q_part, d, Tq, H, uq, pq);
   }
   return (int)cudaGetLastError();
 }
