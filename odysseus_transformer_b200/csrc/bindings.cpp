@@ -125,7 +125,8 @@ std::vector<at::Tensor> add_rmsnorm_fwd(const at::Tensor& x, const at::Tensor& d
 }
 
 std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor& dy, const at::Tensor& x, const at::Tensor& w,
-                                    const at::Tensor& rstd, const c10::optional<at::Tensor>& ds) {
+                                    const at::Tensor& rstd, const c10::optional<at::Tensor>& ds,
+                                    const c10::optional<at::Tensor>& dw_out) {
   check_bf16(dy, "dy"); check_bf16(x, "x"); check_bf16(w, "w");
   ody_req(dy.is_contiguous() && x.is_contiguous() && w.is_contiguous(), "rmsnorm_bwd: contiguous inputs required");
   ody_req(x.dim() >= 1 && x.size(-1) > 0, "rmsnorm_bwd: x must have a non-empty last dim");
@@ -138,7 +139,12 @@ std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor& dy, const at::Tensor& x, c
           "rmsnorm_bwd: all tensors must be on x's device");
   c10::cuda::CUDAGuard guard(x.device());
   auto dx = at::empty_like(x);
-  auto dw = at::empty({dim}, x.options().dtype(at::kFloat));
+  if (dw_out.has_value()) {
+    check_bf16(dw_out.value(), "dw_out");
+    ody_req(dw_out.value().is_contiguous() && dw_out.value().numel() == dim && dw_out.value().get_device() == x.get_device(),
+            "rmsnorm_bwd: dw_out must be a contiguous bf16 tensor of x's last dim");
+  }
+  auto dw = dw_out.has_value() ? dw_out.value() : at::empty({dim}, x.options().dtype(at::kFloat));
   const int nb = ody_rmsnorm_bwd_blocks(rows, (int)dim);
   auto partial = at::empty({nb, dim}, x.options().dtype(at::kFloat));
   const void* dsp = nullptr;
@@ -148,8 +154,9 @@ std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor& dy, const at::Tensor& x, c
             "rmsnorm_bwd: ds must match x");
     dsp = ds.value().data_ptr();
   }
-  ODY_CHECK(ody_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dsp, dx.data_ptr(),
-                            dw.data_ptr<float>(), partial.data_ptr<float>(), rows, (int)dim, cur_stream()), "rmsnorm_bwd");
+  ODY_CHECK(ody_rmsnorm_bwd_to(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dsp, dx.data_ptr(),
+                               dw.data_ptr(), dw_out.has_value() ? 1 : 0, partial.data_ptr<float>(), rows, (int)dim,
+                               cur_stream()), "rmsnorm_bwd");
   g_launches += 2;
   return {dx, dw};
 }
@@ -417,7 +424,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_set_variant", [](int64_t v) { ODY_CHECK(ody_gemm_set_variant((int)v), "gemm_set_variant (0 auto, 1 one CTA, 2 CTA pairs)"); });
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("add_rmsnorm_fwd", &add_rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("rstd"), py::arg("ds"),
+        py::arg("dw_out") = py::none());
   m.def("rope_tables", &rope_tables);
   m.def("rope_inplace_", &rope_inplace_);
   m.def("rope_grouped_", &rope_grouped_);

@@ -273,7 +273,11 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1) rmsnorm_bwd_ring_k(const
 // out[c] = sum over the nblocks rows of partial[nblocks, dim].  Block = 32 columns x 32 row slices: the grid has dim / 32
 // blocks, and a thread adds about ten of the 296 rows - with 8 slices its chain of dependent loads was four times as long:
 // 7.8 -> 3.3 us at dim 1024, 10.6 -> 4.9 at 4096.
-__global__ void __launch_bounds__(1024) colsum_k(const float* __restrict__ partial, float* __restrict__ out, int nblocks, int dim) {
+// OUT: fp32, or bf16 for a gradient that goes straight to where the optimizer reads it.
+__device__ __forceinline__ void store_sum(float* p, float v) { *p = v; }
+__device__ __forceinline__ void store_sum(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
+template <typename OUT>
+__global__ void __launch_bounds__(1024) colsum_k(const float* __restrict__ partial, OUT* __restrict__ out, int nblocks, int dim) {
   __shared__ float red[32][33];
   const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(1024) colsum_k(const float* __restrict__ parti
   // warp `slice` adds up column `slice` of the block
   const float t = warp_sum(red[cx][slice]);
   const int co = blockIdx.x * 32 + slice;
-  if (cx == 0 && co < dim) out[co] = t;
+  if (cx == 0 && co < dim) store_sum(out + co, t);
 }
 
 // ------------------------------------------------------------------------------------------- RoPE
@@ -699,6 +703,11 @@ static int launch_norm_ring(const void* dy, const void* x, const void* w, const 
 
 extern "C" int ody_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* ds,
                                void* dx, float* dw, float* dw_partial, int64_t rows, int dim, cudaStream_t st) {
+  return ody_rmsnorm_bwd_to(dy, x, w, rstd, ds, dx, dw, 0, dw_partial, rows, dim, st);
+}
+
+extern "C" int ody_rmsnorm_bwd_to(const void* dy, const void* x, const void* w, const float* rstd, const void* ds, void* dx,
+                                  void* dw, int dw_bf16, float* dw_partial, int64_t rows, int dim, cudaStream_t st) {
   if (dim % 8 != 0 || dim > 256 * 8 * 8) return (int)cudaErrorInvalidValue;
   const int nb = ody_rmsnorm_bwd_blocks(rows, dim);
   int e = 0;
@@ -711,7 +720,10 @@ extern "C" int ody_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
     rmsnorm_bwd_k<8><<<nb, 256, 0, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)ds,
                                          (bf16*)dx, dw_partial, rows, dim);
   if (e) return e;
-  colsum_k<<<blocks_for(dim, 32), 1024, 0, st>>>(dw_partial, dw, nb, dim);
+  if (dw_bf16)
+    colsum_k<bf16><<<blocks_for(dim, 32), 1024, 0, st>>>(dw_partial, (bf16*)dw, nb, dim);
+  else
+    colsum_k<float><<<blocks_for(dim, 32), 1024, 0, st>>>(dw_partial, (float*)dw, nb, dim);
   return last_err();
 }
 

@@ -17,6 +17,9 @@ int ody_rmsnorm_fwd(const void* x, const void* delta, const void* w, void* sum_o
 int ody_rmsnorm_bwd_blocks(int64_t rows, int dim);
 int ody_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* ds, void* dx,
                     float* dw, float* dw_partial, int64_t rows, int dim, cudaStream_t stream);
+// the same with dw as fp32 (dw_bf16 = 0) or bf16 [dim]
+int ody_rmsnorm_bwd_to(const void* dy, const void* x, const void* w, const float* rstd, const void* ds, void* dx, void* dw,
+                       int dw_bf16, float* dw_partial, int64_t rows, int dim, cudaStream_t stream);
 
 // ---- RoPE (rotate-half).  positions int64 [T]; tables fp32 [T, hd/2].
 int ody_rope_tables(const int64_t* positions, float* cos_out, float* sin_out, int64_t T, int head_dim, float theta,

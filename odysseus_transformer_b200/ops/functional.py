@@ -184,6 +184,18 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 # ----------------------------------------------------------------------------- RMSNorm
 
 
+def _rmsnorm_bwd_native(dy, x, w, rstd, ds):
+    """(dx, gradient of w for autograd or None): the weight gradient goes straight to ``main_grad`` where it can."""
+    mg = getattr(w, "main_grad", None)
+    if (mg is not None and not getattr(w, "_grad_written", False) and mg.dtype == torch.bfloat16 and mg.is_contiguous()
+            and mg.device == x.device):
+        dx, _ = native.lib().rmsnorm_bwd(dy, x, w, rstd, ds, mg)
+        w._grad_written = True
+        return dx, None
+    dx, dw = native.lib().rmsnorm_bwd(dy, x, w, rstd, ds)
+    return dx, deliver_grad(w, dw)
+
+
 class _RMSNorm(Function):
     @staticmethod
     def forward(ctx, x, w, eps):
@@ -199,9 +211,8 @@ class _RMSNorm(Function):
         x, w, rstd = ctx.saved_tensors
         dy = dy.contiguous()
         if native.use_native(x):
-            dx, dw = native.lib().rmsnorm_bwd(dy, x, w, rstd, None)
-        else:
-            dx, dw = R.rmsnorm_bwd(dy, x, w, rstd)
+            return *_rmsnorm_bwd_native(dy, x, w, rstd, None), None
+        dx, dw = R.rmsnorm_bwd(dy, x, w, rstd)
         return dx, deliver_grad(w, dw), None
 
 
@@ -227,10 +238,10 @@ class _AddRMSNorm(Function):
         s, w, rstd = ctx.saved_tensors
         dy = dy.contiguous()
         if native.use_native(s):
-            dx, dw = native.lib().rmsnorm_bwd(dy, s, w, rstd, ds.contiguous())
-        else:
-            dx, dw = R.rmsnorm_bwd(dy, s, w, rstd)
-            dx = (dx.float() + ds.float()).to(dx.dtype)
+            dx, dw = _rmsnorm_bwd_native(dy, s, w, rstd, ds.contiguous())
+            return dx, dx, dw, None
+        dx, dw = R.rmsnorm_bwd(dy, s, w, rstd)
+        dx = (dx.float() + ds.float()).to(dx.dtype)
         return dx, dx, deliver_grad(w, dw), None
 
 
@@ -257,10 +268,9 @@ class _RMSNormKeep(Function):
         s, w, rstd = ctx.saved_tensors
         dy = dy.contiguous()
         if native.use_native(s):
-            dx, dw = native.lib().rmsnorm_bwd(dy, s, w, rstd, ds.contiguous())
-        else:
-            dx, dw = R.rmsnorm_bwd(dy, s, w, rstd)
-            dx = (dx.float() + ds.float()).to(dx.dtype)
+            return *_rmsnorm_bwd_native(dy, s, w, rstd, ds.contiguous()), None
+        dx, dw = R.rmsnorm_bwd(dy, s, w, rstd)
+        dx = (dx.float() + ds.float()).to(dx.dtype)
         return dx, deliver_grad(w, dw), None
 
 

@@ -619,3 +619,17 @@ def test_gemm_split_k_rope(lib, M):
     lib.gemm_set_variant(0)
     _check_status(lib)
     assert ((y.float() - y1.float()).norm() / y1.float().norm()).item() < 2e-3
+
+
+@pytest.mark.parametrize("rows,dim", [(1, 8), (700, 1024), (33, 4096)])
+def test_rmsnorm_bwd_weight_gradient_in_bf16(lib, rows, dim):
+    """The weight gradient written in bf16 where the optimizer reads it is the fp32 one rounded once."""
+    x, w, dy, ds = _rand(rows, dim), _rand(dim) + 1, _rand(rows, dim), _rand(rows, dim)
+    _, rstd = lib.rmsnorm_fwd(x, w, 1e-5)
+    dx, dw = lib.rmsnorm_bwd(dy, x, w, rstd, ds)
+    out = torch.full((dim,), float("nan"), device="cuda", dtype=torch.bfloat16)
+    dx2, _ = lib.rmsnorm_bwd(dy, x, w, rstd, ds, out)
+    _check_status(lib)
+    assert torch.equal(dx, dx2) and torch.equal(out, dw.to(torch.bfloat16))
+    with pytest.raises(RuntimeError):
+        lib.rmsnorm_bwd(dy, x, w, rstd, ds, out[: dim // 2])
