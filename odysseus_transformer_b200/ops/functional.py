@@ -553,10 +553,10 @@ class _Embedding(Function):
         w = ctx.w
         mg = getattr(w, "main_grad", None)
         if mg is not None and not getattr(w, "_grad_written", False):
-            dy = dy.to(mg.dtype)
+            dy = dy.to(mg.dtype).contiguous()
             if (native.use_native(mg) and mg.dim() == 2 and dy.dim() == 2 and ids.dim() == 1 and ids.dtype == torch.int64
-                    and mg.is_contiguous() and mg.shape[1] % 8 == 0 and mg.data_ptr() % 16 == 0):
-                native.lib().embedding_grad_(dy.contiguous(), ids.contiguous(), mg)
+                    and mg.is_contiguous() and mg.shape[1] % 8 == 0 and (mg.data_ptr() | dy.data_ptr()) % 16 == 0):
+                native.lib().embedding_grad_(dy, ids.contiguous(), mg)
             else:
                 mg.zero_()
                 mg.index_add_(0, ids, dy)
