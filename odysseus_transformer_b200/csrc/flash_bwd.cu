@@ -1,8 +1,8 @@
 // Attention backward for sm_100a (head_dim 128, bf16, GQA): dQ, dK, dV from (dO, Q, K, V, O, LSE).
 //
 // The reference gets this from flash_attn_2_cuda.bwd through autograd (reference
-// decoder/odysseus.py:256-263; its ring dependency calls the same kernel per block).  Here it is three
-// kernels built on tcgen05 / TMEM / TMA:
+// decoder/odysseus.py:256-263; its ring dependency calls the same kernel per block).  Here it is a small
+// kernel for the statistics and one launch with two kinds of CTAs built on tcgen05 / TMEM / TMA:
 //
 //   prep   : -delta[h,t] = -sum_d dO*O, and -LSE in the exp2 domain (negated so the kernels can fuse them into packed
 //            fma / add instructions), both padded to 128 rows.
