@@ -41,7 +41,12 @@ constexpr int EPI_BYTES = BM * EPI_COLS * 2;     // 16 KB
 constexpr int SMEM_TILES = STAGES * STAGE_BYTES + 2 * EPI_BYTES;
 constexpr int SMEM_TOTAL = SMEM_TILES + 256 + 1024;
 constexpr int NUM_THREADS = 192;                 // TMA warp, MMA warp, 4 epilogue warps
-constexpr int GROUP_M = 8;                       // raster: 8 pair-tiles (2048 rows) share their B columns in L2
+// Raster: GROUP_M pair-tiles (4096 rows) share their B columns in L2, and a CTA pair walks the k-blocks of every other tile
+// backwards, so that the part of the shared rows of A that the wave before read last is read first again, while the L2
+// still has it.  Long products run at the power cap, where what is not fetched twice comes back as clock: [8192, 22016] from K
+// = 4096 1337 -> 1362 TFLOP/s back to back (8 tiles, all forwards -> this), [12288, 28672] 1335 -> 1364, one product alone 1605
+// -> 1636; 4 or 32 tiles to a group are 5 - 10 % slower than 8.
+constexpr int GROUP_M = 16;
 
 struct Bars {
   uint64_t full[STAGES];        // used in the even CTA only
@@ -184,7 +189,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint32_t phase = 0;
       int issued = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+      bool backwards = false;
+      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs, backwards = !backwards) {
         int tm, tn;
         tile_coords(tile, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * 2 * BM + (int)rank * BM;        // this CTA's rows of A
@@ -195,7 +201,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           uint8_t* sB = sA + A_BYTES;
           if (rank == 0) mbar_expect_tx(&bars->full[stage], 2 * STAGE_BYTES);     // the bytes of both CTAs
           const uint32_t full0 = map_to_cta(&bars->full[stage], 0);
-          const int k0 = kb * BK;
+          const int k0 = (backwards ? kblocks - 1 - kb : kb) * BK;
           if (!A_MN) {
             tma2_load_2d(sA, &tmA, k0, m0, full0);
           } else if (mn3d & 1) {
