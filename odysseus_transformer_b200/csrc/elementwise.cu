@@ -6,6 +6,8 @@
 // Every kernel here moves 16 bytes per thread per access and touches each operand once.
 #include <string.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "ody_kernels.h"
 
@@ -690,11 +692,13 @@ template <int NV, bool DS>
 static int launch_norm_ring(const void* dy, const void* x, const void* w, const float* rstd, const void* ds, void* dx,
                             float* dw_partial, int64_t rows, int dim, int nb, cudaStream_t st) {
   constexpr int SMEM = NORM_STAGES * (DS ? 3 : 2) * NV * 256 * 16;
-  static bool configured = false;
-  if (!configured) {
+  static std::atomic<uint64_t> configured{0};      // one bit per device: the attribute belongs to the device's copy of the kernel
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev > 63 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
     const cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_ring_k<NV, DS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
-    configured = true;
+    if (dev <= 63) configured.fetch_or(1ull << dev, std::memory_order_relaxed);
   }
   rmsnorm_bwd_ring_k<NV, DS><<<nb, 256, SMEM, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)ds,
                                                     (bf16*)dx, dw_partial, rows, dim);
