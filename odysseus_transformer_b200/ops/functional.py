@@ -554,8 +554,10 @@ class _Embedding(Function):
         mg = getattr(w, "main_grad", None)
         if mg is not None and not getattr(w, "_grad_written", False):
             dy = dy.to(mg.dtype).contiguous()
-            if (native.use_native(mg) and mg.dim() == 2 and dy.dim() == 2 and ids.dim() == 1 and ids.dtype == torch.int64
-                    and mg.is_contiguous() and mg.shape[1] % 8 == 0 and (mg.data_ptr() | dy.data_ptr()) % 16 == 0):
+            # the kernel adds the rows that tokens share in no fixed order; index_add_ has an ordered form for who asks for it
+            if (native.use_native(mg) and not torch.are_deterministic_algorithms_enabled() and mg.dim() == 2
+                    and dy.dim() == 2 and ids.dim() == 1 and ids.dtype == torch.int64 and mg.is_contiguous()
+                    and mg.shape[1] % 8 == 0 and (mg.data_ptr() | dy.data_ptr()) % 16 == 0):
                 native.lib().embedding_grad_(dy, ids.contiguous(), mg)
             else:
                 mg.zero_()
