@@ -450,14 +450,31 @@ def cross_entropy_sum(logits: torch.Tensor, targets: torch.Tensor, scale: float 
     return _CrossEntropySum.apply(logits, targets, scale, ignore_index)
 
 
-def _scaled(g: torch.Tensor, scale: torch.Tensor, out: Optional[torch.Tensor]) -> torch.Tensor:
-    """``g * scale`` for a one-element device tensor ``scale``, into ``out`` when given."""
-    if (native.use_native(g) and g.is_contiguous() and g.numel() % 8 == 0 and g.data_ptr() % 16 == 0 and scale.is_cuda
-            and (out is None or (out.is_contiguous() and out.dtype == g.dtype and out.data_ptr() % 16 == 0))):
-        out = torch.empty_like(g) if out is None else out
-        native.lib().scale_into_(out, g, scale.detach().float().reshape(1))
-        return out
-    return torch.mul(g, scale.to(g.dtype)) if out is None else torch.mul(g, scale.to(g.dtype), out=out)
+def _kernel_scales(g: torch.Tensor, scale: torch.Tensor) -> bool:
+    """Whether ``scale_into_`` may form ``g * scale`` in a backward: not while that backward is recorded (``create_graph``) or
+    runs for several incoming gradients at once, where ``scale`` is more than its value."""
+    return (native.use_native(g) and g.is_contiguous() and g.numel() % 8 == 0 and g.data_ptr() % 16 == 0 and scale.is_cuda
+            and not torch.is_grad_enabled() and not torch._C._functorch.is_legacy_batchedtensor(scale))
+
+
+def _scaled(g: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
+    """``g * scale`` for a one-element device tensor ``scale``."""
+    if not _kernel_scales(g, scale):
+        return g * scale.to(g.dtype)
+    out = torch.empty_like(g)
+    native.lib().scale_into_(out, g, scale.float().reshape(1))
+    return out
+
+
+def _deliver_scaled(w: torch.Tensor, g: torch.Tensor, scale: torch.Tensor) -> Optional[torch.Tensor]:
+    """``deliver_grad(w, g * scale)``, scaled on its way to the optimizer's buffer (one pass over [V/n, d]) where a kernel can."""
+    mg = getattr(w, "main_grad", None)
+    if (mg is None or getattr(w, "_grad_written", False) or mg.dtype != g.dtype or mg.shape != g.shape or mg.device != g.device
+            or not mg.is_contiguous() or mg.data_ptr() % 16 or not _kernel_scales(g, scale)):
+        return deliver_grad(w, _scaled(g, scale))
+    native.lib().scale_into_(mg, g, scale.float().reshape(1))
+    w._grad_written = True
+    return None
 
 
 class _ChunkedLinearCrossEntropy(Function):
@@ -514,17 +531,9 @@ class _ChunkedLinearCrossEntropy(Function):
         saved = list(ctx.saved_tensors)
         dh = saved.pop(0) if ctx.have[0] else None
         dw = saved.pop(0) if ctx.have[1] else None
-        gw = None
         if dh is not None:
-            dh = _scaled(dh, dloss, None)
-        if dw is not None:
-            w = ctx.w
-            mg = getattr(w, "main_grad", None)
-            if mg is not None and mg.dtype == dw.dtype and not getattr(w, "_grad_written", False):
-                _scaled(dw, dloss, mg)                     # scaled on its way to the optimizer: one pass over [V/n, d]
-                w._grad_written = True
-            else:
-                gw = deliver_grad(w, _scaled(dw, dloss, None))
+            dh = _scaled(dh, dloss)
+        gw = _deliver_scaled(ctx.w, dw, dloss) if dw is not None else None
         return dh, gw, None, None, None, None, None
 
 

@@ -51,3 +51,44 @@ def test_embedding_gradient_obeys_deterministic_algorithms(recorder, warn_only):
     finally:
         torch.use_deterministic_algorithms(before, warn_only=warn)
     assert recorder.calls == []
+
+
+def _chunked_loss(device="cpu", dtype=torch.float32):
+    g = torch.Generator().manual_seed(0)
+    h = torch.randn(6, 16, generator=g).to(device, dtype).requires_grad_(True)
+    w = torch.randn(24, 16, generator=g).to(device, dtype).requires_grad_(True)
+    t = torch.randint(24, (6,), generator=g).to(device)
+    return h, w, lambda: F.linear_cross_entropy_sum(h, w, t, 0.5, None, 4)
+
+
+def check_recorded_backward(device, dtype):
+    """The incoming gradient is a tensor like any other: a backward that is itself recorded goes through it."""
+    h, w, loss = _chunked_loss(device, dtype)
+    dh, dw = torch.autograd.grad(loss(), (h, w))
+    for main_grad in (False, True):
+        if main_grad:
+            w.main_grad = torch.zeros_like(w)
+        s = torch.tensor(2.0, device=device, requires_grad=True)
+        (g,) = torch.autograd.grad(loss() * s, h, create_graph=True) if main_grad else \
+            torch.autograd.grad(loss() * s, (h, w), create_graph=True)[:1]
+        torch.testing.assert_close(g.detach(), 2 * dh)
+        (ds,) = torch.autograd.grad(g.float().sum(), s)
+        torch.testing.assert_close(ds, dh.float().sum(), rtol=1e-2, atol=1e-3)
+    del w.main_grad
+    # several incoming gradients at once
+    seeds = torch.tensor([1.0, -2.0, 0.5], device=device)
+    many = torch.autograd.grad(loss(), (h, w), seeds, is_grads_batched=True)
+    for got, one in zip(many, (dh, dw)):
+        torch.testing.assert_close(got, torch.stack([one * c for c in seeds.to(dtype)]))
+
+
+def test_recorded_backward_of_the_chunked_loss():
+    check_recorded_backward("cpu", torch.float32)
+
+
+def test_chunked_loss_refuses_a_gradient_buffer_of_another_shape():
+    h, w, loss = _chunked_loss()
+    w.main_grad = torch.zeros(w.numel())
+    with pytest.raises(RuntimeError):
+        loss().backward()
+    assert w.main_grad.shape == (w.numel(),)
