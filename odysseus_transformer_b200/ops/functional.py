@@ -187,8 +187,8 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 def _rmsnorm_bwd_native(dy, x, w, rstd, ds):
     """(dx, gradient of w for autograd or None): the weight gradient goes straight to ``main_grad`` where it can."""
     mg = getattr(w, "main_grad", None)
-    if (mg is not None and not getattr(w, "_grad_written", False) and mg.dtype == torch.bfloat16 and mg.is_contiguous()
-            and mg.device == x.device):
+    if (mg is not None and not getattr(w, "_grad_written", False) and mg.dtype == torch.bfloat16 and mg.shape == w.shape
+            and mg.is_contiguous() and mg.device == x.device):
         dx, _ = native.lib().rmsnorm_bwd(dy, x, w, rstd, ds, mg)
         w._grad_written = True
         return dx, None

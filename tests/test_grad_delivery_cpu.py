@@ -92,3 +92,29 @@ def test_chunked_loss_refuses_a_gradient_buffer_of_another_shape():
     with pytest.raises(RuntimeError):
         loss().backward()
     assert w.main_grad.shape == (w.numel(),)
+
+
+@pytest.mark.parametrize("fn", ["rmsnorm", "add_rmsnorm", "rmsnorm_keep"])
+def test_norm_refuses_a_gradient_buffer_of_another_shape(recorder, fn):
+    """What ``deliver_grad`` refuses - a buffer that the gradient does not broadcast to - the kernel's route refuses too."""
+    z = torch.zeros
+    recorder.rmsnorm_fwd = lambda x, w, eps: (z(4, 8), z(4))
+    recorder.add_rmsnorm_fwd = lambda x, d, w, eps: (z(4, 8), z(4, 8), z(4))
+
+    def bwd(dy, x, w, rstd, ds, dw_out=None):
+        recorder.calls.append(dw_out is not None)
+        return z(4, 8), z(8)
+    recorder.rmsnorm_bwd = bwd
+    x = torch.randn(4, 8, requires_grad=True)
+    for shape, ok in (((8,), True), ((8, 1), False)):
+        w = torch.ones(8, dtype=torch.bfloat16, requires_grad=True)
+        w.main_grad = torch.zeros(shape, dtype=torch.bfloat16)
+        args = (x, x.detach(), w, 1e-5) if fn == "add_rmsnorm" else (x, w, 1e-5)
+        y = getattr(F, fn)(*args)
+        y = y if torch.is_tensor(y) else y[0] + y[1]
+        if ok:
+            y.sum().backward()
+        else:
+            with pytest.raises(RuntimeError):
+                y.sum().backward()
+    assert recorder.calls == [True, False]
