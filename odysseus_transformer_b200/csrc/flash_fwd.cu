@@ -22,6 +22,7 @@
 //
 // q [Tq, H, 128], k/v [Tk, Hkv, 128] with arbitrary row pitch; out [Tq, H, 128] bf16; lse [H, Tq] fp32
 // (natural log).  causal requires Tq == Tk (row i sees keys 0..i).
+#include <float.h>
 #include <type_traits>
 
 #include "ody_kernels.h"
@@ -397,7 +398,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], __uint_as_float(sv[c + i]));
         }
-        m_used = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
+        // finite also when every score is -inf (then all exponentials are 0 and a later block takes over): the difference of
+        // two infinities would make the row NaN although other blocks - or, of a split tile, other parts - are finite
+        m_used = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2, -FLT_MAX);
         ODY_FWD_STAMP(tr, j, t * 5 + 3);
         exp_pass();
       } else {
