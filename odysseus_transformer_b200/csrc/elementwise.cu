@@ -4,6 +4,7 @@
 // The reference gets these from unfused ATen elementwise kernels inside HF Llama, a Triton loss from
 // flash-attn and torch.optim.AdamW (reference train.py:167,173; decoder/odysseus.py:210-213,293-295).
 // Every kernel here moves 16 bytes per thread per access and touches each operand once.
+#include <float.h>
 #include <string.h>
 
 #include <atomic>
@@ -402,7 +403,8 @@ __device__ __forceinline__ float row_lse(const bf16* lr, int64_t V, float* red) 
     float mx = f[0];
 #pragma unroll
     for (int j = 1; j < 8; ++j) mx = fmaxf(mx, f[j]);
-    const float mn = fmaxf(m, mx);
+    // finite also when all logits so far are -inf: their exponentials are 0 then, not those of a difference of infinities
+    const float mn = fmaxf(fmaxf(m, mx), -FLT_MAX);
     float acc = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc += __expf(f[j] - mn);

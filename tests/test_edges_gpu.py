@@ -44,3 +44,23 @@ def test_attention_forward_with_keys_out_of_reach(lib, Tq, Tk, H, lo, hi):
     orf, lser = R.attn_fwd(q, k, v, False, 1.0 / math.sqrt(128))
     torch.testing.assert_close(lse, lser, rtol=1e-3, atol=2e-3)
     torch.testing.assert_close(o.float(), orf.float(), rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("lo,hi", [(4096, 4104), (8000, 8192), (0, 64), (4096, 32000)])
+def test_cross_entropy_with_words_out_of_reach(lib, lo, hi):
+    """Logits of -inf: the loss and its gradient of the other words, as plain fp32 PyTorch gives them."""
+    torch.manual_seed(lo)
+    logits = _rand(5, 32000, scale=3.0)
+    logits[:, lo:hi] = float("-inf")
+    tg = torch.randint(100, 4000, (5,), device="cuda")
+    x = logits.float().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(x, tg, reduction="none")
+    (0.37 * want.sum()).backward()
+    scale = torch.full((1,), 0.37, device="cuda")
+    loss, _ = lib.ce_fwd(logits, tg, -100)
+    got = logits.clone()
+    loss1 = lib.ce_grad_(got, tg, scale, -100)
+    torch.cuda.synchronize()
+    torch.testing.assert_close(loss, want.detach(), rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(loss1, want.detach(), rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(got.float(), x.grad, rtol=1e-2, atol=1e-6)
