@@ -41,7 +41,7 @@ std::vector<at::Tensor> attn_fwd(const at::Tensor& q, const at::Tensor& k, const
                                (float)scale, nullptr, nullptr, 0, 0, 0, part_bytes > 0 ? parts.data_ptr() : nullptr, part_bytes,
                                ody_status_ptr(q), at::cuda::getCurrentCUDAStream().stream());
   req(rc == 0, "flash_fwd failed with code " + std::to_string(rc));
-  ody_count_launches(1);
+  ody_count_launches(part_bytes > 0 ? 2 : 1);      // parts: their sum is a kernel of its own
   return {o, lse};
 }
 
@@ -85,7 +85,7 @@ std::vector<at::Tensor> attn_bwd(const at::Tensor& dO, const at::Tensor& q, cons
                                part_bytes > 0 ? parts.data_ptr() : nullptr, part_bytes, ody_status_ptr(q),
                                at::cuda::getCurrentCUDAStream().stream());
   req(rc == 0, "flash_bwd failed with code " + std::to_string(rc));
-  ody_count_launches(2);
+  ody_count_launches(ody_flash_bwd_launches((int)Tq, (int)Tk, (int)H, (int)Hkv, causal ? 1 : 0, part_bytes > 0 ? 1 : 0));
   return {dq, dk, dv};
 }
 
@@ -150,7 +150,7 @@ void attn_bwd_split(const at::Tensor& dO, const at::Tensor& q, const at::Tensor&
                             causal ? 1 : 0, (float)scale, pq, pk, pv, (int)dq_dests.size(), (int)rows, ody_status_ptr(q),
                             at::cuda::getCurrentCUDAStream().stream());
   req(rc == 0, "flash_bwd (split) failed with code " + std::to_string(rc));
-  ody_count_launches(2);
+  ody_count_launches(ody_flash_bwd_launches((int)Tq, (int)Tk, (int)H, (int)Hkv, causal ? 1 : 0, 0));
 }
 
 }  // namespace

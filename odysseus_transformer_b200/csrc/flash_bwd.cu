@@ -1351,6 +1351,16 @@ extern "C" int64_t ody_flash_bwd_split_bytes(int Tq, int Tk, int H, int Hkv, int
   return kv_part_bytes(pkv, Tk, Hkv) + q_part_bytes(pq, Tq, H);
 }
 
+extern "C" int ody_flash_bwd_launches(int Tq, int Tk, int H, int Hkv, int causal, int with_parts) {
+  using namespace ody;
+  if (g_bwd_variant != 1) return 3;              // statistics, gradients, conversion of dQ
+  if (!with_parts || Tq <= 0 || Tk <= 0 || H <= 0 || Hkv <= 0 || H % Hkv) return 2;
+  SplitUnits ukv, uq;
+  SplitPlan pkv, pq;
+  bwd_plans(Tq, Tk, H, Hkv, causal, &ukv, &pkv, &uq, &pq);
+  return 2 + (pkv.max_parts > 1) + (pq.max_parts > 1);
+}
+
 extern "C" int64_t ody_flash_bwd_workspace_bytes(int Tq, int H) {
   const int64_t Tpad = ((int64_t)Tq + 127) / 128 * 128;
   // -delta and exp2-domain -lse (padded), the statistics tiles, and the fp32 dQ accumulator of the fused kernel

@@ -131,6 +131,8 @@ int ody_flash_bwd_ex(const void* dO, const void* q, const void* k, const void* v
 // the same with scratch for the partial sums of small grids, whose streamed dimension is then split over more CTAs:
 // parts: ody_flash_bwd_split_bytes(...) bytes, 16-byte aligned (0 bytes: these sizes are not split)
 int64_t ody_flash_bwd_split_bytes(int Tq, int Tk, int H, int Hkv, int causal);
+// kernels that a backward of these sizes launches (with_parts: the call is given that scratch)
+int ody_flash_bwd_launches(int Tq, int Tk, int H, int Hkv, int causal, int with_parts);
 int ody_flash_bwd_parts(const void* dO, const void* q, const void* k, const void* v, const void* o, const float* lse, void* dq,
                         void* dk, void* dv, void* workspace, int Tq, int Tk, int H, int Hkv, int64_t do_row, int64_t q_row,
                         int64_t k_row, int64_t v_row, int64_t o_row, int64_t dq_row, int64_t dk_row, int64_t dv_row, int causal,

@@ -64,3 +64,30 @@ def test_cross_entropy_with_words_out_of_reach(lib, lo, hi):
     torch.testing.assert_close(loss, want.detach(), rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(loss1, want.detach(), rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(got.float(), x.grad, rtol=1e-2, atol=1e-6)
+
+
+def test_launches_are_counted(lib):
+    """Every kernel a call launches counts, those that sum the parts of a split among them."""
+    def count(fn):
+        lib.reset_launch_count()
+        fn()
+        return lib.launch_count()
+    g = lambda m, n, k: (lambda a, b: count(lambda: lib.gemm(a, b, None, 0, False)))(_rand(m, k), _rand(n, k))   # noqa: E731
+    assert g(128, 256, 4096) == 2                        # split, sum of the shares
+    assert g(2048, 4096, 1024) == 1
+
+    def attention(Tq, Tk, H, Hkv, causal):
+        q, k, v = _rand(Tq, H, 128), _rand(Tk, Hkv, 128), _rand(Tk, Hkv, 128)
+        sc = 1.0 / math.sqrt(128)
+        o, lse = lib.attn_fwd(q, k, v, causal, sc)
+        return (count(lambda: lib.attn_fwd(q, k, v, causal, sc)),
+                count(lambda: lib.attn_bwd(q, q, k, v, o, lse, causal, sc, None, None, None)))
+    assert attention(4096, 4096, 32, 32, True) == (1, 2)  # full grids: forward; statistics, gradients
+    assert attention(2600, 2600, 4, 1, True) == (2, 4)    # both gradient grids split
+    assert attention(300, 8000, 2, 2, False) == (2, 3)    # only the queries' gradient is
+    try:
+        lib.attn_bwd_set_variant(0)
+        assert attention(1024, 1024, 4, 4, True)[1] == 3  # statistics, gradients, conversion of dQ
+    finally:
+        lib.attn_bwd_set_variant(1)
+    _check_status(lib)
