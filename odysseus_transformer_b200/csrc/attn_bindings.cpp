@@ -9,6 +9,8 @@ namespace py = pybind11;
 
 #include "ody_kernels.h"
 
+#include "scratch.h"
+
 int* ody_status_ptr(const at::Tensor& like);
 void ody_count_launches(int64_t n);
 
@@ -33,15 +35,13 @@ std::vector<at::Tensor> attn_fwd(const at::Tensor& q, const at::Tensor& k, const
   const int64_t Tq = q.size(0), Tk = k.size(0), H = q.size(1), Hkv = k.size(1);
   auto o = at::empty({Tq, H, 128}, q.options());
   auto lse = at::empty({H, Tq}, q.options().dtype(at::kFloat));
-  const int64_t part_bytes = ody_flash_fwd_split_bytes((int)Tq, (int)Tk, (int)H, causal ? 1 : 0);
-  at::Tensor parts;
-  if (part_bytes > 0) parts = at::empty({part_bytes}, q.options().dtype(at::kByte));
+  const ody::OptionalScratch parts(ody_flash_fwd_split_bytes((int)Tq, (int)Tk, (int)H, causal ? 1 : 0), q);
   int rc = ody_flash_fwd_parts(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), (int)Tq, (int)Tk,
                                (int)H, (int)Hkv, q.stride(0), k.stride(0), v.stride(0), o.stride(0), causal ? 1 : 0,
-                               (float)scale, nullptr, nullptr, 0, 0, 0, part_bytes > 0 ? parts.data_ptr() : nullptr, part_bytes,
+                               (float)scale, nullptr, nullptr, 0, 0, 0, parts.ptr(), parts.bytes,
                                ody_status_ptr(q), at::cuda::getCurrentCUDAStream().stream());
   req(rc == 0, "flash_fwd failed with code " + std::to_string(rc));
-  ody_count_launches(part_bytes > 0 ? 2 : 1);      // parts: their sum is a kernel of its own
+  ody_count_launches(parts.bytes > 0 ? 2 : 1);      // parts: their sum is a kernel of its own
   return {o, lse};
 }
 
@@ -75,17 +75,14 @@ std::vector<at::Tensor> attn_bwd(const at::Tensor& dO, const at::Tensor& q, cons
   req(dq.size(0) == Tq && dq.size(1) == H && dk.size(0) == Tk && dk.size(1) == Hkv && dv.size(0) == Tk && dv.size(1) == Hkv,
       "gradient output shape mismatch");
   auto ws = at::empty({ody_flash_bwd_workspace_bytes((int)Tq, (int)H)}, q.options().dtype(at::kByte));
-  const int64_t part_bytes = ody_flash_bwd_split_bytes((int)Tq, (int)Tk, (int)H, (int)Hkv, causal ? 1 : 0);
-  at::Tensor parts;
-  if (part_bytes > 0) parts = at::empty({part_bytes}, q.options().dtype(at::kByte));
+  const ody::OptionalScratch parts(ody_flash_bwd_split_bytes((int)Tq, (int)Tk, (int)H, (int)Hkv, causal ? 1 : 0), q);
   int rc = ody_flash_bwd_parts(dO.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
                                dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), (int)Tq, (int)Tk, (int)H, (int)Hkv,
                                dO.stride(0), q.stride(0), k.stride(0), v.stride(0), o.stride(0), dq.stride(0), dk.stride(0),
                                dv.stride(0), causal ? 1 : 0, (float)scale, nullptr, nullptr, nullptr, 0, 0,
-                               part_bytes > 0 ? parts.data_ptr() : nullptr, part_bytes, ody_status_ptr(q),
-                               at::cuda::getCurrentCUDAStream().stream());
+                               parts.ptr(), parts.bytes, ody_status_ptr(q), at::cuda::getCurrentCUDAStream().stream());
   req(rc == 0, "flash_bwd failed with code " + std::to_string(rc));
-  ody_count_launches(ody_flash_bwd_launches((int)Tq, (int)Tk, (int)H, (int)Hkv, causal ? 1 : 0, part_bytes > 0 ? 1 : 0));
+  ody_count_launches(ody_flash_bwd_launches((int)Tq, (int)Tk, (int)H, (int)Hkv, causal ? 1 : 0, parts.bytes > 0 ? 1 : 0));
   return {dq, dk, dv};
 }
 

@@ -13,6 +13,7 @@
 
 #include "ody_kernels.h"
 #include "epilogue_arg.h"
+#include "scratch.h"
 
 namespace {
 
@@ -84,14 +85,12 @@ at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const c10::optional<at
   ody_req(!(accumulate && residual.has_value()), "gemm: accumulate and residual exclude each other");
   ody_req(rope.is_none() || layout == 0, "gemm: the rotary epilogue belongs to layout 0 (a forward projection)");
   if (K == 0) { if (!accumulate) c.zero_(); return c; }
-  const int64_t ws_bytes = ody_gemm_split_bytes((int)M, (int)N, (int)K);
-  at::Tensor ws;
-  if (ws_bytes > 0) ws = at::empty({ws_bytes}, a.options().dtype(at::kByte));
+  const ody::OptionalScratch ws(ody_gemm_split_bytes((int)M, (int)N, (int)K), a);
   ODY_CHECK(ody_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), c.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0),
                              c.stride(0), (int)layout, accumulate ? 1 : 0, has_epi ? &epi : nullptr,
-                             ws_bytes > 0 ? ws.data_ptr() : nullptr, ws_bytes, status_ptr(a), cur_stream()),
+                             ws.ptr(), ws.bytes, status_ptr(a), cur_stream()),
             "gemm");
-  g_launches += ws_bytes > 0 ? 2 : 1;      // split: the sum of the shares is a kernel of its own
+  g_launches += ws.bytes > 0 ? 2 : 1;      // split: the sum of the shares is a kernel of its own
   return c;
 }
 

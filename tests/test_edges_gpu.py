@@ -91,3 +91,38 @@ def test_launches_are_counted(lib):
     finally:
         lib.attn_bwd_set_variant(1)
     _check_status(lib)
+
+
+def test_calls_run_unsplit_when_scratch_cannot_be_had(lib):
+    """Scratch only makes these calls faster: without memory for it they run as they would unsplit."""
+    q, k, v, do = _rand(300, 2, 128), _rand(8000, 2, 128), _rand(8000, 2, 128), _rand(300, 2, 128)
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    a, b, c = _rand(512, 32000), _rand(1024, 32000), torch.empty(512, 1024, device="cuda", dtype=torch.bfloat16)
+    sc = 1.0 / math.sqrt(128)
+
+    def run():
+        o, lse = lib.attn_fwd(q, k, v, False, sc)
+        lib.reset_launch_count()
+        lib.attn_bwd(do, q, k, v, o, lse, False, sc, dq, dk, dv)
+        lib.gemm(a, b, c, 0, False)
+        torch.cuda.synchronize()
+        return [t.to("cpu", torch.float32) for t in (o, lse, dq, dk, dv, c)], lib.launch_count()
+    want, n = run()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    fill = []
+    try:
+        # two allocator segments of 2 MiB for the calls' small outputs and statistics, but none of 20 MiB, and what is free in
+        # those that there are taken up
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (4 << 20)) / total)
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            for _ in range(2048):
+                fill.append(torch.empty(2 << 20, dtype=torch.uint8, device="cuda"))
+        got, m = run()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        del fill
+    assert m < n                                           # it did run without its sums
+    for x, y in zip(got, want):
+        assert ((x - y).norm() / y.norm()).item() < 5e-3   # the same sums in another order, rounded to bf16
+    _check_status(lib)
