@@ -301,7 +301,7 @@ void embedding_grad_(const at::Tensor& dy, const at::Tensor& ids, at::Tensor dw)
           ids.get_device() == dw.get_device() && dy.get_device() == dw.get_device(), "embedding_grad_: ids [T] int64 on dw's device");
   c10::cuda::CUDAGuard guard(dw.device());
   ODY_CHECK(ody_embedding_grad(dy.data_ptr(), ids.data_ptr<int64_t>(), dw.data_ptr(), dy.size(0), (int)dy.size(1), dw.size(0),
-                               cur_stream()), "embedding_grad");
+                               status_ptr(dw), cur_stream()), "embedding_grad");
   ++g_launches;
 }
 

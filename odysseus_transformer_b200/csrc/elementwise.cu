@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "ody_kernels.h"
+#include "sm100.cuh"
 
 namespace ody {
 
@@ -496,16 +497,20 @@ __global__ void __launch_bounds__(256) scale_k(bf16* dst, const bf16* src, const
 // ------------------------------------------------------------------------------------------- embedding gradient
 
 // dw[ids[t]] += dy[t] in bf16: one thread per 8 columns of a token, one 16-byte vector reduction each.  Tokens that share a
-// row add in no fixed order, as with index_add.  Reads dy once; bound by memory: 36 us at 8192 tokens x 4096, where index_add
+// row add in no fixed order, as with index_add.  An id outside the table is skipped and reported.  Reads dy once; bound by memory: 36 us at 8192 tokens x 4096, where index_add
 // with its scalar reductions took 345.
 __global__ void __launch_bounds__(256) embedding_grad_k(const bf16* __restrict__ dy, const int64_t* __restrict__ ids,
-                                                        bf16* __restrict__ dw, int64_t total, int vpr, int64_t vocab) {
+                                                        bf16* __restrict__ dw, int64_t total, int vpr, int64_t vocab,
+                                                        int* __restrict__ err) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total) return;
   const int64_t t = i / vpr;
   const int c = (int)(i - t * vpr) * 8;
   const int64_t id = ids[t];
-  if (id < 0 || id >= vocab) return;
+  if (id < 0 || id >= vocab) {
+    if (err != nullptr) atomicCAS(err, 0, ODY_ERR_BAD_INDEX);
+    return;
+  }
   const uint4 v = *reinterpret_cast<const uint4*>(dy + i * 8);
   bf16* dst = dw + id * ((int64_t)vpr * 8) + c;
   asm volatile("red.relaxed.gpu.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
@@ -812,13 +817,14 @@ extern "C" int ody_scale(void* dst, const void* src, const float* scale, int64_t
   return last_err();
 }
 
-extern "C" int ody_embedding_grad(const void* dy, const int64_t* ids, void* dw, int64_t T, int dim, int64_t vocab, cudaStream_t st) {
+extern "C" int ody_embedding_grad(const void* dy, const int64_t* ids, void* dw, int64_t T, int dim, int64_t vocab, int* err,
+                                  cudaStream_t st) {
   if (dim % 8 != 0 || vocab <= 0 || (((uintptr_t)dy | (uintptr_t)dw) & 15)) return (int)cudaErrorInvalidValue;
   const cudaError_t e = cudaMemsetAsync(dw, 0, (size_t)vocab * dim * 2, st);
   if (e != cudaSuccess) return (int)e;
   const int64_t total = T * (dim / 8);
   if (total == 0) return 0;
-  embedding_grad_k<<<blocks_for(total, 256), 256, 0, st>>>((const bf16*)dy, ids, (bf16*)dw, total, dim / 8, vocab);
+  embedding_grad_k<<<blocks_for(total, 256), 256, 0, st>>>((const bf16*)dy, ids, (bf16*)dw, total, dim / 8, vocab, err);
   return last_err();
 }
 

@@ -51,8 +51,10 @@ int ody_ce_bwd(void* logits, const int64_t* targets, const float* lse, const flo
 int ody_scale(void* dst, const void* src, const float* scale, int64_t n, cudaStream_t stream);
 // dst = src * scale[0] over n bf16 values (n % 8 == 0; dst may be src)
 int ody_scale(void* dst, const void* src, const float* scale, int64_t n, cudaStream_t stream);
-// dw [vocab, dim] bf16 = 0, then dw[ids[t]] += dy[t] for t < T (bf16 sums in memory, in no fixed order)
-int ody_embedding_grad(const void* dy, const int64_t* ids, void* dw, int64_t T, int dim, int64_t vocab, cudaStream_t stream);
+// dw [vocab, dim] bf16 = 0, then dw[ids[t]] += dy[t] for t < T (bf16 sums in memory, in no fixed order); an id outside
+// [0, vocab) is skipped and reported in *err (device, may be null)
+int ody_embedding_grad(const void* dy, const int64_t* ids, void* dw, int64_t T, int dim, int64_t vocab, int* err,
+                       cudaStream_t stream);
 // when *guard != 0 at run time the kernel changes nothing (a failed step must not reach the master weights).
 int ody_adamw(float* master, float* m, float* v, const void* grad, void* param, int64_t n, float lr, float beta1,
               float beta2, float eps, float weight_decay, int step, float grad_scale, const float* guard,

@@ -19,6 +19,7 @@ enum : int {
   ODY_ERR_TIMEOUT_TMEM_EMPTY = 104,
   ODY_ERR_TIMEOUT_PEER = 105,     // a flag owned by another GPU was never set
   ODY_ERR_TIMEOUT_MISC = 106,
+  ODY_ERR_BAD_INDEX = 107,        // an index outside its table; the access was skipped
 };
 
 #ifdef __CUDACC__

@@ -91,12 +91,12 @@ def launch_count() -> int:
 
 
 class KernelStatusError(RuntimeError):
-    """A bounded device-side wait gave up (codes in ``csrc/sm100.cuh``: 101-104 pipeline stages of one
-    kernel, 105 a flag another GPU never set, 106 other)."""
+    """A kernel reported a failure (codes in ``csrc/sm100.cuh``): a bounded device-side wait gave up (101-104 pipeline
+    stages of one kernel, 105 a flag another GPU never set, 106 other), or an index lay outside its table (107)."""
 
     def __init__(self, status: int, where: str = ""):
-        super().__init__(f"odysseus_transformer_b200 kernel reported status {status} "
-                         f"(a bounded device-side wait expired){' ' + where if where else ''}")
+        what = "an index outside its table" if status == 107 else "a bounded device-side wait expired"
+        super().__init__(f"odysseus_transformer_b200 kernel reported status {status} ({what}){' ' + where if where else ''}")
         self.status = status
 
 

@@ -126,3 +126,22 @@ def test_calls_run_unsplit_when_scratch_cannot_be_had(lib):
     for x, y in zip(got, want):
         assert ((x - y).norm() / y.norm()).item() < 5e-3   # the same sums in another order, rounded to bf16
     _check_status(lib)
+
+
+@pytest.mark.parametrize("bad", [50, -1, 1 << 40])
+def test_embedding_gradient_reports_ids_outside_the_table(lib, bad):
+    """index_add_ refuses such ids; the kernel skips them, says so, and the other tokens' rows are right."""
+    from odysseus_transformer_b200.ops import native
+    dy, ids = _rand(40, 64), torch.arange(40, device="cuda")
+    ids[7] = bad
+    dw = torch.empty(50, 64, device="cuda", dtype=torch.bfloat16)
+    lib.embedding_grad_(dy, ids, dw)
+    torch.cuda.synchronize()
+    assert lib.status(0) == 107
+    with pytest.raises(native.KernelStatusError, match="index"):
+        native.check_status(0)
+    want = torch.zeros_like(dw)
+    want[:40] = dy
+    want[7] = 0
+    assert torch.equal(dw, want)
+    _check_status(lib)
