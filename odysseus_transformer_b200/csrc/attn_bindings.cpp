@@ -4,6 +4,7 @@
 #include <torch/extension.h>
 namespace py = pybind11;
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 
@@ -155,6 +156,11 @@ void attn_bwd_split(const at::Tensor& dO, const at::Tensor& q, const at::Tensor&
 void ody_register_attention(pybind11::module& m) {
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_fwd_split", &attn_fwd_split);
+  // scratch that attn_fwd / attn_bwd of these sizes ask for (the larger of the two)
+  m.def("attn_scratch_bytes", [](int64_t Tq, int64_t Tk, int64_t H, int64_t Hkv, bool causal) {
+    return std::max(ody_flash_fwd_split_bytes((int)Tq, (int)Tk, (int)H, causal ? 1 : 0),
+                    ody_flash_bwd_split_bytes((int)Tq, (int)Tk, (int)H, (int)Hkv, causal ? 1 : 0));
+  });
   m.def("attn_bwd_split", &attn_bwd_split);
   m.def("attn_fwd_set_trace", [](const c10::optional<at::Tensor>& t) {
     if (t.has_value()) req(t.value().is_cuda() && t.value().scalar_type() == at::kLong && t.value().numel() >= 64 * 16, "trace: int64 [64*16]");

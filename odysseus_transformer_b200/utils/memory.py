@@ -22,6 +22,9 @@ projection widths, V vocabulary; activations and weights are bf16):
 * transients of backward: the gradients of one MLP (gate|up and SwiGLU output: 3 I per token), one packed dq|dk|dv
   (q + 2 kv) and the fp32 dQ accumulator of the attention backward (4 bytes x q per token, over the tokens the attention
   core sees).
+* scratch of the attention kernels where a grid would leave SMs idle (few heads per rank, short sequences): the fp32 partial
+  sums of split tiles, as the extension states them for these sizes (at most 512 MiB, part of the transients; a call without memory
+  for them runs without).
 * communication buffers: the symmetric heap (``comm.symm.heap_bytes_estimate``) on the fused backend, outside the
   caching allocator's statistics; on the library backend the two largest gathered weights.
 """
@@ -50,6 +53,24 @@ def saved_bytes_per_token_per_layer(cfg, mode: str, inner: int = 1, fused: bool 
         elems += q                   # the attention output in head layout (attention) and in sequence layout (o_proj)
     stats = 4 * cfg.num_attention_heads + 2 * 4          # log-sum-exp per head, two rstd
     return elems * elem + stats
+
+
+def attention_scratch_bytes(cfg, mode: str, t: int, inner: int, ring: int) -> int:
+    """Scratch of the largest attention call of a step on the fused backend: ``t`` local tokens, ``inner`` ranks sharing the
+    heads, ``ring`` ranks sharing the sequence of the attention core (see the module docstring)."""
+    from ..ops import native
+    if cfg.head_dim != 128 or not native.available():
+        return 0
+    if mode not in ("odysseus", "tpsp", "ulysses"):
+        inner = 1
+    if mode == "ulysses" and inner > 1 and ring == 1:
+        return 0                     # its kernels store to the ranks that own the rows and are not split
+    T, h, hkv = t * inner, max(1, cfg.num_attention_heads // inner), max(1, cfg.num_key_value_heads // inner)
+    blocks = [(T, T, True)]
+    if ring > 1:
+        blocks += [(T, T // 2, False), (T - T // 2, T, False)]
+    f = native.lib().attn_scratch_bytes
+    return max(f(tq, tk, h, hkv, causal) for tq, tk, causal in blocks if tq > 0 and tk > 0)
 
 
 def estimate_memory(cfg, mode: str, seq_length: int, world: int, ulysses_degree: Optional[int] = None,
@@ -81,6 +102,8 @@ def estimate_memory(cfg, mode: str, seq_length: int, world: int, ulysses_degree:
     logits = rows * cfg.vocab_size * elem + 2 * t * cfg.hidden_size * elem
     t_attn = t * inner if mode in ("odysseus", "tpsp", "ulysses") else t     # tokens the attention core sees (heads / inner)
     transient = t * (3 * cfg.intermediate_size + cfg.q_size + 2 * cfg.kv_size) * elem + 4 * t_attn * cfg.q_size // inner
+    scratch = attention_scratch_bytes(cfg, mode, t, inner, world if mode == "ring" else ring_degree) if fused and elem == 2 else 0
+    transient += scratch
     comm = 0.0
     lib_buffers = 0.0
     if world > 1:
@@ -95,7 +118,7 @@ def estimate_memory(cfg, mode: str, seq_length: int, world: int, ulysses_degree:
         peak = states + kept + max(logits, t * per_tok + transient) + lib_buffers
     else:
         peak = states + saved + logits + transient + lib_buffers
-    out = {"states": states, "saved_activations": saved, "logits": logits, "backward_transients": transient,
+    out = {"states": states, "saved_activations": saved, "logits": logits, "backward_transients": transient, "attention_scratch": scratch,
            "library_gather_buffers": lib_buffers, "peak_allocated": peak, "comm_heap": comm, "total_device": peak + comm}
     return {k: v / GIB for k, v in out.items()}
 

@@ -61,6 +61,25 @@ def test_estimate_matches_measured_peaks(mode, L, n, ckpt, peak):
     assert est["peak_allocated"] == pytest.approx(peak, rel=0.06)
 
 
+def test_estimate_knows_the_attention_scratch():
+    from odysseus_transformer_b200.config import get_model_config
+    from odysseus_transformer_b200.ops import native
+    from odysseus_transformer_b200.utils.memory import GIB, estimate_memory
+    if not native.available():
+        pytest.skip("extension not built")
+    cfg = get_model_config("llama3-8b")                                 # a rank of 8: 4 query heads on 1
+    est = estimate_memory(cfg, "odysseus", 20000, 8)
+    assert est["attention_scratch"] * GIB == native.lib().attn_scratch_bytes(20000, 20000, 4, 1, True) > 90 << 20
+    without = estimate_memory(cfg, "odysseus", 20000, 8, fused=False)
+    assert without["attention_scratch"] == 0
+    assert est["backward_transients"] - without["backward_transients"] == pytest.approx(est["attention_scratch"])
+    assert estimate_memory(cfg, "ulysses", 20000, 8)["attention_scratch"] == 0
+    assert estimate_memory(get_model_config("llama2-7b"), "odysseus", 131072, 8)["attention_scratch"] == 0
+    for ring in (1, 2, 4):
+        e = estimate_memory(cfg, "odysseus", 16384, 8, ulysses_degree=8 // ring, ring_degree=ring)
+        assert 0 <= e["attention_scratch"] <= 0.5
+
+
 def test_what_fits():
     from odysseus_transformer_b200.config import get_model_config
     from odysseus_transformer_b200.utils.memory import estimate_memory, fits
