@@ -1,5 +1,8 @@
 """sm_100a kernels against plain PyTorch fp32 references of the same op (needs a B200)."""
+import contextlib
+import ctypes
 import math
+import os
 
 import pytest
 import torch
@@ -21,6 +24,27 @@ def _rand(*shape, scale=1.0, dtype=torch.bfloat16):
 def _check_status(lib):
     torch.cuda.synchronize()
     assert lib.status(0) == 0, f"kernel status {lib.status(0)}"
+
+
+@pytest.fixture(scope="module")
+def splits(lib):
+    """The host rules that decide whether a call is split: functions of the extension's C interface."""
+    import odysseus_transformer_b200
+    c = ctypes.CDLL(os.path.join(os.path.dirname(odysseus_transformer_b200.__file__), "_C.so"))
+    for f, n in ((c.ody_flash_fwd_split_bytes, 4), (c.ody_gemm_split_bytes, 3)):
+        f.restype, f.argtypes = ctypes.c_int64, [ctypes.c_int] * n
+    c.ody_flash_bwd_launches.restype, c.ody_flash_bwd_launches.argtypes = ctypes.c_int, [ctypes.c_int] * 6
+    return c
+
+
+@contextlib.contextmanager
+def _unsplit(lib):
+    """Products on the one-CTA kernel, which a chosen variant never splits."""
+    lib.gemm_set_variant(1)
+    try:
+        yield
+    finally:
+        lib.gemm_set_variant(0)
 
 
 GEMM_SHAPES = [(128, 256, 64), (256, 512, 128), (384, 768, 320), (304, 264, 200), (1000, 72, 136),
@@ -484,17 +508,21 @@ def test_attention_bwd_packed_outputs(lib, bwd_variant):
 
 
 # Sizes whose grids leave SMs idle, so that the streamed dimension is split over more CTAs (csrc/attn_split.cuh): grouped
-# queries on one kv head, few heads, few query rows on many keys and the reverse, lengths next to a block edge.
+# queries on one kv head, few heads, few query rows on many keys and the reverse, lengths next to a block edge.  The last
+# two: how many grids of the forward and of the backward (dK/dV, dQ) are split.
 SPLIT_CASES = [
-    (1531, 1531, 8, 2, True), (2600, 2600, 4, 1, True), (1025, 1025, 4, 4, True), (3073, 3073, 2, 2, True),
-    (300, 8000, 2, 2, False), (8000, 257, 4, 1, False), (129, 4097, 1, 1, False), (4096, 4096, 1, 1, True),
+    (1531, 1531, 8, 2, True, 1, 1), (2600, 2600, 4, 1, True, 1, 2), (1025, 1025, 4, 4, True, 1, 0), (1025, 1025, 1, 1, True, 1, 2),
+    (3073, 3073, 2, 2, True, 1, 2), (300, 8000, 2, 2, False, 1, 1), (8000, 257, 4, 1, False, 0, 1), (129, 4097, 1, 1, False, 1, 1),
+    (4096, 4096, 1, 1, True, 1, 2),
 ]
 
 
-@pytest.mark.parametrize("Tq,Tk,H,Hkv,causal", SPLIT_CASES)
-def test_attention_split_grids(lib, Tq, Tk, H, Hkv, causal):
+@pytest.mark.parametrize("Tq,Tk,H,Hkv,causal,fwd,bwd", SPLIT_CASES)
+def test_attention_split_grids(lib, splits, Tq, Tk, H, Hkv, causal, fwd, bwd):
     """Split grids against fp32 PyTorch, with strided operands and gradients, and twice the same bits."""
     from odysseus_transformer_b200.ops import torch_ref as R
+    assert (splits.ody_flash_fwd_split_bytes(Tq, Tk, H, int(causal)) > 0) == bool(fwd)
+    assert splits.ody_flash_bwd_launches(Tq, Tk, H, Hkv, int(causal), 1) == 2 + bwd
     torch.manual_seed(Tq + 5 * Tk + H)
     q = _rand(Tq, H + 1, 128)[:, 1:]
     kv = _rand(Tk, 2 * Hkv, 128)
@@ -523,7 +551,8 @@ def test_attention_split_grids(lib, Tq, Tk, H, Hkv, causal):
 
 @pytest.mark.parametrize("T,V,ignore", [(37, 32000, True), (5, 128256, False), (64, 8, True), (3, 8200, False)])
 def test_cross_entropy_grad_in_one_pass(lib, T, V, ignore):
-    """Loss and gradient of the one-pass kernel against the two kernels it replaces where the scale is known up front."""
+    """Loss and gradient of the one-pass kernel against fp32 PyTorch, and against the two kernels it replaces where the scale is
+    known up front."""
     torch.manual_seed(V + T)
     logits = _rand(T, V, scale=3.0)
     tg = torch.randint(V, (T,), device="cuda")
@@ -538,6 +567,11 @@ def test_cross_entropy_grad_in_one_pass(lib, T, V, ignore):
     torch.cuda.synchronize()
     torch.testing.assert_close(loss1, loss, rtol=1e-5, atol=1e-5)      # sums of fp32 exponentials in another order
     torch.testing.assert_close(got.float(), want.float(), rtol=1e-2, atol=1e-6)
+    x = logits.float().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(x, tg, reduction="none", ignore_index=-100)
+    (0.37 * ref.sum()).backward()
+    torch.testing.assert_close(loss1, ref.detach(), rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(got.float(), x.grad, rtol=1e-2, atol=1e-6)     # one rounding to bf16: half a step is 2^-9
 
 
 def test_scale_into(lib):
@@ -553,7 +587,7 @@ def test_scale_into(lib):
         lib.scale_into_(dst[:, :64], src[:, :64], scale)
 
 
-@pytest.mark.parametrize("T,V,d", [(1, 8, 8), (777, 50, 1024), (300, 32000, 136), (2048, 100000, 64)])
+@pytest.mark.parametrize("T,V,d", [(1, 8, 8), (777, 50, 1024), (300, 32000, 136), (2048, 100000, 64), (200, 128256, 4096)])
 def test_embedding_grad(lib, T, V, d):
     """Rows that several tokens share are summed in bf16, as index_add into a bf16 gradient does: each of k additions may
     round by half a bf16 step (2^-9) of the partial sum."""
@@ -570,25 +604,25 @@ def test_embedding_grad(lib, T, V, d):
 
 
 # Few output tiles and a long K (the split of csrc/gemm.cu): one tile, ragged edges, the smallest and largest number of shares
-SPLITK_SHAPES = [(128, 256, 2048), (512, 1024, 32000), (8, 8, 65536), (130, 264, 1000), (1, 4096, 11008), (2000, 72, 8200),
+SPLITK_SHAPES = [(128, 256, 2048), (512, 1024, 32000), (8, 8, 65536), (130, 264, 4104), (1, 4096, 11008), (2000, 72, 8200),
                  (128, 1024, 2816)]
 
 
 @pytest.mark.parametrize("layout", [0, 1, 2])
 @pytest.mark.parametrize("M,N,K", SPLITK_SHAPES)
-def test_gemm_split_k(lib, layout, M, N, K):
+def test_gemm_split_k(lib, splits, layout, M, N, K):
     """Against fp32 and against the unsplit kernel; accumulating onto C, with a residual, into a strided output."""
     torch.manual_seed(M + N + K + layout)
     K = K // 8 * 8
     if layout == 2:
         M = max(8, M // 8 * 8)
+    assert splits.ody_gemm_split_bytes(M, N, K) > 0
     a = _rand(M, K) if layout != 2 else _rand(K, M)
     b = _rand(N, K) if layout == 0 else _rand(K, N)
     ref = (a.float() if layout != 2 else a.float().t()) @ (b.float().t() if layout == 0 else b.float())
     c = lib.gemm(a, b, None, layout, False)
-    lib.gemm_set_variant(1)
-    c1 = lib.gemm(a, b, None, layout, False)
-    lib.gemm_set_variant(0)
+    with _unsplit(lib):
+        c1 = lib.gemm(a, b, None, layout, False)
     _check_status(lib)
     assert ((c.float() - ref).norm() / ref.norm()).item() <= 1.05 * ((c1.float() - ref).norm() / ref.norm()).item() + 1e-5
     wide = _rand(M, 2 * N)
@@ -605,18 +639,18 @@ def test_gemm_split_k(lib, layout, M, N, K):
 
 
 @pytest.mark.parametrize("M", [1, 128, 300])
-def test_gemm_split_k_rope(lib, M):
+def test_gemm_split_k_rope(lib, splits, M):
     """The rotary epilogue done by the summing kernel equals the one of the unsplit kernel up to the sum's rounding."""
     from odysseus_transformer_b200.ops import torch_ref as R
     torch.manual_seed(M)
     N, K = 768, 4096
+    assert splits.ody_gemm_split_bytes(M, N, K) > 0
     a, b = _rand(M, K), _rand(N, K)
     cos, sin = R.rope_tables(torch.randint(0, 9999, (M,), device="cuda"), 128, 10000.0)
     rope = (cos, sin, 256, 384)
     y = lib.gemm(a, b, None, 0, False, rope, None)
-    lib.gemm_set_variant(1)
-    y1 = lib.gemm(a, b, None, 0, False, rope, None)
-    lib.gemm_set_variant(0)
+    with _unsplit(lib):
+        y1 = lib.gemm(a, b, None, 0, False, rope, None)
     _check_status(lib)
     assert ((y.float() - y1.float()).norm() / y1.float().norm()).item() < 2e-3
 
@@ -633,3 +667,69 @@ def test_rmsnorm_bwd_weight_gradient_in_bf16(lib, rows, dim):
     assert torch.equal(dx, dx2) and torch.equal(out, dw.to(torch.bfloat16))
     with pytest.raises(RuntimeError):
         lib.rmsnorm_bwd(dy, x, w, rstd, ds, out[: dim // 2])
+
+
+@pytest.mark.parametrize("with_ds", [False, True])
+@pytest.mark.parametrize("rows,dim", [(1500, 4096), (900, 8192), (1190, 1000)])
+def test_rmsnorm_bwd_slots_are_reused(lib, rows, dim, with_ds):
+    """More rows to a block than the ring of fetched rows has slots (4), so that every slot is filled again: against fp32
+    PyTorch, one rounding to bf16 for dx, fp32 sums over the rows for dw."""
+    from odysseus_transformer_b200.ops import torch_ref as R
+    torch.manual_seed(rows)
+    x, w, dy, ds = _rand(rows, dim), _rand(dim) + 1, _rand(rows, dim), _rand(rows, dim)
+    _, rstd = lib.rmsnorm_fwd(x, w, 1e-5)
+    dx, dw = lib.rmsnorm_bwd(dy, x, w, rstd, ds if with_ds else None)
+    torch.cuda.synchronize()
+    dxr, dwr = R.rmsnorm_bwd(dy.float(), x.float(), w.float(), rstd)
+    dxr = dxr + ds.float() if with_ds else dxr
+    torch.testing.assert_close(dx.float(), dxr, rtol=2.0 ** -8, atol=1e-4)
+    torch.testing.assert_close(dw, dwr, rtol=1e-5, atol=1e-5 * math.sqrt(rows) * 4)
+
+
+@pytest.mark.parametrize("dloss", [1.0, 0.3])
+def test_chunked_loss_with_main_grad(lib, dloss):
+    """lm_head + loss in chunks, the weight's gradient written where the optimizer reads it, against fp32 PyTorch: logits and their
+    gradient are bf16 (2^-9 each), chunks add up in a bf16 buffer."""
+    from odysseus_transformer_b200.ops import functional as F
+    torch.manual_seed(3)
+    t, d, V = 700, 512, 4096
+    h, w = _rand(t, d).requires_grad_(True), _rand(V, d, scale=0.05).requires_grad_(True)
+    w.main_grad = torch.full((V, d), float("nan"), device="cuda", dtype=torch.bfloat16)
+    tg = torch.randint(V, (t,), device="cuda")
+    tg[::7] = -100
+    loss = F.linear_cross_entropy_sum(h, w, tg, 1.0 / t, None, 256)
+    (loss * dloss).backward()
+    _check_status(lib)
+    hr, wr = h.detach().float().requires_grad_(True), w.detach().float().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(hr @ wr.t(), tg, reduction="sum", ignore_index=-100) / t
+    (ref * dloss).backward()
+    assert abs(loss.item() - ref.item()) < 2e-3 * ref.item()
+    assert w.grad is None and w._grad_written
+    for got, want in ((h.grad, hr.grad), (w.main_grad, wr.grad)):
+        assert ((got.float() - want).norm() / want.norm()).item() < 1e-2
+
+
+def test_model_step_with_optimizer_fused_vs_library():
+    """A step of the small model with the optimizer attached, so that every gradient goes to ``main_grad`` the way training writes
+    it, with the loss in one piece and in chunks: own kernels against the torch / cuBLAS / flash path, same weights."""
+    from odysseus_transformer_b200.config import get_model_config
+    from odysseus_transformer_b200.mesh import ParallelContext
+    from odysseus_transformer_b200.ops import native
+    from odysseus_transformer_b200.train import Trainer
+    cfg = get_model_config("small")
+    L = 700
+    ctx = ParallelContext(device=torch.device("cuda", 0))
+    batch = torch.randint(cfg.vocab_size, (1, L + 1), generator=torch.Generator().manual_seed(0))
+    for rows in (0, 256):
+        grads, loss = {}, {}
+        for be in ("library", "fused"):
+            native.set_backend(be)
+            tr = Trainer(cfg, "odysseus", ctx, L, seed=0, loss_chunk_rows=rows)
+            loss[be] = tr.train_step(batch).item()
+            grads[be] = {n: p.main_grad.float().clone() for n, p in tr.model.named_parameters()}
+        native.set_backend("fused")
+        native.check_status(0)
+        assert abs(loss["fused"] - loss["library"]) < 2e-2, loss
+        for n, want in grads["library"].items():
+            rel = ((grads["fused"][n] - want).norm() / (want.norm() + 1e-6)).item()
+            assert rel < 0.08, f"{n}, chunks of {rows}: rel grad diff {rel}"      # as for the step without an optimizer
