@@ -62,18 +62,15 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_k(const bf16* __restrict__ x,
   }
 }
 
-// Two rows per loop iteration and one barrier per iteration (the warps' partial dot products go through a
-// double-buffered shared array that every thread sums itself).  The kernel is bound by memory latency, so what matters
-// is how many row loads are in flight per SM: the rows stay in registers as packed bf16 and are unpacked a second time
-// for the output instead of being kept as fp32, which halves the registers and lets two blocks share an SM (with the
-// fp32 copies it was one block per SM and a third of the copy bandwidth).
+// Rows wider than the ring kernel's (below): one row per iteration, one barrier (the warps' partial dot products go through a
+// double-buffered shared array that every thread sums itself).  The row stays in registers as packed bf16 and is unpacked
+// a second time for the output: with fp32 copies 16384 columns would spill.
 template <int NV>
-__global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1) rmsnorm_bwd_k(const bf16* __restrict__ dy, const bf16* __restrict__ x,
+__global__ void __launch_bounds__(256, 1) rmsnorm_bwd_k(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                                                      const bf16* __restrict__ w, const float* __restrict__ rstd,
                                                      const bf16* __restrict__ ds, bf16* __restrict__ dx,
                                                      float* __restrict__ dw_partial, int64_t rows, int dim) {
-  constexpr int R = NV <= 2 ? 2 : 1;      // wider rows would spill
-  __shared__ __align__(16) float red[2][R][8];
+  __shared__ __align__(16) float red[2][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float wv[NV][8], acc[NV][8];
 #pragma unroll
@@ -85,66 +82,54 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1) rmsnorm_bwd_k(const bf16
   }
   const float inv_dim = 1.f / (float)dim;
   int par = 0;
-  for (int64_t row0 = (int64_t)blockIdx.x * R; row0 < rows; row0 += (int64_t)gridDim.x * R, par ^= 1) {
-    float rs[R], dot[R];
-    bf16x8 pa[R][NV], px[R][NV];
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
+    const float rs = rstd[row];
+    bf16x8 pa[NV], px[NV];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t row = row0 + r;
-      rs[r] = row < rows ? rstd[row] : 0.f;
+    for (int i = 0; i < NV; ++i) {
+      const int c = (threadIdx.x + i * blockDim.x) * 8;
+      if (c < dim) {
+        pa[i] = ld8(dy + row * dim + c);
+        px[i] = ld8(x + row * dim + c);
+      }
+    }
+    float dot = 0.f;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int c = (threadIdx.x + i * blockDim.x) * 8;
-        if (c < dim && row < rows) {
-          pa[r][i] = ld8(dy + row * dim + c);
-          px[r][i] = ld8(x + row * dim + c);
+    for (int i = 0; i < NV; ++i) {
+      const int c = (threadIdx.x + i * blockDim.x) * 8;
+      if (c < dim) {
+        float a[8], xh[8];
+        unpack8(pa[i], a);
+        unpack8(px[i], xh);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          xh[j] *= rs;
+          acc[i][j] += a[j] * xh[j];
+          dot += a[j] * wv[i][j] * xh[j];
         }
       }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      dot[r] = 0.f;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int c = (threadIdx.x + i * blockDim.x) * 8;
-        if (c < dim && row0 + r < rows) {
-          float a[8], xh[8];
-          unpack8(pa[r][i], a);
-          unpack8(px[r][i], xh);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            xh[j] *= rs[r];
-            acc[i][j] += a[j] * xh[j];
-            dot[r] += a[j] * wv[i][j] * xh[j];
-          }
-        }
-      }
-      dot[r] = warp_sum(dot[r]);
-      if (lane == 0) red[par][r][wid] = dot[r];
-    }
+    dot = warp_sum(dot);
+    if (lane == 0) red[par][wid] = dot;
     __syncthreads();
+    const float4 lo = *reinterpret_cast<const float4*>(&red[par][0]), hi = *reinterpret_cast<const float4*>(&red[par][4]);
+    dot = ((lo.x + lo.y) + (lo.z + lo.w) + (hi.x + hi.y) + (hi.z + hi.w)) * inv_dim;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const float4 lo = *reinterpret_cast<const float4*>(&red[par][r][0]), hi = *reinterpret_cast<const float4*>(&red[par][r][4]);
-      dot[r] = ((lo.x + lo.y) + (lo.z + lo.w) + (hi.x + hi.y) + (hi.z + hi.w)) * inv_dim;
-      const int64_t row = row0 + r;
+    for (int i = 0; i < NV; ++i) {
+      const int c = (threadIdx.x + i * blockDim.x) * 8;
+      if (c < dim) {
+        float a[8], xh[8], o[8];
+        unpack8(pa[i], a);
+        unpack8(px[i], xh);
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int c = (threadIdx.x + i * blockDim.x) * 8;
-        if (c < dim && row < rows) {
-          float a[8], xh[8], o[8];
-          unpack8(pa[r][i], a);
-          unpack8(px[r][i], xh);
+        for (int j = 0; j < 8; ++j) o[j] = (a[j] * wv[i][j] - xh[j] * rs * dot) * rs;
+        if (ds != nullptr) {
+          float s[8];
+          unpack8(ld8(ds + row * dim + c), s);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = (a[j] * wv[i][j] - xh[j] * rs[r] * dot[r]) * rs[r];
-          if (ds != nullptr) {
-            float s[8];
-            unpack8(ld8(ds + row * dim + c), s);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += s[j];
-          }
-          st8(dx + row * dim + c, pack8(o));
+          for (int j = 0; j < 8; ++j) o[j] += s[j];
         }
+        st8(dx + row * dim + c, pack8(o));
       }
     }
   }
@@ -159,10 +144,11 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1) rmsnorm_bwd_k(const bf16
   }
 }
 
-// The same with rows fetched ahead: a ring of STAGES rows of dy, x and ds per block, filled with 16-byte asynchronous copies.
-// A thread copies exactly the elements it reads itself, so the ring needs no barrier of its own, and the loads of the next
-// rows are in flight while a row's dot product waits at its barrier - which is what bounds the kernel above: 84 -> 60 us at
-// [8192, 4096] with ds inside a training step (four 64 MB streams, 41 us at the copy rate), 4.0 -> 3.6 us at [512, 1024].
+// Up to 8192 columns: rows fetched ahead through a ring of STAGES rows of dy, x and ds per block, filled with 16-byte asynchronous
+// copies.  A thread copies exactly the elements it reads itself, so the ring needs no barrier of its own, and the loads of the
+// next rows are in flight while a row's dot product waits at its barrier - which bounds a kernel that loads a row when it gets
+// to it: 84 -> 60 us at [8192, 4096] with ds inside a training step (four 64 MB streams, 41 us at the copy rate), 4.0 -> 3.6 us
+// at [512, 1024].
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src) : "memory");
 }

@@ -68,7 +68,7 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
 // ------------------------------------------------------------------------------------------- prep
 // delta_pad / lse2_pad: [H, Tpad] fp32 holding -delta and -lse * log2(e); Tpad multiple of 128; rows >= T are zero.
 //
-// stat_tiles: [H, Tpad / 128, 2] tiles of 4 KB for the dK/dV kernel, which adds the per-query-column terms to S^T and
+// stat_tiles: [H, Tpad / 128, 2] tiles of 4 KB for the dK/dV CTAs, which add the per-query-column terms to S^T and
 // dP^T with one extra MMA step each instead of reading them in the softmax loop: D[i][j] += sum_k ONES[i][k] * C[j][k]
 // with C[j][0..15] = {hi, lo, 0 x 6, hi, lo, 0 x 6}, hi + lo the bf16 split of HALF the term (both 16-byte halves are
 // equal, so the operand does not depend on which half the hardware takes as k = 0..7).  Tile 0 carries -lse / scale
@@ -1306,12 +1306,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) flash_bwd_pair_kernel(const __
 }  // namespace ody
 
 static long long* g_bwd_trace = nullptr;
-// Optional per-block timelines (dK/dV kernel in the first 48 x 8 stamps, dQ kernel in the next 48 x 8)
-// Optional per-block timeline of CTA (0,0) of the dK/dV kernel: 48 x 8 SM-clock stamps (see the kernel).
+// Optional per-block timelines: SM-clock stamps of the first dK/dV CTA in the first 48 x 8 words, of the first dQ CTA in the
+// next 48 x 8 (see dkdv_cta and dq_cta).
 extern "C" void ody_flash_bwd_set_trace(long long* buf) { g_bwd_trace = buf; }
 
 static int g_bwd_variant = 1;
-// 1 (default): the split pair (dK/dV kernel + dQ kernel: seven products per block pair, no atomics, bitwise
+// 1 (default): the split pair (dK/dV CTAs and dQ CTAs in one launch: seven products per block pair, no atomics, bitwise
 // reproducible); 0: the fused dK/dV/dQ kernel (five products; dQ summed over KV tiles with fp32 reductions in no fixed
 // order - at present the reduction traffic, not the tensor core, bounds it, and the split pair is the faster one)
 extern "C" int ody_flash_bwd_set_variant(int v) {

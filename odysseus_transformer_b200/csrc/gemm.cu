@@ -464,13 +464,6 @@ extern "C" int64_t ody_gemm_split_bytes(int M, int N, int K) {
   return s > 1 ? (int64_t)s * M * N * 4 : 0;
 }
 
-template <int LAYOUT>
-static int gemm_split(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-                      int accumulate, const void* c_in, int64_t ld_in, const ody::RopeEpi& rp, int* err, cudaStream_t st, float* ws,
-                      int splits) {
-  return ody::launch_gemm<LAYOUT, false, true>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, ws, splits);
-}
-
 // ody_gemm_bf16_ex with scratch (16-byte aligned, ody_gemm_split_bytes of the sizes): products with few tiles split K.
 extern "C" int ody_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                                 int64_t ldc, int layout, int accumulate, const OdyEpilogue* epi, void* ws, int64_t ws_bytes,
@@ -487,9 +480,9 @@ extern "C" int ody_gemm_bf16_ws(const void* A, const void* B, void* C, int M, in
   if (rp.cos != nullptr && layout != 0) return (int)cudaErrorInvalidValue;
   const int splits = gemm_splits(M, N, K);
   switch (layout) {
-    case 0: return gemm_split<0>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
-    case 1: return gemm_split<1>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
-    case 2: return gemm_split<2>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
+    case 0: return ody::launch_gemm<0, false, true>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
+    case 1: return ody::launch_gemm<1, false, true>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
+    case 2: return ody::launch_gemm<2, false, true>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, c_in, ld_in, rp, err, st, (float*)ws, splits);
   }
   return (int)cudaErrorInvalidValue;
 }

@@ -46,15 +46,15 @@ int ody_ce_grad(void* logits, const int64_t* targets, float* loss, const float* 
 int ody_ce_bwd(void* logits, const int64_t* targets, const float* lse, const float* scale, int64_t T, int64_t V,
                int64_t ignore_index, cudaStream_t stream);
 
-// ---- AdamW on flat shards: fp32 master / m / v, bf16 grad in, bf16 param out.  guard (device, may be null):
-// dst = src * scale[0] over n bf16 values (n % 8 == 0; dst may be src)
+// ---- dst = src * scale[0] over n bf16 values (n % 8 == 0; dst may be src)
 int ody_scale(void* dst, const void* src, const float* scale, int64_t n, cudaStream_t stream);
-// dst = src * scale[0] over n bf16 values (n % 8 == 0; dst may be src)
-int ody_scale(void* dst, const void* src, const float* scale, int64_t n, cudaStream_t stream);
-// dw [vocab, dim] bf16 = 0, then dw[ids[t]] += dy[t] for t < T (bf16 sums in memory, in no fixed order); an id outside
+
+// ---- dw [vocab, dim] bf16 = 0, then dw[ids[t]] += dy[t] for t < T (bf16 sums in memory, in no fixed order); an id outside
 // [0, vocab) is skipped and reported in *err (device, may be null)
 int ody_embedding_grad(const void* dy, const int64_t* ids, void* dw, int64_t T, int dim, int64_t vocab, int* err,
                        cudaStream_t stream);
+
+// ---- AdamW on flat shards: fp32 master / m / v, bf16 grad in, bf16 param out.  guard (device, may be null):
 // when *guard != 0 at run time the kernel changes nothing (a failed step must not reach the master weights).
 int ody_adamw(float* master, float* m, float* v, const void* grad, void* param, int64_t n, float lr, float beta1,
               float beta2, float eps, float weight_decay, int step, float grad_scale, const float* guard,
@@ -109,7 +109,7 @@ int ody_flash_fwd(const void* q, const void* k, const void* v, void* o, float* l
 // ---- attention backward.  workspace: ody_flash_bwd_workspace_bytes(Tq, H) bytes of scratch, 16-byte aligned.
 // dq/dk/dv may be row-pitched views (e.g. slices of one packed gradient tensor).
 int64_t ody_flash_bwd_workspace_bytes(int Tq, int H);
-/* 1 (default): dK/dV kernel + dQ kernel, no atomics; 0: one fused dK/dV/dQ kernel, dQ summed with fp32 reductions */
+/* 1 (default): dK/dV and dQ CTAs in one launch, no atomics; 0: one fused dK/dV/dQ kernel, dQ summed with fp32 reductions */
 int ody_flash_bwd_set_variant(int variant);
 /* CTAs of the forward grid (one per 256 query rows and head): the upper bound of a push description's n_cta */
 int ody_flash_fwd_ctas(int Tq, int H);

@@ -342,10 +342,11 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int a_mn_ma
 // ------------------------------------------------------------------------------------------- rotary embedding in a GEMM epilogue
 // The output columns are heads of 128 in groups of `period_cols`; the first `rot_cols` columns of every group belong
 // to heads that are rotated (q and k of a packed q|k|v projection), with the two halves of a head 64 columns apart.
-// An epilogue thread owns one output row and takes the accumulator in chunks of 64 columns, so a chunk is one half of
-// a head: it reads the other half (64 TMEM columns up or down) next to its own and writes
+// An epilogue thread owns one output row and writes
 //   low half:  x_lo * cos - x_hi * sin        high half:  x_hi * cos + x_lo * sin
-// with cos / sin [rows, 64] fp32 indexed by the output row.  cos == nullptr switches it off.
+// with cos / sin [rows, 64] fp32 indexed by the output row.  cos == nullptr switches it off.  Two forms: rope_epi_head takes
+// both halves of a head at once (gemm.cu, gemm_2cta.cu); rope_epi_apply takes one 64-column chunk, i.e. one half, and
+// reads the other (64 TMEM columns up or down) next to it (gemm_comm.cu, whose epilogue hands on chunk by chunk).
 struct RopeEpi {
   const float* cos;
   const float* sin;

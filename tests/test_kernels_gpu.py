@@ -670,7 +670,7 @@ def test_rmsnorm_bwd_weight_gradient_in_bf16(lib, rows, dim):
 
 
 @pytest.mark.parametrize("with_ds", [False, True])
-@pytest.mark.parametrize("rows,dim", [(1500, 4096), (900, 8192), (1190, 1000)])
+@pytest.mark.parametrize("rows,dim", [(1500, 4096), (900, 8192), (1190, 1000), (700, 16384)])
 def test_rmsnorm_bwd_slots_are_reused(lib, rows, dim, with_ds):
     """More rows to a block than the ring of fetched rows has slots (4), so that every slot is filled again: against fp32
     PyTorch, one rounding to bf16 for dx, fp32 sums over the rows for dw."""
