@@ -4,9 +4,10 @@
 // grouped queries on one key / value head, then leave most SMs idle behind the longest CTA (10007 tokens, 4 query heads on 1
 // kv head: the dK/dV grid is 79 CTAs of up to 316 blocks for 148 SMs, where an even share would be 85 blocks).  With a split
 // a tile of `units` blocks is walked by ceil(units / len) CTAs, each writes its fp32 partial result to scratch memory, and
-// one more kernel adds the partials in a fixed order (so results stay reproducible) and rounds once.  Measured: backward of
-// that case 847 -> 480 us, its forward 169 -> 136; 1531 tokens, 8 heads on 2: backward 132 -> 71 us; 300 queries on 8000
-// keys, 2 heads: forward 128 -> 32 us, backward 128 -> 48.
+// one more kernel adds the partials in a fixed order (so results stay reproducible) and rounds once.  This step alone, both
+// sides in one run: backward of that case 847 -> 480 us, its forward 169 -> 136.  Together with the CTA order, the dQ
+// kernel's halves and the one launch of both gradient grids, again in one run: that case 738 -> 361 and 159 -> 128; 1531 tokens, 8
+// heads on 2: backward 120 -> 58, forward 32 -> 28; 300 queries on 8000 keys, 2 heads: forward 118 -> 31, backward 120 -> 46.
 #pragma once
 #include <limits.h>
 #include <stdint.h>

@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(256, 1) rmsnorm_bwd_k(const bf16* __restrict__
 // Up to 8192 columns: rows fetched ahead through a ring of STAGES rows of dy, x and ds per block, filled with 16-byte asynchronous
 // copies.  A thread copies exactly the elements it reads itself, so the ring needs no barrier of its own, and the loads of the
 // next rows are in flight while a row's dot product waits at its barrier - which bounds a kernel that loads a row when it gets
-// to it: 84 -> 60 us at [8192, 4096] with ds inside a training step (four 64 MB streams, 41 us at the copy rate), 4.0 -> 3.6 us
-// at [512, 1024].
+// to it.  With the column sum below, alone: 95 -> 62 us at [8192, 4096] with ds (four 64 MB streams, 41 us at the copy rate),
+// 140 -> 69 at [4096, 8192], 17 -> 15 at [512, 1024].
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src) : "memory");
 }
@@ -419,7 +419,8 @@ __global__ void __launch_bounds__(512) ce_fwd_k(const bf16* __restrict__ logits,
 
 // Loss and gradient of a row in one kernel, for callers that know the scale before they see the loss (the chunked lm_head +
 // loss): the second pass over the row reads it from the L2 (two blocks of 1024 threads per SM, so at most 296 rows are open,
-// 76 MB at 128256 words) and writes the gradient over it.  12288 tokens x 128256: 2586 us for the two kernels, 2197 in one.
+// 76 MB at 128256 words) and writes the gradient over it.  4096 tokens x 128256: 624 us for the two kernels, 529 in one; 8192 x
+// 32000: 337 and 319.
 __global__ void __launch_bounds__(1024, 2) ce_grad_k(bf16* logits, const int64_t* __restrict__ targets,
                                                      float* __restrict__ loss, const float* __restrict__ scale, int64_t V,
                                                      int64_t ignore_index) {
@@ -467,8 +468,8 @@ __global__ void ce_bwd_k(bf16* __restrict__ logits, const int64_t* __restrict__ 
 
 // ------------------------------------------------------------------------------------------- scaling by a device scalar
 
-// dst = src * scale[0], eight values per thread (dst may be src); bound by memory.  A [128256, 4096] gradient and [12288, 4096]
-// rows: 476 us, where a broadcast multiplication by a 0-d tensor took 1503 and a copy of its result 348.
+// dst = src * scale[0], eight values per thread (dst may be src); bound by memory.  [128256, 4096]: 338 us, where a broadcast
+// multiplication by a 0-d tensor and a copy of its result took 1449.
 __global__ void __launch_bounds__(256) scale_k(bf16* dst, const bf16* src, const float* __restrict__ scale, int64_t n) {
   const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
   if (i >= n) return;
@@ -483,8 +484,9 @@ __global__ void __launch_bounds__(256) scale_k(bf16* dst, const bf16* src, const
 // ------------------------------------------------------------------------------------------- embedding gradient
 
 // dw[ids[t]] += dy[t] in bf16: one thread per 8 columns of a token, one 16-byte vector reduction each.  Tokens that share a
-// row add in no fixed order, as with index_add.  An id outside the table is skipped and reported.  Reads dy once; bound by memory: 36 us at 8192 tokens x 4096, where index_add
-// with its scalar reductions took 345.
+// row add in no fixed order, as with index_add.  An id outside the table is skipped and reported.  Reads dy once; bound by
+// memory.  With the zero fill of dw: 75 us at 8192 tokens of 32000 x 4096, where the fill and index_add with its scalar
+// reductions took 353; 204 and 693 at 12288 of 128256.
 __global__ void __launch_bounds__(256) embedding_grad_k(const bf16* __restrict__ dy, const int64_t* __restrict__ ids,
                                                         bf16* __restrict__ dw, int64_t total, int vpr, int64_t vocab,
                                                         int* __restrict__ err) {

@@ -976,8 +976,8 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* 
 // dS_h of a half depend only on that half.  The kernel is bound by the softmax warps (exponentials of one special-function
 // unit per scheduler, then dS): with one barrier per block the two warps of a scheduler computed exponentials at the same
 // time and dS at the same time, so the unit idled during dS; the halves drift apart and one warp's exponentials run under
-// the other's dS.  It costs twice the instructions for S and dP (64 keys each), which the pipe has room for.  Backward of
-// 8192 tokens x 32 heads 1785 -> 1689 us, 32768 x 4 3093 -> 2896, 12288 x 32 (8 kv heads) 3720 -> 3434.
+// the other's dS.  It costs twice the instructions for S and dP (64 keys each), which the pipe has room for.  This step alone,
+// backward of 8192 tokens x 32 heads 1785 -> 1689 us, 32768 x 4 3093 -> 2896, 12288 x 32 (8 kv heads) 3720 -> 3434.
 constexpr int K_STAGES = 3;
 constexpr int HALF = BLK / 2;                    // keys per softmax warpgroup
 struct BarsQ {
@@ -1275,7 +1275,7 @@ __device__ __forceinline__ void dq_cta(const int cta, const __nv_bfloat16* __res
 
 // Both grids in one launch: CTAs 0 .. n_kv - 1 are the dK/dV grid, the others the dQ grid.  They share nothing but their inputs;
 // in one launch the dQ CTAs fill the SMs that the dK/dV grid's last wave leaves idle (4096 queries on 8192 keys, 32 heads on 8:
-// 512 dK/dV CTAs are 3.5 waves), and a small problem runs both side by side.  Backward of that case 1635 -> 1537 us, 2048
+// 512 dK/dV CTAs are 3.5 waves), and a small problem runs both side by side.  This step alone: backward of that case 1635 -> 1537 us, 2048
 // tokens x 32 heads 177 -> 173, 32768 x 4 2906 -> 2885, 8192 x 32 (many waves) unchanged.
 struct PairArgs {
   CUtensorMap tmQ, tmDO, tmK, tmV, tmDK, tmDV, tmDQ;
