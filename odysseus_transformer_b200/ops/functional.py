@@ -36,11 +36,18 @@ class _NoBackward:
 def call(fn, *args):
     """``fn.apply(*args)``, without autograd's wrapping when gradients are off: evaluation of a short prompt is bound by the
     host, and the wrapping was a third of a call's time there (logits of 128 tokens, two layers).  Whatever else looks at
-    ``apply`` - functorch transforms, forward-mode levels, tracing, compilation - still gets it."""
+    ``apply`` - functorch transforms and tensors left over from one, forward-mode levels, tracing, compilation - still gets it."""
     if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
             or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling()):
         return fn.apply(*args)
-    return fn.forward(_NoBackward(), *args)
+    try:
+        return fn.forward(_NoBackward(), *args)
+    except RuntimeError:
+        # a tensor that outlived a functorch transform: kernels cannot read it, apply unwraps it.  Looked for here and not
+        # beforehand, where it took 20 us of a call of 270.
+        if any(isinstance(a, torch.Tensor) and torch._C._functorch.is_functorch_wrapped_tensor(a) for a in args):
+            return fn.apply(*args)
+        raise
 
 
 # ----------------------------------------------------------------------------- GEMM primitives

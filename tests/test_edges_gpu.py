@@ -145,3 +145,18 @@ def test_embedding_gradient_reports_ids_outside_the_table(lib, bad):
     want[7] = 0
     assert torch.equal(dw, want)
     _check_status(lib)
+
+
+def test_evaluation_of_a_tensor_left_over_from_a_transform(lib):
+    """A tensor that outlived a functorch transform goes to the kernels as ``apply`` hands it on: unwrapped."""
+    from odysseus_transformer_b200.ops import functional as F
+    kept, x, w = [], _rand(40, 64), _rand(64)
+
+    def f(t):
+        kept.append(t)
+        return (t * t).sum()
+    torch.func.grad(f)(x)
+    with torch.no_grad():
+        for fn in (lambda t: F.rmsnorm(t, w, 1e-5), lambda t: F.linear(t, x), F.swiglu):
+            assert torch.equal(fn(kept[0]), fn(x))
+    _check_status(lib)

@@ -49,3 +49,28 @@ def test_transforms_are_not_bypassed():
             d = torch.autograd.forward_ad.make_dual(x[0], torch.ones_like(x[0]))
             with pytest.raises((RuntimeError, NotImplementedError)):
                 F.linear(d, w)
+
+
+def test_tensors_left_over_from_a_transform_are_unwrapped():
+    """``apply`` unwraps a tensor that outlived its transform; a kernel cannot read one and says so."""
+    kept = []
+
+    def f(x):
+        kept.append(x)
+        return (x * x).sum()
+    torch.func.grad(f)(torch.ones(3, 8))
+
+    class Kernel(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x, n):
+            if torch._C._functorch.is_functorch_wrapped_tensor(x):
+                raise RuntimeError("no storage")
+            if n < 0:
+                raise RuntimeError("refused")
+            return x * n
+    with torch.no_grad():
+        assert torch.equal(F.call(Kernel, kept[0], 2.0), torch.full((3, 8), 2.0))
+        with pytest.raises(RuntimeError, match="refused"):
+            F.call(Kernel, torch.ones(2), -1.0)
+        with pytest.raises(RuntimeError, match="refused"):
+            F.call(Kernel, kept[0], -1.0)
