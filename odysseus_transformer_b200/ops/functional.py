@@ -24,6 +24,9 @@ from . import native, torch_ref as R
 # ----------------------------------------------------------------------------- calling autograd functions
 
 
+_profiler_enabled = torch._C._autograd._profiler_enabled
+
+
 class _NoBackward:
     """Stands in for an autograd function's ``ctx`` where no backward can follow."""
 
@@ -36,9 +39,10 @@ class _NoBackward:
 def call(fn, *args):
     """``fn.apply(*args)``, without autograd's wrapping when gradients are off: evaluation of a short prompt is bound by the
     host, and the wrapping was a third of a call's time there (logits of 128 tokens, two layers).  Whatever else looks at
-    ``apply`` - functorch transforms and tensors left over from one, forward-mode levels, tracing, compilation - still gets it."""
+    ``apply`` - functorch transforms and tensors left over from one, forward-mode levels, tracing, compilation, a profiler that
+    wants the operators' names - still gets it."""
     if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
-            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling()):
+            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or _profiler_enabled()):
         return fn.apply(*args)
     try:
         return fn.forward(_NoBackward(), *args)

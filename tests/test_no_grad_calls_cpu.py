@@ -74,3 +74,12 @@ def test_tensors_left_over_from_a_transform_are_unwrapped():
             F.call(Kernel, torch.ones(2), -1.0)
         with pytest.raises(RuntimeError, match="refused"):
             F.call(Kernel, kept[0], -1.0)
+
+
+def test_a_profile_names_the_operators():
+    calls = _calls()
+    with torch.no_grad(), torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        calls["rmsnorm"]()
+        calls["linear"]()
+    names = {e.name for e in prof.events()}
+    assert {"_RMSNorm", "_Linear"} <= names
