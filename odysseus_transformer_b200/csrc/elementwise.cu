@@ -10,6 +10,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "ody_kernels.h"
 #include "sm100.cuh"
 
@@ -22,6 +23,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_k(const bf16* __restrict__ x,
                                                      const bf16* __restrict__ w, bf16* __restrict__ sum_out,
                                                      bf16* __restrict__ y, float* __restrict__ rstd, int dim,
                                                      float eps) {
+  after_previous_kernel(x, delta, w);
   __shared__ float red[33];
   const int64_t row = blockIdx.x;
   const bf16* xr = x + row * dim;
@@ -70,6 +72,7 @@ __global__ void __launch_bounds__(256, 1) rmsnorm_bwd_k(const bf16* __restrict__
                                                      const bf16* __restrict__ w, const float* __restrict__ rstd,
                                                      const bf16* __restrict__ ds, bf16* __restrict__ dx,
                                                      float* __restrict__ dw_partial, int64_t rows, int dim) {
+  after_previous_kernel(dy, x, w, rstd, ds);
   __shared__ __align__(16) float red[2][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float wv[NV][8], acc[NV][8];
@@ -162,6 +165,7 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1) rmsnorm_bwd_ring_k(const
                                                           const bf16* __restrict__ w, const float* __restrict__ rstd,
                                                           const bf16* __restrict__ ds, bf16* __restrict__ dx,
                                                           float* __restrict__ dw_partial, int64_t rows, int dim) {
+  after_previous_kernel(dy, x, w, rstd, ds);
   extern __shared__ __align__(16) uint8_t ring_raw[];
   constexpr int NT = DS ? 3 : 2;
   bf16x8* ring = reinterpret_cast<bf16x8*>(ring_raw);          // [STAGES][NT][NV][256]
@@ -268,6 +272,7 @@ __device__ __forceinline__ void store_sum(float* p, float v) { *p = v; }
 __device__ __forceinline__ void store_sum(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 template <typename OUT>
 __global__ void __launch_bounds__(1024) colsum_k(const float* __restrict__ partial, OUT* __restrict__ out, int nblocks, int dim) {
+  after_previous_kernel(partial);
   __shared__ float red[32][33];
   const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -288,6 +293,7 @@ __global__ void __launch_bounds__(1024) colsum_k(const float* __restrict__ parti
 
 __global__ void rope_tables_k(const int64_t* __restrict__ pos, float* __restrict__ cos_o, float* __restrict__ sin_o,
                               int64_t T, int half, float theta) {
+  after_previous_kernel(pos);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T * half) return;
   const int k = (int)(i % half);
@@ -307,6 +313,7 @@ template <bool COPY>
 __global__ void rope_k(const bf16* __restrict__ src, bf16* __restrict__ dst, const float* __restrict__ cos_t,
                        const float* __restrict__ sin_t, int64_t T, int groups, int period, int n_rot, int head_dim,
                        int64_t src_stride, int64_t dst_stride, int inverse) {
+  after_previous_kernel(src, cos_t, sin_t);
   const int half = head_dim >> 1;
   const int vec_per_head = half >> 3;
   const int per_group = COPY ? period : n_rot;
@@ -347,6 +354,7 @@ __global__ void rope_k(const bf16* __restrict__ src, bf16* __restrict__ dst, con
 // ------------------------------------------------------------------------------------------- SwiGLU
 
 __global__ void swiglu_fwd_k(const bf16* __restrict__ gu, bf16* __restrict__ h, int64_t T, int64_t I) {
+  after_previous_kernel(gu);
   const int64_t vpr = I >> 3;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T * vpr) return;
@@ -361,6 +369,7 @@ __global__ void swiglu_fwd_k(const bf16* __restrict__ gu, bf16* __restrict__ h, 
 
 __global__ void swiglu_bwd_k(const bf16* __restrict__ dh, const bf16* __restrict__ gu, bf16* __restrict__ dgu,
                              int64_t T, int64_t I) {
+  after_previous_kernel(dh, gu);
   const int64_t vpr = I >> 3;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T * vpr) return;
@@ -406,6 +415,7 @@ __device__ __forceinline__ float row_lse(const bf16* lr, int64_t V, float* red) 
 __global__ void __launch_bounds__(512) ce_fwd_k(const bf16* __restrict__ logits, const int64_t* __restrict__ targets,
                                                 float* __restrict__ loss, float* __restrict__ lse, int64_t V,
                                                 int64_t ignore_index) {
+  after_previous_kernel(logits, targets);
   __shared__ float red[33];
   const int64_t row = blockIdx.x;
   const bf16* lr = logits + row * V;
@@ -424,6 +434,7 @@ __global__ void __launch_bounds__(512) ce_fwd_k(const bf16* __restrict__ logits,
 __global__ void __launch_bounds__(1024, 2) ce_grad_k(bf16* logits, const int64_t* __restrict__ targets,
                                                      float* __restrict__ loss, const float* __restrict__ scale, int64_t V,
                                                      int64_t ignore_index) {
+  after_previous_kernel(logits, targets, scale);
   __shared__ float red[33];
   const int64_t row = blockIdx.x;
   bf16* lr = logits + row * V;
@@ -448,6 +459,7 @@ __global__ void __launch_bounds__(1024, 2) ce_grad_k(bf16* logits, const int64_t
 
 __global__ void ce_bwd_k(bf16* __restrict__ logits, const int64_t* __restrict__ targets, const float* __restrict__ lse,
                          const float* __restrict__ scale, int64_t V, int64_t ignore_index) {
+  after_previous_kernel(logits, targets, lse, scale);
   const int64_t row = blockIdx.y;
   const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (c >= V) return;
@@ -471,6 +483,7 @@ __global__ void ce_bwd_k(bf16* __restrict__ logits, const int64_t* __restrict__ 
 // dst = src * scale[0], eight values per thread (dst may be src); bound by memory.  [128256, 4096]: 338 us, where a broadcast
 // multiplication by a 0-d tensor and a copy of its result took 1449.
 __global__ void __launch_bounds__(256) scale_k(bf16* dst, const bf16* src, const float* __restrict__ scale, int64_t n) {
+  after_previous_kernel(src, scale);
   const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
   if (i >= n) return;
   const float sc = scale[0];
@@ -490,6 +503,7 @@ __global__ void __launch_bounds__(256) scale_k(bf16* dst, const bf16* src, const
 __global__ void __launch_bounds__(256) embedding_grad_k(const bf16* __restrict__ dy, const int64_t* __restrict__ ids,
                                                         bf16* __restrict__ dw, int64_t total, int vpr, int64_t vocab,
                                                         int* __restrict__ err) {
+  after_previous_kernel(dy, ids);
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total) return;
   const int64_t t = i / vpr;
@@ -511,6 +525,7 @@ __global__ void adamw_k(float* __restrict__ master, float* __restrict__ m, float
                         const bf16* __restrict__ grad, bf16* __restrict__ param, int64_t n, float decay, float beta1,
                         float beta2, float step_size, float inv_sqrt_bc2, float eps, float grad_scale,
                         const float* __restrict__ guard) {
+  after_previous_kernel(master, m, v, grad, guard);
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (i >= n) return;
   // a non-zero guard word (the step's kernel status, summed over ranks) means some gradient is incomplete:
@@ -671,7 +686,7 @@ extern "C" int ody_rmsnorm_fwd(const void* x, const void* delta, const void* w, 
   if (rows == 0) return 0;
   const int nv = (dim + 2047) / 2048;
 #define L(NV)                                                                                               \
-  rmsnorm_fwd_k<NV><<<(unsigned)rows, 256, 0, st>>>((const bf16*)x, (const bf16*)delta, (const bf16*)w,    \
+  launch_kernel(rmsnorm_fwd_k<NV>, (unsigned)rows, 256, 0, st, 1, (const bf16*)x, (const bf16*)delta, (const bf16*)w,    \
                                                     (bf16*)sum_out, (bf16*)y, rstd, dim, eps)
   if (nv <= 1) L(1); else if (nv <= 2) L(2); else if (nv <= 4) L(4); else L(8);
 #undef L
@@ -695,7 +710,7 @@ static int launch_norm_ring(const void* dy, const void* x, const void* w, const 
     if (e != cudaSuccess) return (int)e;
     if (dev <= 63) configured.fetch_or(1ull << dev, std::memory_order_relaxed);
   }
-  rmsnorm_bwd_ring_k<NV, DS><<<nb, 256, SMEM, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)ds,
+  launch_kernel(rmsnorm_bwd_ring_k<NV, DS>, nb, 256, SMEM, st, 1, (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)ds,
                                                     (bf16*)dx, dw_partial, rows, dim);
   return last_err();
 }
@@ -716,13 +731,13 @@ extern "C" int ody_rmsnorm_bwd_to(const void* dy, const void* x, const void* w, 
   if (dim <= 2048) R(1); else if (dim <= 4096) R(2); else if (dim <= 8192) R(4);
 #undef R
   else   // a ring of such rows does not fit the shared memory
-    rmsnorm_bwd_k<8><<<nb, 256, 0, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)ds,
+    launch_kernel(rmsnorm_bwd_k<8>, nb, 256, 0, st, 1, (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)ds,
                                          (bf16*)dx, dw_partial, rows, dim);
   if (e) return e;
   if (dw_bf16)
-    colsum_k<bf16><<<blocks_for(dim, 32), 1024, 0, st>>>(dw_partial, (bf16*)dw, nb, dim);
+    launch_kernel(colsum_k<bf16>, blocks_for(dim, 32), 1024, 0, st, 1, dw_partial, (bf16*)dw, nb, dim);
   else
-    colsum_k<float><<<blocks_for(dim, 32), 1024, 0, st>>>(dw_partial, (float*)dw, nb, dim);
+    launch_kernel(colsum_k<float>, blocks_for(dim, 32), 1024, 0, st, 1, dw_partial, (float*)dw, nb, dim);
   return last_err();
 }
 
@@ -730,7 +745,7 @@ extern "C" int ody_rope_tables(const int64_t* positions, float* cos_out, float* 
                                float theta, cudaStream_t st) {
   const int half = head_dim / 2;
   if (T == 0) return 0;
-  rope_tables_k<<<blocks_for(T * half, 256), 256, 0, st>>>(positions, cos_out, sin_out, T, half, theta);
+  launch_kernel(rope_tables_k, blocks_for(T * half, 256), 256, 0, st, 1, positions, cos_out, sin_out, T, half, theta);
   return last_err();
 }
 
@@ -745,10 +760,10 @@ extern "C" int ody_rope(const void* src, void* dst, const float* cos_t, const fl
   const int64_t total = T * groups * (copy ? period : n_rot) * (head_dim / 16);
   if (total == 0) return 0;
   if (copy)
-    rope_k<true><<<blocks_for(total, 256), 256, 0, st>>>((const bf16*)src, (bf16*)dst, cos_t, sin_t, T, groups, period,
+    launch_kernel(rope_k<true>, blocks_for(total, 256), 256, 0, st, 1, (const bf16*)src, (bf16*)dst, cos_t, sin_t, T, groups, period,
                                                          n_rot, head_dim, src_stride, dst_stride, inverse);
   else
-    rope_k<false><<<blocks_for(total, 256), 256, 0, st>>>((const bf16*)src, (bf16*)dst, cos_t, sin_t, T, groups, period,
+    launch_kernel(rope_k<false>, blocks_for(total, 256), 256, 0, st, 1, (const bf16*)src, (bf16*)dst, cos_t, sin_t, T, groups, period,
                                                           n_rot, head_dim, src_stride, dst_stride, inverse);
   return last_err();
 }
@@ -762,14 +777,14 @@ extern "C" int ody_rope_inplace(void* x, const float* cos_t, const float* sin_t,
 extern "C" int ody_swiglu_fwd(const void* gu, void* h, int64_t T, int64_t I, cudaStream_t st) {
   if (I % 8 != 0) return (int)cudaErrorInvalidValue;
   if (T * I == 0) return 0;
-  swiglu_fwd_k<<<blocks_for(T * (I / 8), 256), 256, 0, st>>>((const bf16*)gu, (bf16*)h, T, I);
+  launch_kernel(swiglu_fwd_k, blocks_for(T * (I / 8), 256), 256, 0, st, 1, (const bf16*)gu, (bf16*)h, T, I);
   return last_err();
 }
 
 extern "C" int ody_swiglu_bwd(const void* dh, const void* gu, void* dgu, int64_t T, int64_t I, cudaStream_t st) {
   if (I % 8 != 0) return (int)cudaErrorInvalidValue;
   if (T * I == 0) return 0;
-  swiglu_bwd_k<<<blocks_for(T * (I / 8), 256), 256, 0, st>>>((const bf16*)dh, (const bf16*)gu, (bf16*)dgu, T, I);
+  launch_kernel(swiglu_bwd_k, blocks_for(T * (I / 8), 256), 256, 0, st, 1, (const bf16*)dh, (const bf16*)gu, (bf16*)dgu, T, I);
   return last_err();
 }
 
@@ -777,7 +792,7 @@ extern "C" int ody_ce_fwd(const void* logits, const int64_t* targets, float* los
                           int64_t ignore_index, cudaStream_t st) {
   if (V % 8 != 0) return (int)cudaErrorInvalidValue;
   if (T == 0) return 0;
-  ce_fwd_k<<<(unsigned)T, 512, 0, st>>>((const bf16*)logits, targets, loss, lse, V, ignore_index);
+  launch_kernel(ce_fwd_k, (unsigned)T, 512, 0, st, 1, (const bf16*)logits, targets, loss, lse, V, ignore_index);
   return last_err();
 }
 
@@ -785,7 +800,7 @@ extern "C" int ody_ce_grad(void* logits, const int64_t* targets, float* loss, co
                            int64_t ignore_index, cudaStream_t st) {
   if (V % 8 != 0) return (int)cudaErrorInvalidValue;
   if (T == 0) return 0;
-  ce_grad_k<<<(unsigned)T, 1024, 0, st>>>((bf16*)logits, targets, loss, scale, V, ignore_index);
+  launch_kernel(ce_grad_k, (unsigned)T, 1024, 0, st, 1, (bf16*)logits, targets, loss, scale, V, ignore_index);
   return last_err();
 }
 
@@ -794,14 +809,14 @@ extern "C" int ody_ce_bwd(void* logits, const int64_t* targets, const float* lse
   if (V % 8 != 0 || T > 65535) return (int)cudaErrorInvalidValue;
   if (T == 0) return 0;
   dim3 grid(blocks_for(V / 8, 256), (unsigned)T);
-  ce_bwd_k<<<grid, 256, 0, st>>>((bf16*)logits, targets, lse, scale, V, ignore_index);
+  launch_kernel(ce_bwd_k, grid, 256, 0, st, 1, (bf16*)logits, targets, lse, scale, V, ignore_index);
   return last_err();
 }
 
 extern "C" int ody_scale(void* dst, const void* src, const float* scale, int64_t n, cudaStream_t st) {
   if (n % 8 != 0 || (((uintptr_t)dst | (uintptr_t)src) & 15)) return (int)cudaErrorInvalidValue;
   if (n == 0) return 0;
-  scale_k<<<blocks_for(n / 8, 256), 256, 0, st>>>((bf16*)dst, (const bf16*)src, scale, n);
+  launch_kernel(scale_k, blocks_for(n / 8, 256), 256, 0, st, 1, (bf16*)dst, (const bf16*)src, scale, n);
   return last_err();
 }
 
@@ -812,7 +827,7 @@ extern "C" int ody_embedding_grad(const void* dy, const int64_t* ids, void* dw, 
   if (e != cudaSuccess) return (int)e;
   const int64_t total = T * (dim / 8);
   if (total == 0) return 0;
-  embedding_grad_k<<<blocks_for(total, 256), 256, 0, st>>>((const bf16*)dy, ids, (bf16*)dw, total, dim / 8, vocab, err);
+  launch_kernel(embedding_grad_k, blocks_for(total, 256), 256, 0, st, 1, (const bf16*)dy, ids, (bf16*)dw, total, dim / 8, vocab, err);
   return last_err();
 }
 
@@ -823,7 +838,7 @@ extern "C" int ody_adamw(float* master, float* m, float* v, const void* grad, vo
   if (n == 0) return 0;
   const double bc1 = 1.0 - pow((double)beta1, (double)step);
   const double bc2 = 1.0 - pow((double)beta2, (double)step);
-  adamw_k<<<blocks_for(n / 8, 256), 256, 0, st>>>(master, m, v, (const bf16*)grad, (bf16*)param, n,
+  launch_kernel(adamw_k, blocks_for(n / 8, 256), 256, 0, st, 1, master, m, v, (const bf16*)grad, (bf16*)param, n,
                                                   1.f - lr * weight_decay, beta1, beta2, (float)(lr / bc1),
                                                   (float)(1.0 / sqrt(bc2)), eps, grad_scale, guard);
   return last_err();

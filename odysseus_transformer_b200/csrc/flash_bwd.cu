@@ -23,6 +23,7 @@
 // of one packed [T, hq + 2 hkv, 128] gradient tensor.
 #include "ody_kernels.h"
 #include "sm100.cuh"
+#include "launch.cuh"
 #include "attn_split.cuh"
 
 // Of every ODY_BWD_POLY_DEN column pairs, the first ODY_BWD_POLY_NUM take their exponentials on the FMA pipe
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const __nv_bfloat16* __restri
                             const float* __restrict__ lse, float* __restrict__ delta_pad, float* __restrict__ lse2_pad,
                             uint8_t* __restrict__ stat_tiles, float inv_scale,
                             int T, int Tpad, int H, int64_t do_row, int64_t o_row) {
+  after_previous_kernel(dO, O, lse);
   const int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wg >= (int64_t)(Tpad / 8) * H) return;
@@ -169,6 +171,7 @@ struct PartDests { __nv_bfloat16* out[2]; int64_t ld[2]; };
 template <int N_OUT>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ part, const PartDests d, int T, int heads,
                                                         const SplitUnits units, const SplitPlan plan) {
+  after_previous_kernel(part);
   const int tile = blockIdx.x, head = blockIdx.y;
   const int n_parts = plan.parts(units(tile));
   const int r = blockIdx.z * 16 + (threadIdx.x >> 4), c = (threadIdx.x & 15) * 8;
@@ -256,6 +259,7 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  after_previous_kernel(stat_tiles);
 
   if (warp < 4) {
    reg_dec<REGS_ISSUE>();
@@ -1051,6 +1055,7 @@ __device__ __forceinline__ void dq_cta(const int cta, const __nv_bfloat16* __res
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  after_previous_kernel(qg, dog, lse2_pad, delta_pad);
 
   if (warp < 4) {
    reg_dec<REGS_ISSUE>();
@@ -1439,7 +1444,7 @@ extern "C" int ody_flash_bwd_parts(const void* dO, const void* q, const void* k,
     const int64_t warps = (int64_t)(Tpad / 8) * H;
     const int threads = 256;
     const int64_t blocks = (warps * 32 + threads - 1) / threads;
-    prep_kernel<<<(unsigned)blocks, threads, 0, st>>>((const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, delta_pad,
+    launch_kernel(prep_kernel, (unsigned)blocks, threads, 0, st, 1, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, delta_pad,
                                                       lse2_pad, stat_tiles, 1.f / scale, Tq, Tpad, H, do_row, o_row);
   }
   CUtensorMap tQ, tDO, tK, tV, tDQ, tDK, tDV;
@@ -1486,14 +1491,14 @@ extern "C" int ody_flash_bwd_parts(const void* dO, const void* q, const void* k,
   pa.q_part = (float*)((uint8_t*)parts + kv_bytes);
   pa.dbg = g_bwd_trace; pa.err = err;
   pa.n_kv = (int)ctas_kv; pa.Tq = Tq; pa.Tk = Tk; pa.Tq_pad = Tpad; pa.H = H; pa.Hkv = Hkv; pa.causal = causal; pa.scale = scale;
-  flash_bwd_pair_kernel<<<(unsigned)(ctas_kv + ctas_q), NUM_THREADS, PAIR_SMEM_TOTAL, st>>>(pa);
+  launch_kernel(flash_bwd_pair_kernel, (unsigned)(ctas_kv + ctas_q), NUM_THREADS, PAIR_SMEM_TOTAL, st, 1, pa);
   if (pkv.max_parts > 1) {
     const PartDests d = {{(__nv_bfloat16*)dv, (__nv_bfloat16*)dk}, {dv_row, dk_row}};
-    sum_parts_kernel<2><<<dim3(kv_tiles, Hkv, BIG / 16), 256, 0, st>>>(pa.kv_part, d, Tk, Hkv, ukv, pkv);
+    launch_kernel(sum_parts_kernel<2>, dim3(kv_tiles, Hkv, BIG / 16), 256, 0, st, 1, pa.kv_part, d, Tk, Hkv, ukv, pkv);
   }
   if (pq.max_parts > 1) {
     const PartDests d = {{(__nv_bfloat16*)dq, nullptr}, {dq_row, 0}};
-    sum_parts_kernel<1><<<dim3(q_tiles, H, BIG / 16), 256, 0, st>>>(pa.q_part, d, Tq, H, uq, pq);
+    launch_kernel(sum_parts_kernel<1>, dim3(q_tiles, H, BIG / 16), 256, 0, st, 1, pa.q_part, d, Tq, H, uq, pq);
   }
   return (int)cudaGetLastError();
 }

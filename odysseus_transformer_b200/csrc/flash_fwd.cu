@@ -27,6 +27,7 @@
 
 #include "ody_kernels.h"
 #include "sm100.cuh"
+#include "launch.cuh"
 #include "peer_comm.cuh"
 #include "attn_split.cuh"
 
@@ -159,6 +160,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  if constexpr (!PUSH) after_previous_kernel();      // a launch that waits for peers lets nothing in behind it
 
   if (warp >= 12) {
     // ------------------------------------------------------------------ comm warps (PUSH only)
@@ -506,6 +508,7 @@ __global__ void __launch_bounds__(256) merge_parts_kernel(const float* __restric
                                                           __nv_bfloat16* __restrict__ o, float* __restrict__ lse, int Tq, int H,
                                                           int64_t o_row, const SplitUnits units, const SplitPlan plan) {
   const int pair = blockIdx.x, head = blockIdx.y;
+  after_previous_kernel(part, part_ml);
   const int n_parts = plan.parts(units(pair));
   const int r = blockIdx.z * 16 + (threadIdx.x >> 4), c = (threadIdx.x & 15) * 8;
   const int row = pair * CTA_ROWS + r;
@@ -663,11 +666,11 @@ extern "C" int ody_flash_fwd_parts(const void* q, const void* k, const void* v, 
     else
       flash_fwd_kernel<true, false><<<grid, NUM_THREADS_PUSH, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, push->n_cta, sm, plan, part, part_ml);
   } else if (ks32) {
-    flash_fwd_kernel<false, true><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm, plan, part, part_ml);
+    launch_kernel(flash_fwd_kernel<false, true>, grid, NUM_THREADS, SMEM_TOTAL, st, 1, tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm, plan, part, part_ml);
   } else {
-    flash_fwd_kernel<false, false><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm, plan, part, part_ml);
+    launch_kernel(flash_fwd_kernel<false, false>, grid, NUM_THREADS, SMEM_TOTAL, st, 1, tQ, tK, tV, tO, lse, Tq, Tk, H, Hkv, causal, scale, err, pp, 0, sm, plan, part, part_ml);
   }
   if (plan.max_parts > 1)
-    merge_parts_kernel<<<dim3(pairs, H, CTA_ROWS / 16), 256, 0, st>>>(part, part_ml, (__nv_bfloat16*)o, lse, Tq, H, o_row, units, plan);
+    launch_kernel(merge_parts_kernel, dim3(pairs, H, CTA_ROWS / 16), 256, 0, st, 1, part, part_ml, (__nv_bfloat16*)o, lse, Tq, H, o_row, units, plan);
   return (int)cudaGetLastError();
 }

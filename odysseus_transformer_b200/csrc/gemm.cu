@@ -15,6 +15,7 @@
 // gemm_2cta.cu holds the same GEMM on CTA pairs (cta_group::2); ody_gemm_bf16 at the end of this file chooses.
 #include "ody_kernels.h"
 #include "sm100.cuh"
+#include "launch.cuh"
 
 namespace ody {
 
@@ -110,6 +111,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  after_previous_kernel(c_in);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -310,6 +312,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 __global__ void __launch_bounds__(256) splitk_sum_kernel(const float* __restrict__ part, int splits, int M, int N,
                                                          const __nv_bfloat16* c_in, int64_t ld_in, int accumulate, const RopeEpi rp,
                                                          __nv_bfloat16* C, int64_t ldc) {
+  after_previous_kernel(part, c_in);
   const int vpr = N / 8;
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= (int64_t)M * vpr) return;
@@ -386,12 +389,11 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (r) return 720000 + r;
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * splits;
   const int grid = tiles < g_num_sms ? tiles : g_num_sms;
-  gemm_bf16_kernel<LAYOUT, ROPE, SPLIT><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tA, tB, tC, (const __nv_bfloat16*)c_in, M, N, K, ld_in,
-                                                                  accumulate, mn3d, rp, err,
-                                                                  part, splits);
+  launch_kernel(gemm_bf16_kernel<LAYOUT, ROPE, SPLIT>, grid, NUM_THREADS, SMEM_TOTAL, st, 1, tA, tB, tC, (const __nv_bfloat16*)c_in,
+                M, N, K, ld_in, accumulate, mn3d, rp, err, part, splits);
   if (SPLIT)
-    splitk_sum_kernel<<<(unsigned)(((int64_t)M * (N / 8) + 255) / 256), 256, 0, st>>>(part, splits, M, N, (const __nv_bfloat16*)c_in, ld_in,
-                                                                                      accumulate, rp, (__nv_bfloat16*)C, ldc);
+    launch_kernel(splitk_sum_kernel, (unsigned)(((int64_t)M * (N / 8) + 255) / 256), 256, 0, st, 1, part, splits, M, N,
+                  (const __nv_bfloat16*)c_in, ld_in, accumulate, rp, (__nv_bfloat16*)C, ldc);
   return (int)cudaGetLastError();
 }
 

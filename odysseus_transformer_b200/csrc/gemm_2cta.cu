@@ -21,6 +21,7 @@
 // thread reaches them on every path.
 #include "ody_kernels.h"
 #include "sm100.cuh"
+#include "launch.cuh"
 
 // defined in gemm.cu: validates an epilogue description and resolves it into kernel arguments
 extern "C" int ody_gemm_resolve_epilogue(const OdyEpilogue* epi, const void* C, int M, int N, int64_t ldc, int* accumulate,
@@ -181,6 +182,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   cluster_sync_all();          // both CTAs' barriers exist before anything may signal them from the other side
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  after_previous_kernel(c_in);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (each CTA loads its own halves)
@@ -379,19 +381,19 @@ static int launch(const void* A, const void* B, void* C, int M, int N, int K, in
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = SMEM_TOTAL;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   if (g_max_pairs == 0) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = SMEM_TOTAL;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     int dev = 0, sms = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -415,10 +417,9 @@ static int launch(const void* A, const void* B, void* C, int M, int N, int K, in
   if (r) return 720000 + r;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
   const int pairs = tiles < g_max_pairs ? tiles : g_max_pairs;
-  cfg.gridDim = dim3(2 * pairs);
   const __nv_bfloat16* c_in = (const __nv_bfloat16*)c_src;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm2_bf16_kernel<LAYOUT, ROPE>, tA, tB, tC, c_in, M, N, K, ld_in, accumulate, mn3d, rp, err);
-  return (int)e;
+  return launch_kernel(gemm2_bf16_kernel<LAYOUT, ROPE>, 2 * pairs, NUM_THREADS, SMEM_TOTAL, st, 2, tA, tB, tC, c_in, M, N, K, ld_in,
+                       accumulate, mn3d, rp, err);
 }
 
 }  // namespace g2

@@ -160,3 +160,45 @@ def test_evaluation_of_a_tensor_left_over_from_a_transform(lib):
         for fn in (lambda t: F.rmsnorm(t, w, 1e-5), lambda t: F.linear(t, x), F.swiglu):
             assert torch.equal(fn(kept[0]), fn(x))
     _check_status(lib)
+
+
+def test_back_to_back_launches(lib):
+    """Kernels come in while their predecessor drains: a chain in which each reads what the one before wrote gives the bits it
+    gives with the GPU waited for after every call, over small and full grids."""
+    def chain(T, wait):
+        torch.manual_seed(T)
+        x, w, wq, wo = _rand(T, 1024), _rand(1024) + 1, _rand(1536, 1024, scale=0.03), _rand(1024, 1024, scale=0.03)
+        pos, tg = torch.arange(T, device="cuda"), torch.randint(1024, (T,), device="cuda")
+        big = _rand(8192, 8192)
+        torch.cuda.synchronize()
+        kept = []
+        for _ in range(0 if wait else 8):                # about 6 ms of work, so that the calls below queue up behind it
+            lib.gemm(big, big, None, 0, False)
+
+        def do(r):
+            if wait:
+                torch.cuda.synchronize()
+            return r
+        for _ in range(6):
+            cos, sin = do(lib.rope_tables(pos, 128, 10000.0))
+            h, rstd = do(lib.rmsnorm_fwd(x, w, 1e-5))
+            qkv = do(lib.gemm(h, wq, None, 0, False, (cos, sin, 1280, 1536), None)).view(T, 12, 128)
+            q, k, v = qkv[:, :8], qkv[:, 8:10], qkv[:, 10:]
+            o, lse = do(lib.attn_fwd(q, k, v, True, 0.1))
+            y = do(lib.gemm(o.view(T, 1024), wo, None, 0, False, None, x))
+            act = do(lib.swiglu_fwd(torch.cat([y, y], 1)))
+            dgu = do(lib.swiglu_bwd(act, torch.cat([y, y], 1)))
+            dx, dw = do(lib.rmsnorm_bwd(dgu[:, :1024].contiguous(), x, w, rstd, y))
+            d = do(lib.attn_bwd(dx.view(T, 8, 128), q, k, v, o, lse, True, 0.1, None, None, None))
+            do(lib.rope_inplace_(d[0], 8, cos, sin, True))
+            g = do(lib.gemm(d[0].view(T, 1024), y, None, 2, False))
+            loss, l2 = do(lib.ce_fwd(y, tg, -100))
+            z = y.clone()
+            do(lib.ce_bwd_(z, tg, l2, torch.ones(1, device="cuda"), -100))
+            kept += [h, qkv, o, lse, y, act, dgu, dx, dw, *d, g, loss, z]
+            x = (y.float() / y.float().pow(2).mean().sqrt()).to(torch.bfloat16)
+        return kept
+    for T in (1, 300, 4096):
+        got, want = chain(T, False), chain(T, True)
+        _check_status(lib)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
