@@ -21,18 +21,12 @@
 // Splitting dQ from dK/dV recomputes S and dP once more but needs no atomics and is deterministic.
 // Gradients are written with TMA stores through row-pitched tensor maps, so dq/dk/dv may be slices
 // of one packed [T, hq + 2 hkv, 128] gradient tensor.
+#include <type_traits>
+
 #include "ody_kernels.h"
 #include "sm100.cuh"
 #include "launch.cuh"
 #include "attn_split.cuh"
-
-// Of every ODY_BWD_POLY_DEN column pairs, the first ODY_BWD_POLY_NUM take their exponentials on the FMA pipe
-// (exp2_poly2) instead of the special-function unit.  Measured on B200: any mix is a few percent slower than
-// all-MUFU - the softmax warps are bound by the latency of their dependent chains, not by either pipe - so it is off.
-#ifndef ODY_BWD_POLY_NUM
-#define ODY_BWD_POLY_NUM 0
-#define ODY_BWD_POLY_DEN 2
-#endif
 
 namespace ody {
 namespace bwd {
@@ -141,7 +135,9 @@ struct BarsKV {
 };
 constexpr int KV_SMEM_TILES = 2 * BIG_BYTES + STAGES * (2 * BLK_BYTES + STAT_BYTES) + STAT_TILE;   // + the all-ones operand
 constexpr int KV_SMEM_TOTAL = KV_SMEM_TILES + 256 + 1024;
-// TMEM columns: S^T 0..127 (P^T, bf16, overwrites 0..63), dP^T 128..255 (dS^T overwrites 128..191), dV 256, dK 384
+// TMEM columns: S^T 0..127 (64 query columns for each of the two softmax warps of a lane quarter; P^T, bf16, overwrites the first
+// 32 of each), dP^T 128..255 (dS^T likewise), dV 256, dK 384
+constexpr int HALF = BLK / 2;                    // streamed rows per softmax warp, in both CTA kinds
 constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
 
 // CTA order of the dK/dV grid.  Causal: the KV tiles of all heads that see the most query blocks (the first ones) come first,
@@ -200,7 +196,15 @@ struct SplitMaps {
   int rows;     // 0 = unused
 };
 
-// One CTA of the dK/dV grid (flash_bwd_pair_kernel below runs it)
+// One CTA of the dK/dV grid (flash_bwd_pair_kernel below runs it).  Its period is a chain - S^T, exponentials, dV and the next S^T -
+// with the tensor pipe idle under the exponentials, so what counts is what the softmax warps do besides them: each writes P^T
+// and dS^T over columns that only it has read, where the two warps of a lane quarter met at a barrier twice a block; blocks
+// off the diagonal run without the masks; TMEM loads come in two pieces, the second under the arithmetic of the first; a
+// warp arrives once, not 32 times.  The same in the dQ CTAs.  Backward, us: 8192 tokens x 32 heads 1682 -> 1570, 32768 x 4 2933 ->
+// 2712, 12288 x 32 on 8 3400 -> 3179, 4096 on 8192 keys x 32 on 8 1540 -> 1404, 2048 x 32 173 -> 158.
+// Measured and not kept: this kernel in two independent 64-query halves, as the dQ CTAs are (1793 us at 8192 x 32: an instruction 64
+// columns wide with both operands in shared memory takes 48 cycles for its reads, not 32); sixteen softmax warps with 32
+// columns each in both (1588); the five-product kernel below with sixteen (1906 -> 1746, 3520 -> 3155 at 32768 x 4).
 __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, const CUtensorMap& tmDO, const CUtensorMap& tmK,
                                          const CUtensorMap& tmV, const CUtensorMap& tmDK, const CUtensorMap& tmDV,
                                          const uint8_t* __restrict__ stat_tiles, int Tq, int Tk, int Tq_pad,
@@ -244,8 +248,8 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
     }
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->p_full, 256);
-    mbar_init(&bars->ds_full, 256);
+    mbar_init(&bars->p_full, 8);                  // one arrival per softmax warp
+    mbar_init(&bars->ds_full, 8);
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->drain, 1);
     bars->abort_flag = 0;
@@ -356,7 +360,7 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
         const uint64_t dmn = desc_advance(d_mn0, stage * BLK_BYTES);
 #pragma unroll
         for (int kk = 0; kk < BLK / 16; ++kk)      // dV += P^T dO
-          if (leader) umma_ts(tmem + COL_DV, tmem + COL_ST + kk * 8, desc_advance(dmn, kk * 2048), IDESC_ACC, kk > 0 ? 1u : acc0);
+          if (leader) umma_ts(tmem + COL_DV, tmem + COL_ST + (kk >> 2) * HALF + (kk & 3) * 8, desc_advance(dmn, kk * 2048), IDESC_ACC, kk > 0 ? 1u : acc0);
         if (leader) umma_commit(&bars->d_empty[stage]);
         if (it + 1 < total && !issue_s(it + 1)) { ok = false; break; }
         if (!mbar_wait(&bars->ds_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
@@ -364,7 +368,7 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
         const uint64_t qmn = desc_advance(q_mn0, stage * BLK_BYTES);
 #pragma unroll
         for (int kk = 0; kk < BLK / 16; ++kk)      // dK += dS^T Q
-          if (leader) umma_ts(tmem + COL_DK, tmem + COL_DPT + kk * 8, desc_advance(qmn, kk * 2048), IDESC_ACC, kk > 0 ? 1u : acc0);
+          if (leader) umma_ts(tmem + COL_DK, tmem + COL_DPT + (kk >> 2) * HALF + (kk & 3) * 8, desc_advance(qmn, kk * 2048), IDESC_ACC, kk > 0 ? 1u : acc0);
         if (leader) umma_commit(&bars->q_empty[stage]);
         if (it + 1 < total && !issue_dp(it + 1)) { ok = false; break; }
       }
@@ -393,78 +397,74 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
       // ---- part 1: S^T -> P^T
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 2] = clock64();                             // S^T(it) complete
+      if (!ok) break;
       uint32_t sv[64];
-      if (ok) {
-        tc_fence_after();
-        tmem_ld_32x32(tmem + COL_ST + hf * 64 + lane_off, sv);
-        tmem_ld_32x32(tmem + COL_ST + hf * 64 + 32 + lane_off, sv + 32);
-        tmem_ld_wait();
-      }
-      // P^T is written over the first 64 columns of S^T: the other warp of this lane quarter must have read
-      // its inputs before either of us stores; the two also agree here on leaving the loop
-      if (!named_barrier_and(4 + q, 64, ok)) { ok = false; break; }
-      if (strace) dbg[it * 8 + 3] = clock64();                             // S^T in registers, pair agreed
-      const bool diag = causal && (qrow0 < kv0 + BIG);     // some (q, kv) pairs of this half block are masked
+      tc_fence_after();
+      tmem_ld_32x32(tmem + COL_ST + hf * HALF + lane_off, sv);
+      tmem_ld_wait32(sv);
+      tmem_ld_32x32(tmem + COL_ST + hf * HALF + 32 + lane_off, sv + 32);   // on its way while the first 32 are worked on
+      if (strace) dbg[it * 8 + 3] = clock64();                             // S^T in registers
       {
         uint32_t pp[32];
+        auto exponentials = [&](auto masked) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          // the accumulator already holds s - lse / scale: x = that * scale * log2(e), two query columns at once
-          const uint64_t x2 = mul2(pk2u(sv[2 * c], sv[2 * c + 1]), sl2_2);
-          float p0, p1;
-          if ((c % ODY_BWD_POLY_DEN) < ODY_BWD_POLY_NUM) {
-            exp2_poly2(x2, p0, p1);
-          } else {
+          for (int c = 0; c < 32; ++c) {
+            if (c == 16) tmem_ld_wait32(sv + 32);
+            // the accumulator already holds s - lse / scale: x = that * scale * log2(e), two query columns at once
+            const uint64_t x2 = mul2(pk2u(sv[2 * c], sv[2 * c + 1]), sl2_2);
+            float p0, p1;
             upk2(x2, p0, p1);
             p0 = exp2_mufu(p0);
             p1 = exp2_mufu(p1);
+            if constexpr (decltype(masked)::value) {
+              if (qrow0 + 2 * c < kv0 + r) p0 = 0.f;
+              if (qrow0 + 2 * c + 1 < kv0 + r) p1 = 0.f;
+            }
+            sv[2 * c] = __float_as_uint(p0);
+            sv[2 * c + 1] = __float_as_uint(p1);
+            pp[c] = pack_bf16(p0, p1);
           }
-          if (diag) {
-            if (qrow0 + 2 * c < kv0 + r) p0 = 0.f;
-            if (qrow0 + 2 * c + 1 < kv0 + r) p1 = 0.f;
-          }
-          sv[2 * c] = __float_as_uint(p0);
-          sv[2 * c + 1] = __float_as_uint(p1);
-          pp[c] = pack_bf16(p0, p1);
-        }
+        };
+        // blocks without masked (q, kv) pairs run an instance without the masks
+        if (causal && qrow0 < kv0 + BIG) exponentials(std::true_type()); else exponentials(std::false_type());
         if (dbg != nullptr) {   // tracing only: pin every packed value before the stamp
           asm volatile("" ::"r"(pp[0]), "r"(pp[1]), "r"(pp[2]), "r"(pp[3]), "r"(pp[4]), "r"(pp[5]), "r"(pp[6]), "r"(pp[7]), "r"(pp[8]), "r"(pp[9]), "r"(pp[10]), "r"(pp[11]), "r"(pp[12]), "r"(pp[13]), "r"(pp[14]), "r"(pp[15]));
           asm volatile("" ::"r"(pp[16]), "r"(pp[17]), "r"(pp[18]), "r"(pp[19]), "r"(pp[20]), "r"(pp[21]), "r"(pp[22]), "r"(pp[23]), "r"(pp[24]), "r"(pp[25]), "r"(pp[26]), "r"(pp[27]), "r"(pp[28]), "r"(pp[29]), "r"(pp[30]), "r"(pp[31]));
         }
         if (strace) dbg[it * 8 + 4] = clock64();                           // P^T computed
-        tmem_st_32x16(tmem + COL_ST + hf * 32 + lane_off, pp);
-        tmem_st_32x16(tmem + COL_ST + hf * 32 + 16 + lane_off, pp + 16);
+        // over the scores that this warp alone has read: no warp waits for another here
+        tmem_st_32x16(tmem + COL_ST + hf * HALF + lane_off, pp);
+        tmem_st_32x16(tmem + COL_ST + hf * HALF + 16 + lane_off, pp + 16);
         tmem_st_wait();
         if (strace) dbg[it * 8 + 5] = clock64();                           // P^T stored
         tc_fence_before();
-        mbar_arrive(&bars->p_full);
+        mbar_arrive_warp(&bars->p_full, lane);
       }
       // ---- part 2: dP^T -> dS^T = P^T * (dP^T - delta) * scale
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
       uint32_t dp[64];
-      if (ok) {
-        tc_fence_after();
-        tmem_ld_32x32(tmem + COL_DPT + hf * 64 + lane_off, dp);
-        tmem_ld_32x32(tmem + COL_DPT + hf * 64 + 32 + lane_off, dp + 32);
-        tmem_ld_wait();
-      }
-      if (!named_barrier_and(4 + q, 64, ok)) { ok = false; break; }
-      if (strace) dbg[it * 8 + 6] = clock64();                             // dP^T in registers, pair agreed
+      tc_fence_after();
+      tmem_ld_32x32(tmem + COL_DPT + hf * HALF + lane_off, dp);
+      tmem_ld_wait32(dp);
+      tmem_ld_32x32(tmem + COL_DPT + hf * HALF + 32 + lane_off, dp + 32);
+      if (strace) dbg[it * 8 + 6] = clock64();                             // dP^T in registers
       {
         uint32_t ds[32];
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
+          if (c == 16) tmem_ld_wait32(dp + 32);
           // dS = P * (dP - delta), the accumulator already holding dP - delta; the softmax scale is applied once, to
           // dK, in the epilogue
           float d0, d1;
           upk2(mul2(pk2u(sv[2 * c], sv[2 * c + 1]), pk2u(dp[2 * c], dp[2 * c + 1])), d0, d1);
           ds[c] = pack_bf16(d0, d1);
         }
-        tmem_st_32x16(tmem + COL_DPT + hf * 32 + lane_off, ds);
-        tmem_st_32x16(tmem + COL_DPT + hf * 32 + 16 + lane_off, ds + 16);
+        tmem_st_32x16(tmem + COL_DPT + hf * HALF + lane_off, ds);
+        tmem_st_32x16(tmem + COL_DPT + hf * HALF + 16 + lane_off, ds + 16);
         tmem_st_wait();
         tc_fence_before();
-        mbar_arrive(&bars->ds_full);
+        mbar_arrive_warp(&bars->ds_full, lane);
       }
       if (strace) dbg[it * 8 + 7] = clock64();
     }
@@ -983,7 +983,6 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* 
 // the other's dS.  It costs twice the instructions for S and dP (64 keys each), which the pipe has room for.  This step alone,
 // backward of 8192 tokens x 32 heads 1785 -> 1689 us, 32768 x 4 3093 -> 2896, 12288 x 32 (8 kv heads) 3720 -> 3434.
 constexpr int K_STAGES = 3;
-constexpr int HALF = BLK / 2;                    // keys per softmax warpgroup
 struct BarsQ {
   uint64_t k_full[K_STAGES], k_empty[K_STAGES];
   uint64_t v_full[K_STAGES], v_empty[K_STAGES];
@@ -1041,9 +1040,9 @@ __device__ __forceinline__ void dq_cta(const int cta, const __nv_bfloat16* __res
     mbar_init(&bars->a_ready, 256);
     for (int h = 0; h < 2; ++h) {
       mbar_init(&bars->s_full[h], 1);
-      mbar_init(&bars->s_free[h], 128);
+      mbar_init(&bars->s_free[h], 4);              // one arrival per softmax warp of the half
       mbar_init(&bars->dp_full[h], 1);
-      mbar_init(&bars->ds_full[h], 128);
+      mbar_init(&bars->ds_full[h], 4);
     }
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->drain, 1);
@@ -1182,48 +1181,48 @@ __device__ __forceinline__ void dq_cta(const int cta, const __nv_bfloat16* __res
       const bool strace = dbg != nullptr && cta == 0 && threadIdx.x == 128 && it < 48;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[hf], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 4] = clock64();                             // S(it) complete
-      uint32_t sv[64];
-      if (ok) {
-        tc_fence_after();
-        tmem_ld_32x32(tmem + COL_S + hf * 64 + lane_off, sv);
-        tmem_ld_32x32(tmem + COL_S + hf * 64 + 32 + lane_off, sv + 32);
-        tmem_ld_wait();
-        tc_fence_before();
-        mbar_arrive(&bars->s_free[hf]);                       // S(it) is in registers
-      }
-      const bool diag = causal && (kvb0 + 63 > q0);
-      const bool tail = kvb0 + 64 > Tk;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        float p0, p1;
-        upk2(fma2(pk2u(sv[2 * c], sv[2 * c + 1]), sl2_2, nlse2_2), p0, p1);
-        p0 = exp2_mufu(p0);
-        p1 = exp2_mufu(p1);
-        if (diag) {
-          if (kvb0 + 2 * c > q0 + r) p0 = 0.f;
-          if (kvb0 + 2 * c + 1 > q0 + r) p1 = 0.f;
-        }
-        if (tail) {
-          if (kvb0 + 2 * c >= Tk) p0 = 0.f;
-          if (kvb0 + 2 * c + 1 >= Tk) p1 = 0.f;
-        }
-        sv[2 * c] = __float_as_uint(p0);
-        sv[2 * c + 1] = __float_as_uint(p1);
-      }
-      if (strace) dbg[it * 8 + 5] = clock64();                             // P computed (as far as the compiler kept it here)
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_full[hf], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
-      if (strace) dbg[it * 8 + 6] = clock64();                             // dP(it) complete
-      uint32_t dp[64];
-      if (ok) {
-        tc_fence_after();
-        tmem_ld_32x32(tmem + COL_DP + hf * 64 + lane_off, dp);
-        tmem_ld_32x32(tmem + COL_DP + hf * 64 + 32 + lane_off, dp + 32);
-        tmem_ld_wait();
-      }
       if (!ok) break;
+      uint32_t sv[64];
+      tc_fence_after();
+      tmem_ld_32x32(tmem + COL_S + hf * HALF + lane_off, sv);
+      tmem_ld_wait32(sv);
+      tmem_ld_32x32(tmem + COL_S + hf * HALF + 32 + lane_off, sv + 32);    // on its way while the first 32 are worked on
+      auto exponentials = [&](auto masked) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          if (c == 16) {
+            tmem_ld_wait32(sv + 32);
+            tc_fence_before();
+            mbar_arrive_warp(&bars->s_free[hf], lane);        // S(it) is in registers
+          }
+          float p0, p1;
+          upk2(fma2(pk2u(sv[2 * c], sv[2 * c + 1]), sl2_2, nlse2_2), p0, p1);
+          p0 = exp2_mufu(p0);
+          p1 = exp2_mufu(p1);
+          if constexpr (decltype(masked)::value) {
+            const int k0 = kvb0 + 2 * c;
+            if (k0 >= Tk || (causal && k0 > q0 + r)) p0 = 0.f;
+            if (k0 + 1 >= Tk || (causal && k0 + 1 > q0 + r)) p1 = 0.f;
+          }
+          sv[2 * c] = __float_as_uint(p0);
+          sv[2 * c + 1] = __float_as_uint(p1);
+        }
+      };
+      // blocks without masked keys (the diagonal, the end of the keys) run an instance without the masks
+      if ((causal && kvb0 + 63 > q0) || kvb0 + 64 > Tk) exponentials(std::true_type()); else exponentials(std::false_type());
+      if (strace) dbg[it * 8 + 5] = clock64();                             // P computed (as far as the compiler kept it here)
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_full[hf], par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
+      if (strace) dbg[it * 8 + 6] = clock64();                             // dP(it) complete
+      if (!ok) break;
+      uint32_t dp[64];
+      tc_fence_after();
+      tmem_ld_32x32(tmem + COL_DP + hf * HALF + lane_off, dp);
+      tmem_ld_wait32(dp);
+      tmem_ld_32x32(tmem + COL_DP + hf * HALF + 32 + lane_off, dp + 32);
       uint32_t ds[32];
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
+        if (c == 16) tmem_ld_wait32(dp + 32);
         // dS = P * (dP - delta); the softmax scale is applied once, to dQ, in the epilogue
         float d0, d1;
         upk2(mul2(pk2u(sv[2 * c], sv[2 * c + 1]), add2(pk2u(dp[2 * c], dp[2 * c + 1]), ndelta_2)), d0, d1);
@@ -1233,7 +1232,7 @@ __device__ __forceinline__ void dq_cta(const int cta, const __nv_bfloat16* __res
       tmem_st_32x16(tmem + COL_DP + hf * HALF + 16 + lane_off, ds + 16);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars->ds_full[hf]);
+      mbar_arrive_warp(&bars->ds_full[hf], lane);
       if (strace) dbg[it * 8 + 7] = clock64();                             // dS published
     }
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_done, 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
