@@ -141,7 +141,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&bars->s_full[t], 1);
-      mbar_init(&bars->p_full[t], 128);
+      mbar_init(&bars->p_full[t], 4);          // one arrival per warp
       mbar_init(&bars->o_done[t], 1);
     }
     mbar_init(&bars->drain, 1);
@@ -330,21 +330,28 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     bool ok = true;
     // Only a tile's last block can hold masked keys (the diagonal, the end of the keys): all others run an instance without
     // the masks (this step alone: 8192 tokens x 32 heads 494 -> 486 us, 32768 x 4 913 -> 896).
-    auto block = [&](int j, auto masked) -> bool {
-      const bool tr = blockIdx.x == 0 && (threadIdx.x == 128 || threadIdx.x == 256);
+    auto block = [&](int j, auto first, auto masked) -> bool {
+      [[maybe_unused]] const bool tr = blockIdx.x == 0 && (threadIdx.x == 128 || threadIdx.x == 256);
       ODY_FWD_STAMP(tr, j, t * 5 + 0);
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[t], j & 1, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (!ok) return false;
       ODY_FWD_STAMP(tr, j, t * 5 + 1);
       tc_fence_after();
+      // The scores come in four pieces of 32 columns.  A tile's first block needs them all for its maximum and the masked block
+      // changes them first; every other block starts its exponentials on the first piece while the next is on its way (with
+      // one arrival a warp: 8192 tokens x 32 heads 494 -> 489 us, 32768 x 4 911 -> 899, 12288 x 32 1037 -> 1028).
+      constexpr bool FIRST = decltype(first)::value, MASKED = decltype(masked)::value;
       uint32_t sv[128];
       tmem_ld_32x32(col_s, sv);
-      tmem_ld_32x32(col_s + 32, sv + 32);
-      tmem_ld_32x32(col_s + 64, sv + 64);
-      tmem_ld_32x32(col_s + 96, sv + 96);
-      tmem_ld_wait();
+      if constexpr (FIRST || MASKED) {
+        tmem_ld_32x32(col_s + 32, sv + 32);
+        tmem_ld_32x32(col_s + 64, sv + 64);
+        tmem_ld_32x32(col_s + 96, sv + 96);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) tmem_ld_wait32(sv + 32 * g);
+      }
       ODY_FWD_STAMP(tr, j, t * 5 + 2);
-      if constexpr (decltype(masked)::value) {
+      if constexpr (MASKED) {
         const int kv0 = (b0 + j) * BN;
         if (b0 + j == diag) {
 #pragma unroll
@@ -363,12 +370,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // separate maximum pass in front of the exponentials; a block that moves it further is redone (rare).
       const uint64_t sl2_2 = pk2(sl2, sl2);
       float rsum, rmax;
-      auto exp_pass = [&]() {
+      auto exp_pass = [&](auto loads) {
         const uint64_t nm_2 = pk2(-m_used, -m_used);
         uint64_t rs2 = pk2(0.f, 0.f);
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
+          if constexpr (decltype(loads)::value) {
+            tmem_ld_wait32(sv + 32 * g);
+            if (g < 3) tmem_ld_32x32(col_s + 32 * (g + 1), sv + 32 * (g + 1));
+          }
           uint32_t pk[16];
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
@@ -390,7 +401,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         rsum = r0 + r1;
         rmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       };
-      if (j == 0) {
+      if constexpr (FIRST) {
         // first block: there is no maximum in use yet
         float mx[4];
 #pragma unroll
@@ -404,10 +415,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // two infinities would make the row NaN although other blocks - or, of a split tile, other parts - are finite
         m_used = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2, -FLT_MAX);
         ODY_FWD_STAMP(tr, j, t * 5 + 3);
-        exp_pass();
+        exp_pass(std::false_type());
       } else {
         ODY_FWD_STAMP(tr, j, t * 5 + 3);
-        exp_pass();
+        exp_pass(std::bool_constant<!MASKED>());
         const float m_new = fmaxf(m_used, rmax * sl2);
         const bool need = (m_new - m_used) > 8.f;
         if (__any_sync(0xffffffffu, need)) {
@@ -425,19 +436,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
             tmem_st_32x16(col_o + c * 16, o);
           }
-          exp_pass();
+          exp_pass(std::false_type());
         }
       }
       l += rsum;
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars->p_full[t]);
+      mbar_arrive_warp(&bars->p_full[t], lane);
       ODY_FWD_STAMP(tr, j, t * 5 + 4);
       return true;
     };
-    for (int j = 0; j + 1 < nt; ++j)
-      if (!block(j, std::false_type())) break;
-    if (ok && nt > 0) block(nt - 1, std::true_type());
+    if (nt == 1) block(0, std::true_type(), std::true_type());
+    if (nt > 1) block(0, std::true_type(), std::false_type());
+    for (int j = 1; ok && j + 1 < nt; ++j) block(j, std::false_type(), std::false_type());
+    if (ok && nt > 1) block(nt - 1, std::false_type(), std::true_type());
     // epilogue: O / l -> bf16 -> swizzled smem (this tile's Q is dead by now) -> TMA store; lse
     if (ok && nt > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t], 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
     uint8_t* stage = sQ + t * TILE_BYTES;
