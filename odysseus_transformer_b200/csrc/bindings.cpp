@@ -63,8 +63,9 @@ void check_bf16(const at::Tensor& t, const char* name) {
 }
 
 // ------------------------------------------------------------------------------------------- GEMM
-at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const c10::optional<at::Tensor>& out, int64_t layout,
-                bool accumulate, const py::object& rope, const c10::optional<at::Tensor>& residual) {
+// bn > 0: gemm_cluster.cu with these tiles and shares of K, whatever the choice would be
+at::Tensor gemm_as(const at::Tensor& a, const at::Tensor& b, const c10::optional<at::Tensor>& out, int64_t layout,
+                   bool accumulate, const py::object& rope, const c10::optional<at::Tensor>& residual, int64_t bn, int64_t splits) {
   check_bf16(a, "a");
   check_bf16(b, "b");
   ody_req(a.dim() == 2 && b.dim() == 2, "gemm expects 2-D operands");
@@ -85,13 +86,26 @@ at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const c10::optional<at
   ody_req(!(accumulate && residual.has_value()), "gemm: accumulate and residual exclude each other");
   ody_req(rope.is_none() || layout == 0, "gemm: the rotary epilogue belongs to layout 0 (a forward projection)");
   if (K == 0) { if (!accumulate) c.zero_(); return c; }
-  const ody::OptionalScratch ws(ody_gemm_split_bytes((int)M, (int)N, (int)K), a);
+  if (bn > 0) {
+    ODY_CHECK(ody_gemm_bf16_cluster(a.data_ptr(), b.data_ptr(), c.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0),
+                                    c.stride(0), (int)layout, accumulate ? 1 : 0, has_epi ? &epi : nullptr, (int)bn, (int)splits,
+                                    status_ptr(a), cur_stream()), "gemm_cluster");
+    ++g_launches;
+    return c;
+  }
+  int plan_bn, plan_splits;
+  const bool cluster = ody_gemm_cluster_plan((int)M, (int)N, (int)K, has_epi && epi.rope_cos != nullptr, &plan_bn, &plan_splits) != 0;
+  const ody::OptionalScratch ws(cluster ? 0 : ody_gemm_split_bytes((int)M, (int)N, (int)K), a);
   ODY_CHECK(ody_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), c.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0),
                              c.stride(0), (int)layout, accumulate ? 1 : 0, has_epi ? &epi : nullptr,
                              ws.ptr(), ws.bytes, status_ptr(a), cur_stream()),
             "gemm");
   g_launches += ws.bytes > 0 ? 2 : 1;      // split: the sum of the shares is a kernel of its own
   return c;
+}
+at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const c10::optional<at::Tensor>& out, int64_t layout,
+                bool accumulate, const py::object& rope, const c10::optional<at::Tensor>& residual) {
+  return gemm_as(a, b, out, layout, accumulate, rope, residual, 0, 0);
 }
 
 // ------------------------------------------------------------------------------------------- RMSNorm
@@ -420,6 +434,8 @@ void ody_register_comm(pybind11::module& m);
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("out") = py::none(), py::arg("layout") = 0,
         py::arg("accumulate") = false, py::arg("rope") = py::none(), py::arg("residual") = py::none());
+  m.def("gemm_cluster", &gemm_as, py::arg("a"), py::arg("b"), py::arg("out") = py::none(), py::arg("layout") = 0,
+        py::arg("accumulate") = false, py::arg("rope") = py::none(), py::arg("residual") = py::none(), py::arg("bn") = 64, py::arg("splits") = 1);
   m.def("gemm_set_variant", [](int64_t v) { ODY_CHECK(ody_gemm_set_variant((int)v), "gemm_set_variant (0 auto, 1 one CTA, 2 CTA pairs)"); });
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("add_rmsnorm_fwd", &add_rmsnorm_fwd);

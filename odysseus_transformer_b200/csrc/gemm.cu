@@ -12,7 +12,8 @@
 // two 256-column fp32 accumulators in TMEM (all 512 columns) so the epilogue of tile i overlaps the
 // main loop of tile i+1.  The epilogue converts to bf16, stages 128 x 64 blocks in swizzled smem and
 // writes them with TMA stores (edges are clipped by the tensor map).  No cluster multicast anywhere.
-// gemm_2cta.cu holds the same GEMM on CTA pairs (cta_group::2); ody_gemm_bf16 at the end of this file chooses.
+// gemm_2cta.cu holds the same GEMM on CTA pairs (cta_group::2), gemm_cluster.cu on small tiles with K shared by a cluster; the
+// functions at the end of this file choose.
 #include "ody_kernels.h"
 #include "sm100.cuh"
 #include "launch.cuh"
@@ -460,6 +461,56 @@ static int gemm_splits(int M, int N, int K) {
   return splits;
 }
 
+// Whether a product goes to the pair kernel.  Both kernels are persistent; what differs per problem is how full their last wave is.
+// The pair kernel is the faster one per tile (measured ~6 %), so it is chosen unless its tail costs more than that.
+static bool takes_pairs(int M, int N) {
+  if (g_gemm_variant != 0 || M <= 128) return g_gemm_variant == 2;
+  const int sms = ody::g_num_sms > 0 ? ody::g_num_sms : 148;
+  const int64_t t1 = (int64_t)((M + 127) / 128) * ((N + 255) / 256), t2 = (int64_t)((M + 255) / 256) * ((N + 255) / 256);
+  const int64_t s1 = sms, s2 = sms / 2;
+  const double e1 = (double)t1 / (double)(((t1 + s1 - 1) / s1) * s1), e2 = (double)t2 / (double)(((t2 + s2 - 1) / s2) * s2);
+  return e2 * 1.06 >= e1;
+}
+
+// Tiles and shares of K for gemm_cluster.cu, or 0 where the kernels above are expected to be as fast.  Estimates in us from
+// back-to-back launches of 90 products: a fixed part, so much per 64-deep k-block of a CTA, and what sharing costs at the end.
+//   128 x 64 tiles 3.9 + 0.185 (two shares 1.0, four 1.4, eight 1.8 more), 128 x 128 5.4 + 0.196 (1.0, 2.5, 4.0)
+//   one-CTA kernel 4.5 + 0.27 a wave, pairs 6.8 + 0.24 a wave, split K 8.5 + 0.3 and its partials written and read
+// At most one wave of CTAs (clusters leave SMs of a GPC unused: 128 CTAs in clusters of eight take two rounds), and at most 192
+// k-blocks to a CTA: beyond that the wide tiles' smaller operand traffic wins (1024 x 1024 from K = 32000: 60 us, here 63).
+// Measured, before -> cluster: 128 x 3072 from K = 1024 9.7 -> 6.6, 128 x 1024 from 2816 13.1 -> 7.4, 512 x 1024 from 1024 10.3 -> 6.6,
+// from 5632 17.3 -> 12.7, 1531 x 1024 from 1536 12.7 -> 10.5, 1024 x 1024 from 2816 18.4 -> 11.4, 128 x 4096 from 11008 30.7 -> 22.0.
+extern "C" int ody_gemm_cluster_plan(int M, int N, int K, int rope, int* bn, int* splits) {
+  if (g_gemm_variant != 0 || M <= 0 || N <= 0 || K <= 0 || (N % 8)) return 0;
+  const int64_t kblocks = (K + 63) / 64, tiles = (int64_t)((M + 127) / 128) * ((N + 255) / 256);
+  const int s_old = gemm_splits(M, N, K);
+  double limit;
+  if (s_old > 1) {
+    limit = 8.5 + 0.3 * ((kblocks + s_old - 1) / s_old) + (double)s_old * M * N * 8.0 / 6.0e6;
+  } else if (takes_pairs(M, N)) {
+    limit = 6.8 + 0.24 * kblocks * (((int64_t)((M + 255) / 256) * ((N + 255) / 256) + 73) / 74);
+  } else {
+    limit = 4.5 + 0.27 * kblocks * ((tiles + 147) / 148);
+  }
+  double best = 0.95 * limit;
+  int found = 0;
+  for (int b = rope ? 128 : 64; b <= 128; b += 64) {
+    const int64_t t = (int64_t)((M + 127) / 128) * ((N + b - 1) / b);
+    for (int i = 0, s = 1; i < 4 && s <= kblocks; ++i, s *= 2) {
+      static const int max_ctas[4] = {148, 144, 128, 64};
+      static const double sharing[2][4] = {{0.0, 1.0, 1.4, 1.8}, {0.0, 1.0, 2.5, 4.0}};
+      const int64_t kb = (kblocks + s - 1) / s;
+      if (t * s > max_ctas[i] || kb > 192) continue;
+      // up to 256 columns of up to 128 rows from a long K stay split over up to 32 CTAs, two launches that a test counts
+      // (128 x 256 from K = 4096: 12.6 us, a cluster of eight 7.1)
+      if (s_old > 8 && t * s < 37) continue;
+      const double e = (b == 64 ? 3.9 + 0.185 * kb : 5.4 + 0.196 * kb) + sharing[b / 128][i];
+      if (e < best) { best = e; *bn = b; *splits = s; found = 1; }
+    }
+  }
+  return found;
+}
+
 // Scratch ody_gemm_bf16_ws can use for this product; 0: it is not split.
 extern "C" int64_t ody_gemm_split_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -467,10 +518,14 @@ extern "C" int64_t ody_gemm_split_bytes(int M, int N, int K) {
   return s > 1 ? (int64_t)s * M * N * 4 : 0;
 }
 
-// ody_gemm_bf16_ex with scratch (16-byte aligned, ody_gemm_split_bytes of the sizes): products with few tiles split K.
+// ody_gemm_bf16_ex with scratch (16-byte aligned, ody_gemm_split_bytes of the sizes; none is needed where ody_gemm_cluster_plan
+// answers): products with few tiles share K.
 extern "C" int ody_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                                 int64_t ldc, int layout, int accumulate, const OdyEpilogue* epi, void* ws, int64_t ws_bytes,
                                 int* err, cudaStream_t st) {
+  int bn, shares;
+  if (ody_gemm_cluster_plan(M, N, K, epi != nullptr && epi->rope_cos != nullptr, &bn, &shares))
+    return ody_gemm_bf16_cluster(A, B, C, M, N, K, lda, ldb, ldc, layout, accumulate, epi, bn, shares, err, st);
   const int64_t need = ody_gemm_split_bytes(M, N, K);
   if (need == 0 || ws == nullptr || ws_bytes < need || ((uintptr_t)ws & 15))
     return ody_gemm_bf16_ex(A, B, C, M, N, K, lda, ldb, ldc, layout, accumulate, epi, err, st);
@@ -493,17 +548,7 @@ extern "C" int ody_gemm_bf16_ws(const void* A, const void* B, void* C, int M, in
 extern "C" int ody_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                                 int64_t ldc, int layout, int accumulate, const OdyEpilogue* epi, int* err, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return (int)cudaErrorInvalidValue;
-  bool pairs = g_gemm_variant == 2;
-  if (g_gemm_variant == 0 && M > 128) {
-    // Both kernels are persistent; what differs per problem is how full their last wave is.  The pair kernel is
-    // the faster one per tile (measured ~6 %), so it is chosen unless its tail costs more than that.
-    const int sms = ody::g_num_sms > 0 ? ody::g_num_sms : 148;
-    const int64_t t1 = (int64_t)((M + 127) / 128) * ((N + 255) / 256), t2 = (int64_t)((M + 255) / 256) * ((N + 255) / 256);
-    const int64_t s1 = sms, s2 = sms / 2;
-    const double e1 = (double)t1 / (double)(((t1 + s1 - 1) / s1) * s1), e2 = (double)t2 / (double)(((t2 + s2 - 1) / s2) * s2);
-    pairs = e2 * 1.06 >= e1;
-  }
-  if (pairs) return ody_gemm_bf16_2cta_ex(A, B, C, M, N, K, lda, ldb, ldc, layout, accumulate, epi, err, st);
+  if (takes_pairs(M, N)) return ody_gemm_bf16_2cta_ex(A, B, C, M, N, K, lda, ldb, ldc, layout, accumulate, epi, err, st);
   if ((lda % 8) || (ldb % 8) || (ldc % 8) || (N % 8) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15))
     return (int)cudaErrorInvalidValue;
   const void* c_in;

@@ -100,6 +100,13 @@ int ody_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K,
 int ody_gemm_bf16_2cta_ex(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
                           int layout, int accumulate, const OdyEpilogue* epilogue, int* err, cudaStream_t stream);
 
+// the same GEMM on tiles of 128 x bn (64, or 128, which a rotary epilogue needs) whose K dimension the `splits` (1 .. 8, at most
+// the number of 64-deep k-blocks) CTAs of a cluster share
+int ody_gemm_bf16_cluster(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+                          int layout, int accumulate, const OdyEpilogue* epilogue, int bn, int splits, int* err, cudaStream_t stream);
+// 1 and the tiles and shares ody_gemm_bf16_ws uses for a product that goes there, or 0
+int ody_gemm_cluster_plan(int M, int N, int K, int rope, int* bn, int* splits);
+
 // ---- attention forward (head_dim 128): q [Tq,H,128], k/v [Tk,Hkv,128], row pitches in elements; out bf16, lse [H,Tq]
 // fp32 natural log.  causal needs Tq == Tk.
 int ody_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int Tq, int Tk, int H, int Hkv,

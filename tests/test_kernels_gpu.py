@@ -733,3 +733,60 @@ def test_model_step_with_optimizer_fused_vs_library():
         for n, want in grads["library"].items():
             rel = ((grads["fused"][n] - want).norm() / (want.norm() + 1e-6)).item()
             assert rel < 0.08, f"{n}, chunks of {rows}: rel grad diff {rel}"      # as for the step without an optimizer
+
+
+# Tiles of 128 x 64 and 128 x 128, K shared by the CTAs of a cluster (csrc/gemm_cluster.cu): one tile and one k-block, rows and
+# columns that end inside a tile, a K that ends inside a k-block, shares of unequal length, more k-blocks than ring slots
+CLUSTER_SHAPES = [(8, 8, 8, 1), (128, 64, 64, 1), (1, 3072, 1024, 8), (130, 72, 200, 3), (264, 200, 456, 2), (512, 1024, 1032, 5),
+                  (304, 264, 4096, 8), (640, 136, 1600, 7), (2000, 320, 1160, 1)]
+
+
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K,shares", CLUSTER_SHAPES)
+def test_gemm_cluster(lib, layout, M, N, K, shares, bn):
+    """Against fp32, within one rounding to bf16 (relative error below 2^-8); accumulating into a strided output, with a residual;
+    twice the same bits."""
+    torch.manual_seed(M + N + K + layout)
+    if layout == 2:
+        M = max(8, M // 8 * 8)
+    a = _rand(M, K) if layout != 2 else _rand(K, M)
+    b = _rand(N, K) if layout == 0 else _rand(K, N)
+    ref = (a.float() if layout != 2 else a.float().t()) @ (b.float().t() if layout == 0 else b.float())
+    c = lib.gemm_cluster(a, b, None, layout, False, None, None, bn, shares)
+    _check_status(lib)
+    assert ((c.float() - ref).norm() / ref.norm()).item() < 2.0 ** -8
+    assert torch.equal(c, lib.gemm_cluster(a, b, None, layout, False, None, None, bn, shares))
+    wide = _rand(M, 2 * N)
+    want, left = wide.float().clone(), wide[:, :N].clone()
+    want[:, N:] += ref
+    lib.gemm_cluster(a, b, wide[:, N:], layout, True, None, None, bn, shares)
+    res = _rand(M, N)
+    y = lib.gemm_cluster(a, b, None, layout, False, None, res, bn, shares)
+    _check_status(lib)
+    assert ((wide.float() - want).norm() / want.norm()).item() < 2.0 ** -8 and torch.equal(wide[:, :N], left)
+    assert ((y.float() - (ref + res.float())).norm() / (ref + res.float()).norm()).item() < 2.0 ** -8
+
+
+@pytest.mark.parametrize("M,shares", [(1, 8), (128, 3), (300, 1)])
+def test_gemm_cluster_rope(lib, M, shares):
+    """The rotary epilogue equals the one-CTA kernel's up to the order of the sums (one bf16 rounding apart where they differ)."""
+    from odysseus_transformer_b200.ops import torch_ref as R
+    torch.manual_seed(M)
+    N, K = 768, 1088
+    a, b, res = _rand(M, K), _rand(N, K), _rand(M, N)
+    cos, sin = R.rope_tables(torch.randint(0, 9999, (M,), device="cuda"), 128, 10000.0)
+    rope = (cos, sin, 256, 384)
+    for r in (None, res):
+        y = lib.gemm_cluster(a, b, None, 0, False, rope, r, 128, shares)
+        with _unsplit(lib):
+            y1 = lib.gemm(a, b, None, 0, False, rope, r)
+        _check_status(lib)
+        assert ((y.float() - y1.float()).norm() / y1.float().norm()).item() < 2e-3
+    with pytest.raises(RuntimeError):
+        lib.gemm_cluster(a, b, None, 0, False, rope, None, 64, shares)        # half a head per tile
+    for bn, n in ((64, 0), (64, 9), (32, 1)):
+        with pytest.raises(RuntimeError):
+            lib.gemm_cluster(a, b, None, 0, False, None, None, bn, n)
+    with pytest.raises(RuntimeError):
+        lib.gemm_cluster(a[:, :64], b[:, :64], None, 0, False, None, None, 64, 2)   # one k-block, two shares
