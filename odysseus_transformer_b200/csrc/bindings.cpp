@@ -430,6 +430,7 @@ void ody_count_launches(int64_t n) { g_launches += n; }
 // attention (defined in attn_bindings.cpp)
 void ody_register_attention(pybind11::module& m);
 void ody_register_comm(pybind11::module& m);
+void ody_register_layer(pybind11::module& m);      // layer_bindings.cpp
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("out") = py::none(), py::arg("layout") = 0,
@@ -466,4 +467,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_launches", &add_launches);
   ody_register_attention(m);
   ody_register_comm(m);
+  ody_register_layer(m);
 }

@@ -27,21 +27,50 @@ Inter-layer activations are ``[T/N, d]``; the residual add happens in the epilog
 """
 from __future__ import annotations
 
+import math
 import zlib
 from typing import Callable, Dict, Optional
 
 import torch
 import torch.nn as nn
+from torch.nn.modules import module as _module
 
 from ..comm import torch_backend as C
 from ..config import ModelConfig
 from ..mesh import ParallelContext, get_context
 from ..ops import functional as F
-from ..parallel.linear import LinearZeRO3, Zero3Schedule, zero3_embedding
+from ..ops import native
+from ..parallel.linear import ColumnParallelLinearAG, LinearZeRO3, RowParallelLinearRS, Zero3Schedule, zero3_embedding
 from ..parallel.odysseus import OdysseusMLP, ReplicatedMLP
 from ..parallel.ring import RingAttention
 from ..parallel.tpsp import TPSPAttention, TPSPMLP
 from ..parallel.ulysses import SequenceParallelAttention
+
+
+# blocks whose forward a layer may run as one node: their projections, heads, and the forwards they are known by
+_ATTENTION = {TPSPAttention: ("n_local_heads", "n_local_kv_heads"), SequenceParallelAttention: ("hq", "hkv"), RingAttention: ("hq", "hkv")}
+_MLP = {OdysseusMLP: ("gate_up_proj", "down_proj"), TPSPMLP: ("w1w3", "w2")}
+_FORWARDS = {c: c.forward for c in (*_ATTENTION, *_MLP, LinearZeRO3, ColumnParallelLinearAG, RowParallelLinearRS)}
+# bytes a layer keeps for its backward up to which it runs as one node: a layer of more tokens keeps the GPU busy longer than its
+# launches take (at 96 MB of the narrowest model its kernels take 500 us, its single calls 350), and goes on freeing activations
+# block by block in backward
+_ONE_NODE_BYTES = 96 << 20
+
+
+def _unwatched(m: nn.Module) -> bool:
+    """``m`` is called as its class defines it: no hooks, no other forward."""
+    return (_FORWARDS.get(type(m)) is type(m).forward and "forward" not in m.__dict__
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
+
+
+def _own_linear(m: nn.Module) -> Optional[torch.Tensor]:
+    """The weight of a projection that is one GEMM on this GPU alone, else ``None``."""
+    if not _unwatched(m) or C.group_size(m.group) > 1:
+        return None
+    if type(m) is not LinearZeRO3 and (m.bias is not None or not m.sequence_parallel or getattr(m, "gather_output", False)
+                                       or not getattr(m, "input_is_parallel", True)):
+        return None
+    return m.weight
 
 
 class DecoderLayer(nn.Module):
@@ -49,6 +78,7 @@ class DecoderLayer(nn.Module):
                  sched: Optional[Zero3Schedule], dtype, device, use_zero3_linear: bool = True, pack_qkv: bool = True):
         super().__init__()
         d = cfg.hidden_size
+        self.pctx = ctx
         self.eps = cfg.rms_norm_eps
         self.input_layernorm = nn.Parameter(torch.ones(d, dtype=dtype, device=device))
         if mode in ("odysseus", "tpsp"):
@@ -67,10 +97,39 @@ class DecoderLayer(nn.Module):
         for p in (self.input_layernorm, self.post_attention_layernorm):
             p.grad_sync_group = ctx.world_group
 
+    def _one_node(self, x, cos, sin):
+        """Arguments of ``F.decoder_layer`` when the layer may run as one autograd node, else ``None``: one GPU, own kernels, few
+        enough tokens that the host's launches bound it, and nothing that wants to see the blocks' single calls."""
+        a, m = self.self_attn, self.mlp
+        heads, names = _ATTENTION.get(type(a)), _MLP.get(type(m))
+        if (heads is None or names is None or self.pctx.inner_size > 1 or self.pctx.ring_size > 1 or a.head_dim != 128
+                or not getattr(a, "pack_weight", True) or not native.use_native(x) or x.dim() != 2 or x.shape[0] == 0
+                or not F.epilogue_fusion("rope") or not native.has_native_attention_bwd() or not F.plain_call()
+                or not (_unwatched(a) and _unwatched(m))
+                or _module._global_forward_hooks or _module._global_forward_pre_hooks
+                or _module._global_backward_hooks or _module._global_backward_pre_hooks):
+            return None
+        w = [_own_linear(p) for p in (a.qkv_proj, a.o_proj, getattr(m, names[0]), getattr(m, names[1]))]
+        if any(t is None or t.dtype != torch.bfloat16 for t in w):
+            return None
+        # norms, residual stream, q|k|v, attention output, gate|up and their product, in bf16
+        if 2 * x.shape[0] * (3 * x.shape[1] + w[0].shape[0] + w[1].shape[1] + w[2].shape[0] + w[3].shape[1]) > _ONE_NODE_BYTES:
+            return None
+        weights = (self.input_layernorm, w[0], w[1], self.post_attention_layernorm, w[2], w[3])
+        if torch.is_grad_enabled() and not all(t.requires_grad for t in weights):
+            return None
+        return x, cos, sin, getattr(a, heads[0]), getattr(a, heads[1]), self.eps, 1.0 / math.sqrt(a.head_dim), weights
+
     def forward(self, x, delta, cos, sin):
         """(x, delta): residual stream and the not-yet-added output of the previous block (None when that block
         added it itself)."""
         if F.epilogue_fusion("residual"):
+            node = self._one_node(x, cos, sin) if delta is None else None
+            if node is not None:
+                try:
+                    return F.decoder_layer(*node), None
+                except torch.OutOfMemoryError:      # the blocks' own calls need less at a time
+                    pass
             # each block's output projection adds the residual stream in its own epilogue; the norms only normalise
             if delta is None:
                 x, h = F.rmsnorm_keep(x, self.input_layernorm, self.eps)

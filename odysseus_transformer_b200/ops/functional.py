@@ -36,13 +36,19 @@ class _NoBackward:
         pass
 
 
+def plain_call() -> bool:
+    """Whether nothing watches or transforms the calls made now: no functorch transform, forward-mode level, tracing, compilation
+    or profile, each of which is to see the single operators."""
+    return not (torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
+                or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or _profiler_enabled())
+
+
 def call(fn, *args):
     """``fn.apply(*args)``, without autograd's wrapping when gradients are off: evaluation of a short prompt is bound by the
     host, and the wrapping was a third of a call's time there (logits of 128 tokens, two layers).  Whatever else looks at
     ``apply`` - functorch transforms and tensors left over from one, forward-mode levels, tracing, compilation, a profiler that
     wants the operators' names - still gets it."""
-    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
-            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or _profiler_enabled()):
+    if torch.is_grad_enabled() or not plain_call():
         return fn.apply(*args)
     try:
         return fn.forward(_NoBackward(), *args)
@@ -195,11 +201,14 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 # ----------------------------------------------------------------------------- RMSNorm
 
 
+def _norm_grad_in_place(w, mg, x) -> bool:
+    return mg.dtype == torch.bfloat16 and mg.shape == w.shape and mg.is_contiguous() and mg.device == x.device
+
+
 def _rmsnorm_bwd_native(dy, x, w, rstd, ds):
     """(dx, gradient of w for autograd or None): the weight gradient goes straight to ``main_grad`` where it can."""
     mg = getattr(w, "main_grad", None)
-    if (mg is not None and not getattr(w, "_grad_written", False) and mg.dtype == torch.bfloat16 and mg.shape == w.shape
-            and mg.is_contiguous() and mg.device == x.device):
+    if mg is not None and not getattr(w, "_grad_written", False) and _norm_grad_in_place(w, mg, x):
         dx, _ = native.lib().rmsnorm_bwd(dy, x, w, rstd, ds, mg)
         w._grad_written = True
         return dx, None
@@ -423,6 +432,47 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
               scale: Optional[float] = None) -> torch.Tensor:
     """Softmax attention, q [T,H,hd], k/v [T,Hkv,hd] (GQA when Hkv < H)."""
     return call(_Attention, q, k, v, causal, scale)
+
+
+# ----------------------------------------------------------------------------- decoder layer as one node
+
+
+class _DecoderLayer(Function):
+    """A whole decoder layer on one GPU: two calls into the extension instead of eight autograd nodes and their single launches.
+    The same kernels in the same order on the same values as the blocks' own calls; what the backward needs is one buffer."""
+
+    @staticmethod
+    def forward(ctx, x, cos, sin, hq, hkv, eps, scale, *weights):
+        keep = any(ctx.needs_input_grad)
+        y, kept = native.lib().decoder_layer_fwd(x, weights, cos, sin, hq, hkv, eps, scale, keep)
+        if keep:
+            ctx.save_for_backward(x, cos, sin, kept, *weights)
+            ctx.args = (hq, hkv, scale)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, cos, sin, kept, *weights = ctx.saved_tensors
+        hq, hkv, scale = ctx.args
+        out, acc = [], []
+        for w in weights:
+            mg, written = getattr(w, "main_grad", None), bool(getattr(w, "_grad_written", False))
+            if mg is not None and w.dim() == 1 and (written or not _norm_grad_in_place(w, mg, x)):
+                mg = None                       # a norm's gradient that deliver_grad has to convert or add
+            out.append(mg)
+            acc.append(written)
+        dx, *dw = native.lib().decoder_layer_bwd(dy.contiguous(), x, weights, cos, sin, kept, hq, hkv, scale, out, acc)
+        for i, (w, mg) in enumerate(zip(weights, out)):
+            if mg is not None:
+                w._grad_written = True
+            elif w.dim() == 1:
+                dw[i] = deliver_grad(w, dw[i])
+        return (dx, None, None, None, None, None, None, *dw)
+
+
+def decoder_layer(x, cos, sin, hq: int, hkv: int, eps: float, scale: float, weights):
+    """``weights``: input norm, q|k|v, output projection, post-attention norm, gate|up and down, all on this GPU."""
+    return call(_DecoderLayer, x, cos, sin, hq, hkv, eps, scale, *weights)
 
 
 # ----------------------------------------------------------------------------- cross-entropy

@@ -202,3 +202,75 @@ def test_back_to_back_launches(lib):
         got, want = chain(T, False), chain(T, True)
         _check_status(lib)
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("mode", ["odysseus", "tpsp", "ulysses", "ring", "dp"])
+@pytest.mark.parametrize("tokens,checkpoint", [(1, False), (300, False), (300, True)])
+def test_decoder_layer_as_one_node(lib, monkeypatch, mode, tokens, checkpoint):
+    """Logits, gradients and updated weights of a step are those of the blocks' own calls: the loss and all that does not follow the
+    embedding's gradient, which is summed in no fixed order, bit for bit.  With a hook on a block its layer keeps those calls."""
+    from odysseus_transformer_b200.config import get_model_config
+    from odysseus_transformer_b200.mesh import ParallelContext, set_context
+    from odysseus_transformer_b200.models import llama
+    from odysseus_transformer_b200.ops import functional as F
+    from odysseus_transformer_b200.train import Trainer
+    ctx = ParallelContext(device=torch.device("cuda", 0), backend="fused")
+    set_context(ctx)
+    cfg = get_model_config("small-gqa")
+    batch = torch.randint(cfg.vocab_size, (1, tokens + 1), generator=torch.Generator().manual_seed(1)).pin_memory()
+    made = []
+    monkeypatch.setattr(F, "decoder_layer", lambda *a, f=F.decoder_layer: made.append(1) or f(*a))
+
+    def run(limit, prepare=None):
+        monkeypatch.setattr(llama, "_ONE_NODE_BYTES", limit)
+        tr = Trainer(cfg, mode, ctx, tokens, lr=1e-3, seed=3, grad_checkpoint=checkpoint)
+        if prepare is not None:
+            prepare(tr.model)
+        made.clear()
+        loss = tr.train_step(batch).clone()
+        n, o, emb = len(made), tr.optimizer, tr.model.embed_tokens.numel()
+        got = [loss, o.flat_grad[emb:].clone(), o.master[emb:].clone()]
+        with torch.no_grad():
+            tr.model.embed_tokens.zero_().add_(0.01)
+            got.append(tr.model(batch[:, :-1].cuda(), torch.arange(tokens, device="cuda").unsqueeze(0)))
+        torch.cuda.synchronize()
+        return n, got
+    n0, want = run(0)
+    n1, got = run(96 << 20)
+    assert n0 == 0 and n1 == 2 * (2 if checkpoint else 1)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    hooked = []
+    n2, other = run(96 << 20, lambda m: m.layers[0].mlp.register_forward_hook(lambda *a: hooked.append(1)))
+    assert n2 == n1 // 2 and hooked and torch.equal(other[0], want[0])
+    _check_status(lib)
+
+
+def test_decoder_layer_node_adds_and_returns_gradients(lib):
+    """Without ``main_grad`` the gradients come back through autograd; with one that is written they are added to it."""
+    from odysseus_transformer_b200.ops import functional as F
+    torch.manual_seed(0)
+    T, d, hq, hkv, inter = 200, 256, 4, 2, 384
+    shapes = [(d,), ((hq + 2 * hkv) * 128, d), (d, hq * 128), (d,), (2 * inter, d), (d, inter)]
+    ws = [torch.nn.Parameter(_rand(*s, scale=0.05) + (1 if len(s) == 1 else 0)) for s in shapes]
+    x, dy = _rand(T, d).requires_grad_(True), _rand(T, d)
+    cos, sin = lib.rope_tables(torch.arange(T, device="cuda"), 128, 10000.0)
+
+    def step():
+        for t in (x, *ws):
+            t.grad = None
+        F.decoder_layer(x, cos, sin, hq, hkv, 1e-5, 128 ** -0.5, ws).backward(dy)
+        return x.grad
+    dx = step()
+    plain = [w.grad.clone() for w in ws]
+    for w in ws:
+        w.main_grad, w._grad_written = torch.full_like(w, float("nan")), False
+    assert torch.equal(step(), dx) and all(w.grad is None and w._grad_written for w in ws)
+    assert all(torch.equal(w.main_grad, g) for w, g in zip(ws, plain))
+    assert torch.equal(step(), dx)
+    _check_status(lib)
+    for w, g in zip(ws, plain):                              # twice the gradient, each sum rounded once to bf16
+        assert ((w.main_grad.float() - 2 * g.float()).norm() / (2 * g.float()).norm()).item() < 2.0 ** -8
+    with pytest.raises(RuntimeError):
+        F.decoder_layer(x, cos[:-1], sin[:-1], hq, hkv, 1e-5, 0.1, ws)
+    with pytest.raises(RuntimeError):
+        F.decoder_layer(x, cos, sin, hq, hkv, 1e-5, 0.1, [*ws[:5], ws[5][:, :-8]])

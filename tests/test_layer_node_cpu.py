@@ -1,0 +1,103 @@
+"""When a decoder layer runs as one autograd node: the calls that must keep the blocks' own path (no kernel is launched here)."""
+import pytest
+import torch
+
+from odysseus_transformer_b200.config import get_model_config
+from odysseus_transformer_b200.mesh import ParallelContext, set_context
+from odysseus_transformer_b200.models import llama
+from odysseus_transformer_b200.ops import functional as F
+from odysseus_transformer_b200.ops import native
+
+TOKENS = 16
+ROW = 2 * (3 * 512 + 1024 + 512 + 192 + 96)      # bytes a token keeps
+
+
+@pytest.fixture
+def layer(request, monkeypatch):
+    monkeypatch.setattr(native, "use_native", lambda t: t.dtype == torch.bfloat16)
+    monkeypatch.setattr(native, "has_native_attention_bwd", lambda: True)
+    ctx = ParallelContext(device=torch.device("cpu"), backend="fused")
+    set_context(ctx)
+    cfg = get_model_config("small-gqa").replace(hidden_size=512, num_attention_heads=4, num_key_value_heads=2, intermediate_size=96)
+    kw = getattr(request, "param", {})
+    return llama.DecoderLayer(cfg, ctx, kw.get("mode", "odysseus"), 0, None, kw.get("dtype", torch.bfloat16), torch.device("cpu"),
+                              kw.get("zero3", True), kw.get("pack", True))
+
+
+def _node(layer, dtype=torch.bfloat16, tokens=TOKENS):
+    cos, sin = F.rope_tables(torch.arange(TOKENS), 128, 10000.0)
+    return layer._one_node(torch.empty(tokens, 512, dtype=dtype), cos, sin)
+
+
+@pytest.mark.parametrize("layer", [{"mode": m} for m in ("odysseus", "tpsp", "ulysses", "ring", "dp")], indirect=True)
+def test_taken_on_one_gpu(layer):
+    args = _node(layer)
+    weights = args[-1]
+    assert args[3:5] == (4, 2) and len(weights) == 6 and all(a.requires_grad for a in weights)
+    assert [tuple(t.shape) for t in weights] == [(512,), (1024, 512), (512, 512), (512,), (192, 512), (512, 96)]
+
+
+@pytest.mark.parametrize("layer", [{"pack": False}, {"zero3": False}, {"dtype": torch.float32}], indirect=True)
+def test_other_blocks_keep_their_path(layer):
+    assert _node(layer) is None
+
+
+def test_watched_or_changed_layers_keep_their_path(layer, monkeypatch):
+    assert _node(layer) is not None
+    for m in (layer.self_attn, layer.mlp, layer.self_attn.qkv_proj, layer.self_attn.o_proj, layer.mlp.gate_up_proj, layer.mlp.down_proj):
+        for register in (m.register_forward_hook, m.register_forward_pre_hook, m.register_full_backward_hook):
+            h = register(lambda *a: None)
+            assert _node(layer) is None
+            h.remove()
+        m.forward = lambda *a, **k: None
+        assert _node(layer) is None
+        del m.forward
+    h = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    assert _node(layer) is None
+    h.remove()
+    with monkeypatch.context() as p:
+        p.setattr(type(layer.mlp), "forward", lambda self, x, residual=None: x)
+        assert _node(layer) is None
+    layer.self_attn.qkv_proj.sequence_parallel = False
+    assert _node(layer) is None
+    layer.self_attn.qkv_proj.sequence_parallel = True
+    layer.self_attn.o_proj.bias = torch.nn.Parameter(torch.zeros(512, dtype=torch.bfloat16))
+    assert _node(layer) is None
+    layer.self_attn.o_proj.bias = None
+    layer.mlp.down_proj.weight.requires_grad_(False)
+    assert _node(layer) is None
+    with torch.no_grad():
+        assert _node(layer) is not None
+
+
+def test_other_calls_keep_their_path(layer):
+    assert _node(layer, dtype=torch.float32) is None
+    assert _node(layer, tokens=0) is None
+    assert _node(layer, tokens=llama._ONE_NODE_BYTES // ROW) is not None
+    assert _node(layer, tokens=llama._ONE_NODE_BYTES // ROW + 1) is None
+    keep = F.fuse_epilogues()
+    try:
+        F.fuse_epilogues(rope=False)
+        assert _node(layer) is None
+    finally:
+        F.fuse_epilogues(**keep)
+    with torch.autograd.forward_ad.dual_level():
+        assert _node(layer) is None
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]):
+        assert _node(layer) is None
+    seen = []
+    torch.func.vmap(lambda t: seen.append(_node(layer)) or t)(torch.zeros(2))
+    assert seen == [None]
+
+
+def test_blocks_run_by_themselves_when_memory_is_short(layer, monkeypatch):
+    def full(*args):
+        raise torch.OutOfMemoryError("no memory")
+    monkeypatch.setattr(F, "decoder_layer", full)
+    called = []
+    layer.self_attn.forward = lambda h, cos, sin, residual=None: called.append("attention") or residual
+    layer.mlp.forward = lambda h, residual=None: called.append("mlp") or residual
+    monkeypatch.setattr(layer, "_one_node", lambda *a: (1,))
+    monkeypatch.setattr(F, "rmsnorm_keep", lambda x, w, eps: (x, x))
+    y, delta = layer(torch.zeros(2, 512, dtype=torch.bfloat16), None, None, None)
+    assert called == ["attention", "mlp"] and delta is None and y.shape == (2, 512)
