@@ -8,13 +8,12 @@
 //            fma / add instructions), both padded to 128 rows.
 //   dkdv   : one CTA per (128-row KV tile, kv head).  K and V stay in shared memory; 128-row blocks of Q
 //            and dO stream through two TMA rings.  S^T = K Q^T and dP^T = V dO^T land in TMEM (kv rows on
-//            lanes), eight warps (two per lane quarter, 64 columns each) turn them into P^T and dS^T (bf16,
-//            written back over the same TMEM columns) and the tensor core accumulates dV += P^T dO,
-//            dK += dS^T Q in TMEM (128 + 128 + 128 + 128 = 512 columns).  Every tcgen05.mma is 128x128x16:
-//            a single thread issues one instruction per ~80 cycles whatever its shape, so 64-wide blocks
-//            would leave the tensor core half idle.  S^T / dP^T are single buffered; the issue order
-//            dV(i), S^T(i+1), dK(i), dP^T(i+1) keeps the in-order tensor pipe busy while the softmax warps
-//            work on the other matrix.  Query heads sharing the kv head are looped inside.
+//            lanes), eight warps (two per lane quarter, 64 columns each) turn them into P^T and dS^T (bf16, both
+//            written over the columns of dP^T) and the tensor core accumulates dV += P^T dO, dK += dS^T Q in
+//            TMEM (128 + 128 + 128 + 128 = 512 columns).  Every tcgen05.mma is 128x128x16: with both operands in
+//            shared memory an instruction of 64 columns takes 48 cycles, one of 128 takes 64.  S^T / dP^T are
+//            single buffered; the issue order S^T(i+1), dK(i), dV(i), dP^T(i+1) lets the exponentials of block
+//            i+1 run under the other three products.  Query heads sharing the kv head are looped inside.
 //   dq     : one CTA per (128-row query tile, head).  Q and dO stay in TMEM; 128-row blocks of K and V stream.
 //            S = Q K^T, dP = dO V^T, dS (bf16 in TMEM) and dQ += dS K, each in two independent 64-key halves.
 //
@@ -128,15 +127,15 @@ struct BarsKV {
   uint64_t kv_full;
   uint64_t q_full[STAGES], q_empty[STAGES];      // Q block + its lse2 / delta rows
   uint64_t d_full[STAGES], d_empty[STAGES];      // dO block
-  uint64_t s_full, dp_full, p_full, ds_full;     // one completion per block each: parity = block & 1
+  uint64_t s_full, s_free, dp_full, ds_full;     // one completion per block each: parity = block & 1
   uint64_t acc_done, drain;
   uint32_t tmem_base;
   int abort_flag;
 };
 constexpr int KV_SMEM_TILES = 2 * BIG_BYTES + STAGES * (2 * BLK_BYTES + STAT_BYTES) + STAT_TILE;   // + the all-ones operand
 constexpr int KV_SMEM_TOTAL = KV_SMEM_TILES + 256 + 1024;
-// TMEM columns: S^T 0..127 (64 query columns for each of the two softmax warps of a lane quarter; P^T, bf16, overwrites the first
-// 32 of each), dP^T 128..255 (dS^T likewise), dV 256, dK 384
+// TMEM columns: S^T 0..127, dP^T 128..255 (64 query columns for each of the two softmax warps of a lane quarter; P^T, bf16, takes
+// the first 32 of each once they are read, dS^T the others), dV 256, dK 384
 constexpr int HALF = BLK / 2;                    // streamed rows per softmax warp, in both CTA kinds
 constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
 
@@ -196,12 +195,15 @@ struct SplitMaps {
   int rows;     // 0 = unused
 };
 
-// One CTA of the dK/dV grid (flash_bwd_pair_kernel below runs it).  Its period is a chain - S^T, exponentials, dV and the next S^T -
-// with the tensor pipe idle under the exponentials, so what counts is what the softmax warps do besides them: each writes P^T
+// One CTA of the dK/dV grid (flash_bwd_pair_kernel below runs it).  Its period was a chain - S^T, exponentials, dV and the next S^T -
+// with the tensor pipe idle under the exponentials, so what counted is what the softmax warps do besides them: each writes P^T
 // and dS^T over columns that only it has read, where the two warps of a lane quarter met at a barrier twice a block; blocks
 // off the diagonal run without the masks; TMEM loads come in two pieces, the second under the arithmetic of the first; a
 // warp arrives once, not 32 times.  The same in the dQ CTAs.  Backward, us: 8192 tokens x 32 heads 1682 -> 1570, 32768 x 4 2933 ->
 // 2712, 12288 x 32 on 8 3400 -> 3179, 4096 on 8192 keys x 32 on 8 1540 -> 1404, 2048 x 32 173 -> 158.
+// Then P^T moved over dP^T: S^T(i+1) may follow as soon as the warps hold S^T(i), not P^T(i) and dV(i), so the chain is S^T,
+// exponentials, dS, dP^T without a wait for dV in it.  Backward, us: 8192 x 32 1545 -> 1525, 32768 x 4 2673 -> 2571, 12288 x 32 on 8
+// 3115 -> 3016, 2048 x 32 157 -> 155; the period of a block 2869 -> 2690 cycles, of which the pipe works 2100.
 // Measured and not kept: this kernel in two independent 64-query halves, as the dQ CTAs are (1793 us at 8192 x 32: an instruction 64
 // columns wide with both operands in shared memory takes 48 cycles for its reads, not 32); sixteen softmax warps with 32
 // columns each in both (1588); the five-product kernel below with sixteen (1906 -> 1746, 3520 -> 3155 at 32768 x 4).
@@ -247,8 +249,8 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
       mbar_init(&bars->d_full[s], 1); mbar_init(&bars->d_empty[s], 1);
     }
     mbar_init(&bars->s_full, 1);
+    mbar_init(&bars->s_free, 8);                  // one arrival per softmax warp
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->p_full, 8);                  // one arrival per softmax warp
     mbar_init(&bars->ds_full, 8);
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->drain, 1);
@@ -345,31 +347,29 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
       // not kept: two issuing warps on two schedulers (warp 1: dV(it), S^T(it+1); warp 2: dK(it), dP^T(it+1); the same
       // split in the dQ kernel): with two queues the pipe interleaves their instructions and every product completes
       // later, 688 / 800 TFLOP/s.
-      // The tensor pipe executes in issue order, so S^T(it+1) may overwrite P^T(it) once dV(it) has been issued,
-      // and dP^T(it+1) may overwrite dS^T(it) once dK(it) has.  While the softmax warps turn dP^T(it) into
-      // dS^T(it) the pipe runs dV(it) and S^T(it+1); while they turn S^T(it+1) into P^T(it+1) it runs dK(it)
-      // and dP^T(it+1).
+      // S^T(it+1) needs only that the softmax warps hold S^T(it) in registers: P^T goes over dP^T, not over S^T, so the exponentials
+      // of a block run while the pipe still works on the block before.  The pipe executes in issue order, so dP^T(it+1) may
+      // overwrite P^T(it) and dS^T(it) once dV(it) and dK(it) have been issued.
       for (int it = 0; it < total && ok; ++it) {
         const int stage = it % STAGES;
         const uint32_t par = it & 1;
-        const uint32_t acc0 = it > 0 ? 1u : 0u;
         if (trace && it < 48) dbg[it * 8 + 0] = clock64();
-        if (!mbar_wait(&bars->p_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-        if (trace && it < 48) dbg[it * 8 + 1] = clock64();                 // P^T(it) seen
+        if (it + 1 < total) {
+          if (!mbar_wait(&bars->s_free, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+          if (!issue_s(it + 1)) { ok = false; break; }
+        }
+        if (!mbar_wait(&bars->ds_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        if (trace && it < 48) dbg[it * 8 + 1] = clock64();                 // P^T(it) and dS^T(it) seen
         tc_fence_after();
-        const uint64_t dmn = desc_advance(d_mn0, stage * BLK_BYTES);
+        const uint64_t dmn = desc_advance(d_mn0, stage * BLK_BYTES), qmn = desc_advance(q_mn0, stage * BLK_BYTES);
+#pragma unroll
+        for (int kk = 0; kk < BLK / 16; ++kk)      // dK += dS^T Q: first, so that the fetch of the Q block after next starts
+          if (leader) umma_ts(tmem + COL_DK, tmem + COL_DPT + (kk >> 2) * HALF + 32 + (kk & 3) * 8, desc_advance(qmn, kk * 2048), IDESC_ACC, (it | kk) > 0 ? 1u : 0u);
+        if (leader) umma_commit(&bars->q_empty[stage]);
 #pragma unroll
         for (int kk = 0; kk < BLK / 16; ++kk)      // dV += P^T dO
-          if (leader) umma_ts(tmem + COL_DV, tmem + COL_ST + (kk >> 2) * HALF + (kk & 3) * 8, desc_advance(dmn, kk * 2048), IDESC_ACC, kk > 0 ? 1u : acc0);
+          if (leader) umma_ts(tmem + COL_DV, tmem + COL_DPT + (kk >> 2) * HALF + (kk & 3) * 8, desc_advance(dmn, kk * 2048), IDESC_ACC, (it | kk) > 0 ? 1u : 0u);
         if (leader) umma_commit(&bars->d_empty[stage]);
-        if (it + 1 < total && !issue_s(it + 1)) { ok = false; break; }
-        if (!mbar_wait(&bars->ds_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-        tc_fence_after();
-        const uint64_t qmn = desc_advance(q_mn0, stage * BLK_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < BLK / 16; ++kk)      // dK += dS^T Q
-          if (leader) umma_ts(tmem + COL_DK, tmem + COL_DPT + (kk >> 2) * HALF + (kk & 3) * 8, desc_advance(qmn, kk * 2048), IDESC_ACC, kk > 0 ? 1u : acc0);
-        if (leader) umma_commit(&bars->q_empty[stage]);
         if (it + 1 < total && !issue_dp(it + 1)) { ok = false; break; }
       }
       if (ok) {
@@ -394,7 +394,7 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
       const uint32_t par = it & 1;
       const int qrow0 = (i0 + (u0 + it) % per_head) * BLK + hf * 64;
       const bool strace = dbg != nullptr && cta == 0 && threadIdx.x == 128 && it < 48;
-      // ---- part 1: S^T -> P^T
+      // ---- part 1: S^T -> P^T, in registers
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
       if (strace) dbg[it * 8 + 2] = clock64();                             // S^T(it) complete
       if (!ok) break;
@@ -404,68 +404,63 @@ __device__ __forceinline__ void dkdv_cta(const int cta, const CUtensorMap& tmQ, 
       tmem_ld_wait32(sv);
       tmem_ld_32x32(tmem + COL_ST + hf * HALF + 32 + lane_off, sv + 32);   // on its way while the first 32 are worked on
       if (strace) dbg[it * 8 + 3] = clock64();                             // S^T in registers
-      {
-        uint32_t pp[32];
-        auto exponentials = [&](auto masked) {
+      uint32_t pp[32];
+      auto exponentials = [&](auto masked) {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            if (c == 16) tmem_ld_wait32(sv + 32);
-            // the accumulator already holds s - lse / scale: x = that * scale * log2(e), two query columns at once
-            const uint64_t x2 = mul2(pk2u(sv[2 * c], sv[2 * c + 1]), sl2_2);
-            float p0, p1;
-            upk2(x2, p0, p1);
-            p0 = exp2_mufu(p0);
-            p1 = exp2_mufu(p1);
-            if constexpr (decltype(masked)::value) {
-              if (qrow0 + 2 * c < kv0 + r) p0 = 0.f;
-              if (qrow0 + 2 * c + 1 < kv0 + r) p1 = 0.f;
-            }
-            sv[2 * c] = __float_as_uint(p0);
-            sv[2 * c + 1] = __float_as_uint(p1);
-            pp[c] = pack_bf16(p0, p1);
+        for (int c = 0; c < 32; ++c) {
+          if (c == 16) {
+            tmem_ld_wait32(sv + 32);
+            tc_fence_before();
+            mbar_arrive_warp(&bars->s_free, lane);            // S^T(it) is in registers
           }
-        };
-        // blocks without masked (q, kv) pairs run an instance without the masks
-        if (causal && qrow0 < kv0 + BIG) exponentials(std::true_type()); else exponentials(std::false_type());
-        if (dbg != nullptr) {   // tracing only: pin every packed value before the stamp
-          asm volatile("" ::"r"(pp[0]), "r"(pp[1]), "r"(pp[2]), "r"(pp[3]), "r"(pp[4]), "r"(pp[5]), "r"(pp[6]), "r"(pp[7]), "r"(pp[8]), "r"(pp[9]), "r"(pp[10]), "r"(pp[11]), "r"(pp[12]), "r"(pp[13]), "r"(pp[14]), "r"(pp[15]));
-          asm volatile("" ::"r"(pp[16]), "r"(pp[17]), "r"(pp[18]), "r"(pp[19]), "r"(pp[20]), "r"(pp[21]), "r"(pp[22]), "r"(pp[23]), "r"(pp[24]), "r"(pp[25]), "r"(pp[26]), "r"(pp[27]), "r"(pp[28]), "r"(pp[29]), "r"(pp[30]), "r"(pp[31]));
+          // the accumulator already holds s - lse / scale: x = that * scale * log2(e), two query columns at once
+          const uint64_t x2 = mul2(pk2u(sv[2 * c], sv[2 * c + 1]), sl2_2);
+          float p0, p1;
+          upk2(x2, p0, p1);
+          p0 = exp2_mufu(p0);
+          p1 = exp2_mufu(p1);
+          if constexpr (decltype(masked)::value) {
+            if (qrow0 + 2 * c < kv0 + r) p0 = 0.f;
+            if (qrow0 + 2 * c + 1 < kv0 + r) p1 = 0.f;
+          }
+          sv[2 * c] = __float_as_uint(p0);
+          sv[2 * c + 1] = __float_as_uint(p1);
+          pp[c] = pack_bf16(p0, p1);
         }
-        if (strace) dbg[it * 8 + 4] = clock64();                           // P^T computed
-        // over the scores that this warp alone has read: no warp waits for another here
-        tmem_st_32x16(tmem + COL_ST + hf * HALF + lane_off, pp);
-        tmem_st_32x16(tmem + COL_ST + hf * HALF + 16 + lane_off, pp + 16);
-        tmem_st_wait();
-        if (strace) dbg[it * 8 + 5] = clock64();                           // P^T stored
-        tc_fence_before();
-        mbar_arrive_warp(&bars->p_full, lane);
-      }
-      // ---- part 2: dP^T -> dS^T = P^T * (dP^T - delta) * scale
+      };
+      // blocks without masked (q, kv) pairs run an instance without the masks
+      if (causal && qrow0 < kv0 + BIG) exponentials(std::true_type()); else exponentials(std::false_type());
+      if (strace) dbg[it * 8 + 4] = clock64();                             // P^T computed
+      // ---- part 2: dP^T -> dS^T = P^T * (dP^T - delta); both go over the columns of dP^T that this warp alone has read
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_full, par, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
+      if (strace) dbg[it * 8 + 5] = clock64();                             // dP^T(it) complete
       if (!ok) break;
       uint32_t dp[64];
       tc_fence_after();
       tmem_ld_32x32(tmem + COL_DPT + hf * HALF + lane_off, dp);
-      tmem_ld_wait32(dp);
       tmem_ld_32x32(tmem + COL_DPT + hf * HALF + 32 + lane_off, dp + 32);
+      tmem_ld_wait32(dp);
+      tmem_ld_wait32(dp + 32);
       if (strace) dbg[it * 8 + 6] = clock64();                             // dP^T in registers
-      {
-        uint32_t ds[32];
+      tmem_st_32x16(tmem + COL_DPT + hf * HALF + lane_off, pp);
+      tmem_st_32x16(tmem + COL_DPT + hf * HALF + 16 + lane_off, pp + 16);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          if (c == 16) tmem_ld_wait32(dp + 32);
+      for (int h = 0; h < 2; ++h) {
+        uint32_t ds[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
           // dS = P * (dP - delta), the accumulator already holding dP - delta; the softmax scale is applied once, to
           // dK, in the epilogue
+          const int e = 32 * h + 2 * c;
           float d0, d1;
-          upk2(mul2(pk2u(sv[2 * c], sv[2 * c + 1]), pk2u(dp[2 * c], dp[2 * c + 1])), d0, d1);
+          upk2(mul2(pk2u(sv[e], sv[e + 1]), pk2u(dp[e], dp[e + 1])), d0, d1);
           ds[c] = pack_bf16(d0, d1);
         }
-        tmem_st_32x16(tmem + COL_DPT + hf * HALF + lane_off, ds);
-        tmem_st_32x16(tmem + COL_DPT + hf * HALF + 16 + lane_off, ds + 16);
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive_warp(&bars->ds_full, lane);
+        tmem_st_32x16(tmem + COL_DPT + hf * HALF + 32 + 16 * h + lane_off, ds);
       }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive_warp(&bars->ds_full, lane);
       if (strace) dbg[it * 8 + 7] = clock64();
     }
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_done, 0, abort_flag, err, ODY_ERR_TIMEOUT_MISC));
@@ -566,8 +561,9 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
 }
 
 // (Staging dQ_blk in the dS^T tile and adding it with TMA reductions, cp.reduce.async.bulk.tensor, measured slower than
-// the per-thread vector reductions: 2.32 ms against 2.02 ms at T = 8192 x 32 heads.  Either way the L2 absorbs the
-// partial dQ at about 2.2 TB/s, which is what bounds this kernel.)
+// the per-thread vector reductions: 2.32 ms against 2.02 ms at T = 8192 x 32 heads.  What bounds this kernel is the chain of a
+// block, five products and two passes of the softmax warps one after another in one CTA's TMEM, not the reductions: alone, the
+// L2 absorbs fp32 reductions of either kind at 6.0 TB/s, and here they come at 2.2.)
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                        const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -1317,7 +1313,8 @@ extern "C" void ody_flash_bwd_set_trace(long long* buf) { g_bwd_trace = buf; }
 static int g_bwd_variant = 1;
 // 1 (default): the split pair (dK/dV CTAs and dQ CTAs in one launch: seven products per block pair, no atomics, bitwise
 // reproducible); 0: the fused dK/dV/dQ kernel (five products; dQ summed over KV tiles with fp32 reductions in no fixed
-// order - at present the reduction traffic, not the tensor core, bounds it, and the split pair is the faster one)
+// order - the chain of a block bounds it, not the tensor core, and the split pair is the faster one: 1545 us against 1906 at
+// 8192 tokens x 32 heads, 2673 against 3520 at 32768 x 4)
 extern "C" int ody_flash_bwd_set_variant(int v) {
   if (v < 0 || v > 1) return (int)cudaErrorInvalidValue;
   g_bwd_variant = v;
