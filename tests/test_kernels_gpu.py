@@ -790,3 +790,27 @@ def test_gemm_cluster_rope(lib, M, shares):
             lib.gemm_cluster(a, b, None, 0, False, None, None, bn, n)
     with pytest.raises(RuntimeError):
         lib.gemm_cluster(a[:, :64], b[:, :64], None, 0, False, None, None, 64, 2)   # one k-block, two shares
+
+
+@pytest.mark.parametrize("V", [8, 4096, 4104, 16392, 32768, 32776, 65544])
+def test_cross_entropy_at_the_edges_of_a_round(lib, V):
+    """A block takes 512 threads x 8 vectors x 8 columns of a row at a time: rows that end inside, at and behind a round, with
+    targets in each place of a vector and in the row's first and last.  fp32 sums of at most 65544 terms in some order err by
+    far less than 1e-5 of the sum; a gradient is rounded to bf16 once (half a step: 2^-9)."""
+    torch.manual_seed(V)
+    tg = torch.tensor([i for i in range(8)] + [V - 8 + i for i in range(8)] + [V // 2, -100], device="cuda")
+    x = _rand(len(tg), V, scale=4.0)
+    x[3, :] = 2.0                                        # equal logits
+    x[5, V - 1] = 60.0                                   # one that outweighs all others, in the last place
+    ref = x.double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(ref, tg, reduction="none", ignore_index=-100)
+    want.sum().backward()
+    one = torch.ones(1, device="cuda")
+    loss, lse = lib.ce_fwd(x, tg, -100)
+    a, b = x.clone(), x.clone()
+    lib.ce_bwd_(a, tg, lse, one, -100)
+    loss1 = lib.ce_grad_(b, tg, one, -100)
+    for got in (loss, loss1):
+        torch.testing.assert_close(got.double(), want.detach(), rtol=1e-5, atol=1e-5)
+    for got in (a, b):
+        torch.testing.assert_close(got.double(), ref.grad, rtol=2 ** -8, atol=1e-6)
