@@ -12,8 +12,8 @@
 //   * every MMA is a tcgen05.mma issued by ONE thread in program order: S_t = Q_t K^T (operands in shared
 //     memory) and O_t += P_t V (P_t read from TMEM).  TMEM holds S_A, S_B, O_A, O_B (4 x 128 fp32 columns);
 //     the bf16 probabilities P_t are written over the first 64 columns of S_t once its thread has S_t in
-//     registers - the in-order tensor pipe runs Q K^T of the next block only after P V has read them (announcing
-//     P in 32-key pieces so that P V could start early measured slower: four store waits instead of one);
+//     registers - the in-order tensor pipe runs Q K^T of the next block only after P V has read them.  P is announced in
+//     two halves of 64 keys, so that P V of the first runs under the exponentials of the second;
 //   * two softmax warpgroups, one thread per query row: 128 scores straight from TMEM, no exchange between
 //     threads, exp2 domain, lazy rescaling of O (the running maximum used for exponentiation only moves when
 //     it would grow by more than 2^8, so the O read-modify-write is rare) - and because that maximum is known
@@ -33,8 +33,7 @@
 
 // KS32: Q and K sit in shared memory as eight [128 rows x 32 B] slices (32-byte swizzle) instead of two
 // [128 rows x 128 B] halves (128-byte swizzle), so that each Q K^T instruction reads two contiguous 4 KB blocks.
-// (Moving part of the exponentials from the special-function unit to an FMA-pipe polynomial, or announcing P in four
-// pieces so that P V starts early, both measured slower than this form.)
+// (Moving part of the exponentials from the special-function unit to an FMA-pipe polynomial measured slower than this form.)
 
 // Development aid, compiled only with -DODY_ATTN_TRACE: SM-clock stamps of one CTA's first blocks, written to a buffer
 // given with ody_flash_fwd_set_trace ([64 blocks][16] int64: 0-4 softmax of tile A, 5-9 softmax of tile B, 10-13 MMA thread).
@@ -53,6 +52,12 @@ constexpr int CTA_ROWS = 2 * BM;             // two query tiles per CTA
 constexpr int TILE_BYTES = 128 * HD * 2;     // 32 KB: two 64-column halves of [128 rows x 128 B]
 constexpr int HALF_BYTES = TILE_BYTES / 2;
 constexpr int KV_STAGES = 2;
+// Pieces of 32 keys of P that are announced first.  A tile's period is a chain - scores, exponentials, P V, next scores, with about 1000
+// cycles from the last probability to the next score - so P V of these leaves it: 3460 -> 3120 cycles.  Forward, us: 8192 tokens x
+// 32 heads 489 -> 473, 32768 x 4 901 -> 863, 4096 on 8192 keys x 32 on 8 515 -> 493, 12288 x 32 1026 -> 987.  With three first (492
+// and 907), or with the scores of the next block's first 64 keys computed under the exponentials of this one's last (two buffers
+// that swap roles; 573 and 1060: a product of 64 columns takes 48 cycles, one of 128 takes 64), it is slower.
+constexpr int P_PIECES = 2;
 constexpr int SMEM_TILES = TILE_BYTES * (2 + 2 * KV_STAGES);
 constexpr int SMEM_TOTAL = SMEM_TILES + 512 + 1024;
 // Warp roles by warpgroup: 0 TMA producer, 1 MMA issuer, 2-3 idle | 4..7 softmax of tile A | 8..11 softmax of
@@ -77,7 +82,7 @@ struct Bars {
   uint64_t q_full[2];
   uint64_t k_full[KV_STAGES], k_empty[KV_STAGES];
   uint64_t v_full[KV_STAGES], v_empty[KV_STAGES];
-  uint64_t s_full[2], p_full[2], o_done[2];
+  uint64_t s_full[2], p_full[2], p_rest[2], pv_part[2], o_done[2];   // [tile]; p_full: the first P_PIECES pieces of P, p_rest: the others
   uint64_t drain;
   uint32_t tmem_base;
   int abort_flag;
@@ -142,6 +147,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     for (int t = 0; t < 2; ++t) {
       mbar_init(&bars->s_full[t], 1);
       mbar_init(&bars->p_full[t], 4);          // one arrival per warp
+      mbar_init(&bars->p_rest[t], 4);
+      mbar_init(&bars->pv_part[t], 1);
       mbar_init(&bars->o_done[t], 1);
     }
     mbar_init(&bars->drain, 1);
@@ -246,15 +253,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
           if (leader) umma_commit(&bars->s_full[t]);
         };
-        // O_t (+)= P_t V(j)
-        auto issue_pv = [&](int t, int j) {
+        // O_t (+)= P_t V(j), keys [16 k0, 16 k1)
+        auto issue_pv = [&](int t, int j, auto k0, auto k1) {
           const uint64_t v = desc_advance(vdesc0, (j & 1) * TILE_BYTES);
           const uint32_t pa = tmem + COL_S + t * BN;
           const uint32_t d = tmem + COL_O + t * HD;
-          if (leader) umma_ts(d, pa, v, IDESC_PV, j > 0 ? 1u : 0u);
 #pragma unroll
-          for (int kk = 1; kk < BN / 16; ++kk) if (leader) umma_ts(d, pa + kk * 8, desc_advance(v, kk * 2048), IDESC_PV, 1u);
+          for (int kk = decltype(k0)::value; kk < decltype(k1)::value; ++kk)
+            if (leader) umma_ts(d, pa + kk * 8, desc_advance(v, kk * 2048), IDESC_PV, kk > 0 || j > 0 ? 1u : 0u);
         };
+        using K0 = std::integral_constant<int, 0>;
+        using K1 = std::integral_constant<int, 2 * P_PIECES>;
+        using K2 = std::integral_constant<int, BN / 16>;
         ok = mbar_wait(&bars->q_full[0], 0, abort_flag, err, ODY_ERR_TIMEOUT_FULL) &&
              mbar_wait(&bars->k_full[0], 0, abort_flag, err, ODY_ERR_TIMEOUT_FULL);
         if (ok) {
@@ -284,7 +294,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
               have_v = true;
             }
             tc_fence_after();
-            issue_pv(t, j);
+            issue_pv(t, j, K0(), K1());
+            if (leader) umma_commit(&bars->pv_part[t]);
+            if (!mbar_wait(&bars->p_rest[t], j & 1, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+            tc_fence_after();
+            issue_pv(t, j, K1(), K2());
             if (j + 1 < nt) {
               if (!have_k1) {
                 if (!mbar_wait(&bars->k_full[s1], ph1, abort_flag, err, ODY_ERR_TIMEOUT_FULL)) { ok = false; break; }
@@ -366,16 +380,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       // One pass over the 128 scores: exponentials against the maximum in use (packed pairs, x = s * scale * log2(e) - m),
       // P back over S in four 32-column pieces, the row sum, and - on the side, off the dependent chain - the row maximum
-      // of THIS block.  The maximum in use only has to be within 2^8 of the true one, so the common case needs no
-      // separate maximum pass in front of the exponentials; a block that moves it further is redone (rare).
+      // of THIS half.  The maximum in use only has to be within 2^8 of the true one, so the common case needs no
+      // separate maximum pass in front of the exponentials; a half that moves it further is redone (rare).
       const uint64_t sl2_2 = pk2(sl2, sl2);
-      float rsum, rmax;
-      auto exp_pass = [&](auto loads) {
+      uint64_t rs2 = pk2(0.f, 0.f);
+      float rmax;
+      auto exp_pass = [&](auto g0, auto g1, auto loads) {
         const uint64_t nm_2 = pk2(-m_used, -m_used);
-        uint64_t rs2 = pk2(0.f, 0.f);
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
+        for (int g = decltype(g0)::value; g < decltype(g1)::value; ++g) {
           if constexpr (decltype(loads)::value) {
             tmem_ld_wait32(sv + 32 * g);
             if (g < 3) tmem_ld_32x32(col_s + 32 * (g + 1), sv + 32 * (g + 1));
@@ -396,10 +410,47 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
           tmem_st_32x16(col_s + g * 16, pk);
         }
-        float r0, r1;
-        upk2(rs2, r0, r1);
-        rsum = r0 + r1;
         rmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      };
+      using G0 = std::integral_constant<int, 0>;
+      using G1 = std::integral_constant<int, P_PIECES>;
+      using G2 = std::integral_constant<int, 4>;
+      // Pieces [g0, g1) against the maximum in use; when that moved by more than 2^8 for some row of this warp (rare): O, l and
+      // the sum so far are rescaled and these pieces are redone.
+      auto part = [&](auto g0, auto g1) -> bool {
+        const uint64_t before = rs2;
+        exp_pass(g0, g1, std::bool_constant<!MASKED>());
+        const float m_new = fmaxf(m_used, rmax * sl2);
+        const bool need = (m_new - m_used) > 8.f;
+        if (__any_sync(0xffffffffu, need)) {
+          // P V of block j-1 completed before S(j) was announced; of this block's the pipe may hold those of the first pieces,
+          // and P V of the pieces at hand waits for this thread
+          if constexpr (decltype(g0)::value > 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_part[t], j & 1, abort_flag, err, ODY_ERR_TIMEOUT_TMEM_FULL));
+            if (!ok) return false;
+            tc_fence_after();
+          }
+          const float alpha = need ? exp2_mufu(m_used - m_new) : 1.f;
+          if (need) m_used = m_new;
+          l *= alpha;
+          rs2 = mul2(before, pk2(alpha, alpha));
+#pragma unroll 1
+          for (int c = 0; c < 8; ++c) {
+            uint32_t o[16];
+            tmem_ld_32x16(col_o + c * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x16(col_o + c * 16, o);
+          }
+          exp_pass(g0, g1, std::false_type());
+        }
+        return true;
+      };
+      auto announce = [&](uint64_t* bar) {
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive_warp(bar, lane);
       };
       if constexpr (FIRST) {
         // first block: there is no maximum in use yet
@@ -415,34 +466,19 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // two infinities would make the row NaN although other blocks - or, of a split tile, other parts - are finite
         m_used = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2, -FLT_MAX);
         ODY_FWD_STAMP(tr, j, t * 5 + 3);
-        exp_pass(std::false_type());
+        exp_pass(G0(), G1(), std::false_type());
+        announce(&bars->p_full[t]);
+        exp_pass(G1(), G2(), std::false_type());
       } else {
         ODY_FWD_STAMP(tr, j, t * 5 + 3);
-        exp_pass(std::bool_constant<!MASKED>());
-        const float m_new = fmaxf(m_used, rmax * sl2);
-        const bool need = (m_new - m_used) > 8.f;
-        if (__any_sync(0xffffffffu, need)) {
-          // the running maximum moved by more than 2^8 for some row of this warp: rescale O and l, redo the block.
-          // P V of block j-1 completed before S(j) was announced and P V of block j waits for this thread, so O is ours.
-          const float alpha = need ? exp2_mufu(m_used - m_new) : 1.f;
-          if (need) m_used = m_new;
-          l *= alpha;
-#pragma unroll 1
-          for (int c = 0; c < 8; ++c) {
-            uint32_t o[16];
-            tmem_ld_32x16(col_o + c * 16, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x16(col_o + c * 16, o);
-          }
-          exp_pass(std::false_type());
-        }
+        if (!part(G0(), G1())) return false;
+        announce(&bars->p_full[t]);
+        if (!part(G1(), G2())) return false;
       }
-      l += rsum;
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive_warp(&bars->p_full[t], lane);
+      float r0, r1;
+      upk2(rs2, r0, r1);
+      l += r0 + r1;
+      announce(&bars->p_rest[t]);
       ODY_FWD_STAMP(tr, j, t * 5 + 4);
       return true;
     };

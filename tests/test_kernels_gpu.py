@@ -814,3 +814,25 @@ def test_cross_entropy_at_the_edges_of_a_round(lib, V):
         torch.testing.assert_close(got.double(), want.detach(), rtol=1e-5, atol=1e-5)
     for got in (a, b):
         torch.testing.assert_close(got.double(), ref.grad, rtol=2 ** -8, atol=1e-6)
+
+
+@pytest.mark.parametrize("at", [0, 63, 64, 127])
+@pytest.mark.parametrize("Tk", [512, 449])
+def test_attention_fwd_rescale_in_either_half_of_a_block(lib, at, Tk):
+    """P of a block is announced in two halves, and the maximum in use may move in either: one key a block (first and last of a
+    half) outweighs all keys before it by far more than 2^8 for the even rows, for the odd ones it weighs nothing.  Bounds as
+    for the other forward tests: bf16 output, fp32 statistics."""
+    from odysseus_transformer_b200.ops import torch_ref as R
+    torch.manual_seed(at + Tk)
+    H = 2
+    q, k, v = _rand(Tk, H, 128).abs(), _rand(Tk, H, 128, scale=0.05).abs(), _rand(Tk, H, 128)
+    q[1::2] *= -1
+    for b, j in enumerate(range(at, Tk, 128)):
+        k[j] = _rand(H, 128).abs() * 3.0 * (b + 1)
+    scale = 1.0 / math.sqrt(128)
+    for causal in (False, True):
+        o, lse = lib.attn_fwd(q, k, v, causal, scale)
+        _check_status(lib)
+        orf, lser = R.attn_fwd(q, k, v, causal, scale)
+        torch.testing.assert_close(o.float(), orf.float(), rtol=2e-2, atol=2e-2)
+        torch.testing.assert_close(lse, lser, rtol=1e-3, atol=2e-2)
