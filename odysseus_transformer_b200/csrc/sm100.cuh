@@ -138,6 +138,12 @@ __device__ __forceinline__ float exp2_mufu(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// The same, in program order among its kind
+__device__ __forceinline__ float exp2_in_order(float x) {
+  float y;
+  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // Packed fp32 pairs (sm_100 executes add / mul / fma on two floats per instruction): the softmax warps are bound
 // by instruction issue, so pairing halves the cost of their elementwise arithmetic.
 __device__ __forceinline__ uint64_t pk2(float a, float b) {
