@@ -443,7 +443,7 @@ extern "C" int ody_gemm_resolve_epilogue(const OdyEpilogue* epi, const void* C, 
 // others in a long chain (512 x 1024 from K = 32000, the gradient of a small model's last hidden state: 16 tiles of 500
 // k-blocks).  Estimates in us: 0.3 per 64-deep k-block of a 128 x 256 tile, operands at 6 TB/s, and for a split one
 // more launch and its partials written and read in the L2; a split has to promise a sixth.  That product
-// 158 -> 52 us with its sum, 128 x 1024 from K = 2816 25.3 -> 21.3.
+// 158 -> 52 us with its sum.  Products that fit one wave of the cluster kernel with a shorter K go there (ody_gemm_cluster_plan).
 static int gemm_splits(int M, int N, int K) {
   const int sms = 148;
   if (g_gemm_variant != 0 || (N % 8)) return 1;
