@@ -116,7 +116,8 @@ class DecoderLayer(nn.Module):
         if 2 * x.shape[0] * (3 * x.shape[1] + w[0].shape[0] + w[1].shape[1] + w[2].shape[0] + w[3].shape[1]) > _ONE_NODE_BYTES:
             return None
         weights = (self.input_layernorm, w[0], w[1], self.post_attention_layernorm, w[2], w[3])
-        if torch.is_grad_enabled() and not all(t.requires_grad for t in weights):
+        # a gradient per weight: one that fills two places has to be summed, which the blocks' nodes do one after the other
+        if torch.is_grad_enabled() and (not all(t.requires_grad for t in weights) or len(set(map(id, weights))) < len(weights)):
             return None
         return x, cos, sin, getattr(a, heads[0]), getattr(a, heads[1]), self.eps, 1.0 / math.sqrt(a.head_dim), weights
 

@@ -444,6 +444,8 @@ class _DecoderLayer(Function):
     @staticmethod
     def forward(ctx, x, cos, sin, hq, hkv, eps, scale, *weights):
         keep = any(ctx.needs_input_grad)
+        if keep and len(set(map(id, weights))) < len(weights):
+            raise ValueError("decoder_layer: a weight that fills two places has one gradient, which the backward would write twice")
         y, kept = native.lib().decoder_layer_fwd(x, weights, cos, sin, hq, hkv, eps, scale, keep)
         if keep:
             ctx.save_for_backward(x, cos, sin, kept, *weights)
@@ -471,7 +473,8 @@ class _DecoderLayer(Function):
 
 
 def decoder_layer(x, cos, sin, hq: int, hkv: int, eps: float, scale: float, weights):
-    """``weights``: input norm, q|k|v, output projection, post-attention norm, gate|up and down, all on this GPU."""
+    """``weights``: input norm, q|k|v, output projection, post-attention norm, gate|up and down, all on this GPU; where
+    gradients are wanted, six different tensors."""
     return call(_DecoderLayer, x, cos, sin, hq, hkv, eps, scale, *weights)
 
 

@@ -274,3 +274,24 @@ def test_decoder_layer_node_adds_and_returns_gradients(lib):
         F.decoder_layer(x, cos[:-1], sin[:-1], hq, hkv, 1e-5, 0.1, ws)
     with pytest.raises(RuntimeError):
         F.decoder_layer(x, cos, sin, hq, hkv, 1e-5, 0.1, [*ws[:5], ws[5][:, :-8]])
+
+
+def test_decoder_layer_with_shared_norm_weight(lib):
+    """One weight for both norms of a layer gets the sum of both gradients, in ``main_grad``: what two copies of it get, added."""
+    from odysseus_transformer_b200.config import get_model_config
+    from odysseus_transformer_b200.mesh import ParallelContext, set_context
+    from odysseus_transformer_b200.train import Trainer
+    ctx = ParallelContext(device=torch.device("cuda", 0), backend="fused")
+    set_context(ctx)
+    cfg = get_model_config("small")
+    tr = Trainer(cfg, "odysseus", ctx, 300, lr=0.0, seed=3)
+    batch = torch.randint(cfg.vocab_size, (1, 301), generator=torch.Generator().manual_seed(1)).pin_memory()
+    layer = tr.model.layers[0]
+    first, second = layer.input_layernorm, layer.post_attention_layernorm
+    tr.train_step(batch)
+    want = first.main_grad.float() + second.main_grad.float()
+    layer.post_attention_layernorm = first
+    tr.train_step(batch)
+    _check_status(lib)
+    # the contributions and their sum are each rounded to bf16 (2^-9 of them) on either side
+    assert ((first.main_grad.float() - want).norm() / want.norm()).item() < 2.0 ** -7

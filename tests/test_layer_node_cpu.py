@@ -70,6 +70,24 @@ def test_watched_or_changed_layers_keep_their_path(layer, monkeypatch):
         assert _node(layer) is not None
 
 
+def test_layers_with_shared_weights_keep_their_path(layer):
+    """Two contributions to one gradient: the layer's backward writes each weight's gradient once, the blocks' nodes add them."""
+    own = layer.post_attention_layernorm
+    layer.post_attention_layernorm = layer.input_layernorm
+    assert _node(layer) is None
+    with torch.no_grad():
+        assert _node(layer) is not None
+    layer.post_attention_layernorm = own
+    assert _node(layer) is not None
+    weight = torch.nn.Parameter(torch.empty(512, 512, dtype=torch.bfloat16))
+    layer.self_attn.o_proj.weight = layer.mlp.down_proj.weight = weight          # as for an MLP as wide as the model
+    assert _node(layer) is None
+    cos, sin = F.rope_tables(torch.arange(TOKENS), 128, 10000.0)
+    norm = layer.input_layernorm
+    with pytest.raises(ValueError, match="two places"):
+        F.decoder_layer(torch.empty(TOKENS, 512), cos, sin, 4, 2, 1e-5, 0.1, (norm, own.new_empty(1), own.new_empty(2), norm, own, own))
+
+
 def test_other_calls_keep_their_path(layer):
     assert _node(layer, dtype=torch.float32) is None
     assert _node(layer, tokens=0) is None
