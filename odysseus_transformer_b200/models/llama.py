@@ -121,16 +121,29 @@ class DecoderLayer(nn.Module):
             return None
         return x, cos, sin, getattr(a, heads[0]), getattr(a, heads[1]), self.eps, 1.0 / math.sqrt(a.head_dim), weights
 
-    def forward(self, x, delta, cos, sin):
+    def forward(self, x, delta, cos, sin, route: Optional[list] = None):
         """(x, delta): residual stream and the not-yet-added output of the previous block (None when that block
-        added it itself)."""
-        if F.epilogue_fusion("residual"):
-            node = self._one_node(x, cos, sin) if delta is None else None
+        added it itself).
+
+        ``route``: an empty list from whoever runs the layer under a checkpoint.  The first run notes in it which way it took; the
+        recomputation takes the same, whatever has changed since (a profiler, hooks, free memory), as it must save the same tensors."""
+        if route:
+            if route[0] is not None:
+                return F.decoder_layer(x, cos, sin, *route[0]), None
+        elif delta is None and F.epilogue_fusion("residual"):
+            node = self._one_node(x, cos, sin)
             if node is not None:
                 try:
-                    return F.decoder_layer(*node), None
+                    y = F.decoder_layer(*node)
                 except torch.OutOfMemoryError:      # the blocks' own calls need less at a time
                     pass
+                else:
+                    if route is not None:
+                        route.append(node[3:])
+                    return y, None
+        if route == []:
+            route.append(None)
+        if F.epilogue_fusion("residual"):
             # each block's output projection adds the residual stream in its own epilogue; the norms only normalise
             if delta is None:
                 x, h = F.rmsnorm_keep(x, self.input_layernorm, self.eps)
@@ -146,6 +159,9 @@ class DecoderLayer(nn.Module):
         a = self.self_attn(h, cos, sin)
         x, h = F.add_rmsnorm(x, a, self.post_attention_layernorm, self.eps)
         return x, self.mlp(h)
+
+
+_LAYER_FORWARD = DecoderLayer.forward
 
 
 class LlamaForCausalLM(nn.Module):
@@ -200,7 +216,9 @@ class LlamaForCausalLM(nn.Module):
         for layer in self.layers:
             if self.gradient_checkpointing and torch.is_grad_enabled():
                 from torch.utils.checkpoint import checkpoint
-                x, delta = checkpoint(layer, x, delta, cos, sin, use_reentrant=False)
+                # a layer that was replaced, wrapped or given another forward takes the four arguments it knows
+                route = {"route": []} if getattr(layer.forward, "__func__", None) is _LAYER_FORWARD else {}
+                x, delta = checkpoint(layer, x, delta, cos, sin, use_reentrant=False, **route)
             else:
                 x, delta = layer(x, delta, cos, sin)
         if delta is None:

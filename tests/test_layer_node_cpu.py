@@ -88,6 +88,94 @@ def test_layers_with_shared_weights_keep_their_path(layer):
         F.decoder_layer(torch.empty(TOKENS, 512), cos, sin, 4, 2, 1e-5, 0.1, (norm, own.new_empty(1), own.new_empty(2), norm, own, own))
 
 
+class _Node(torch.autograd.Function):
+    """Stands in for the layer's node on the CPU: the same tensors saved, gradients of ones."""
+
+    @staticmethod
+    def forward(ctx, x, cos, sin, hq, hkv, eps, scale, *weights):
+        ctx.save_for_backward(x, cos, sin, torch.zeros(64, dtype=torch.uint8), *weights)
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, _, _, _, *weights = ctx.saved_tensors
+        return (dy, None, None, None, None, None, None, *[torch.ones_like(w) for w in weights])
+
+
+@pytest.fixture
+def model(monkeypatch):
+    """Two checkpointed layers on the CPU that may run as one node; ``calls`` has an entry for each that did."""
+    from types import SimpleNamespace
+    monkeypatch.setattr(llama, "native", SimpleNamespace(use_native=lambda t: True, has_native_attention_bwd=lambda: True))
+    calls = []
+
+    def node(*args):
+        calls.append(1)
+        return _Node.apply(*args[:-1], *args[-1])
+    monkeypatch.setattr(F, "decoder_layer", node)
+    ctx = ParallelContext(device=torch.device("cpu"), backend="fused")
+    set_context(ctx)
+    cfg = get_model_config("small-gqa").replace(hidden_size=512, num_attention_heads=4, num_key_value_heads=2, intermediate_size=96,
+                                                num_hidden_layers=2, vocab_size=64)
+    m = llama.LlamaForCausalLM(cfg, "odysseus", ctx, dtype=torch.bfloat16, device=torch.device("cpu"))
+    m.init_weights(0)
+    m.gradient_checkpointing_enable()
+    m.calls = calls
+    return m
+
+
+def _loss(m):
+    ids = torch.arange(TOKENS).unsqueeze(0)
+    return m(ids, ids, labels=ids)
+
+
+def _profile():
+    return torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU])
+
+
+def test_recomputation_takes_the_way_of_the_forward(model):
+    """A checkpoint wants the same tensors saved again; what decides between node and blocks may have changed by then."""
+    loss = _loss(model)
+    assert len(model.calls) == 2
+    with _profile():
+        loss.backward()
+    assert len(model.calls) == 4 and all(p.grad is not None for p in model.layers.parameters())
+    model.calls.clear()
+    with _profile():
+        loss = _loss(model)
+    loss.backward()
+    assert not model.calls
+    loss = _loss(model)
+    model.layers[1].mlp.register_forward_hook(lambda *a: None)
+    loss.backward()
+    assert len(model.calls) == 4
+
+
+def test_recomputation_after_memory_was_short(model, monkeypatch):
+    """The forward's fallback to the blocks holds for the recomputation; a recomputation that is short of memory says so."""
+    node = F.decoder_layer
+
+    def full(*args):
+        raise torch.OutOfMemoryError("no memory")
+    monkeypatch.setattr(F, "decoder_layer", full)
+    loss = _loss(model)
+    monkeypatch.setattr(F, "decoder_layer", node)
+    loss.backward()
+    assert not model.calls
+    loss = _loss(model)
+    monkeypatch.setattr(F, "decoder_layer", full)
+    with pytest.raises(torch.OutOfMemoryError):
+        loss.backward()
+
+
+def test_replaced_layers_get_four_arguments(model):
+    seen = []
+    forward = model.layers[0].forward
+    model.layers[0].forward = lambda x, delta, cos, sin: seen.append(1) or forward(x, delta, cos, sin)
+    _loss(model).backward()
+    assert len(seen) == 2
+
+
 def test_other_calls_keep_their_path(layer):
     assert _node(layer, dtype=torch.float32) is None
     assert _node(layer, tokens=0) is None
