@@ -97,9 +97,10 @@ class DecoderLayer(nn.Module):
         for p in (self.input_layernorm, self.post_attention_layernorm):
             p.grad_sync_group = ctx.world_group
 
-    def _one_node(self, x, cos, sin):
+    def _one_node(self, x, cos, sin, repeated=False):
         """Arguments of ``F.decoder_layer`` when the layer may run as one autograd node, else ``None``: one GPU, own kernels, few
-        enough tokens that the host's launches bound it, and nothing that wants to see the blocks' single calls."""
+        enough tokens that the host's launches bound it, and nothing that wants to see the blocks' single calls or the tensors that
+        they save.  ``repeated``: what sees those is a checkpoint whose recomputation takes the same way (``forward``'s ``route``)."""
         a, m = self.self_attn, self.mlp
         heads, names = _ATTENTION.get(type(a)), _MLP.get(type(m))
         if (heads is None or names is None or self.pctx.inner_size > 1 or self.pctx.ring_size > 1 or a.head_dim != 128
@@ -117,7 +118,8 @@ class DecoderLayer(nn.Module):
             return None
         weights = (self.input_layernorm, w[0], w[1], self.post_attention_layernorm, w[2], w[3])
         # a gradient per weight: one that fills two places has to be summed, which the blocks' nodes do one after the other
-        if torch.is_grad_enabled() and (not all(t.requires_grad for t in weights) or len(set(map(id, weights))) < len(weights)):
+        if torch.is_grad_enabled() and (not all(t.requires_grad for t in weights) or len(set(map(id, weights))) < len(weights)
+                                        or not repeated and F.saved_tensors_seen()):
             return None
         return x, cos, sin, getattr(a, heads[0]), getattr(a, heads[1]), self.eps, 1.0 / math.sqrt(a.head_dim), weights
 
@@ -131,7 +133,7 @@ class DecoderLayer(nn.Module):
             if route[0] is not None:
                 return F.decoder_layer(x, cos, sin, *route[0]), None
         elif delta is None and F.epilogue_fusion("residual"):
-            node = self._one_node(x, cos, sin)
+            node = self._one_node(x, cos, sin, route is not None)
             if node is not None:
                 try:
                     y = F.decoder_layer(*node)

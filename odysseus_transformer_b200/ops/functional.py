@@ -43,6 +43,11 @@ def plain_call() -> bool:
                 or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or _profiler_enabled())
 
 
+def saved_tensors_seen() -> bool:
+    """Whether hooks see the tensors that are saved for backward now (a checkpoint, an offload to the host, a user's own)."""
+    return torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
+
+
 def call(fn, *args):
     """``fn.apply(*args)``, without autograd's wrapping when gradients are off: evaluation of a short prompt is bound by the
     host, and the wrapping was a third of a call's time there (logits of 128 tokens, two layers).  Whatever else looks at

@@ -88,6 +88,15 @@ def test_layers_with_shared_weights_keep_their_path(layer):
         F.decoder_layer(torch.empty(TOKENS, 512), cos, sin, 4, 2, 1e-5, 0.1, (norm, own.new_empty(1), own.new_empty(2), norm, own, own))
 
 
+def test_saved_tensor_hooks_see_the_blocks_tensors(layer):
+    """A hook that stores, counts or converts what is saved gets the blocks' tensors, not the node's one buffer of bytes."""
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t):
+        assert _node(layer) is None
+        with torch.no_grad():
+            assert _node(layer) is not None
+    assert _node(layer) is not None
+
+
 class _Node(torch.autograd.Function):
     """Stands in for the layer's node on the CPU: the same tensors saved, gradients of ones."""
 
@@ -166,6 +175,16 @@ def test_recomputation_after_memory_was_short(model, monkeypatch):
     monkeypatch.setattr(F, "decoder_layer", full)
     with pytest.raises(torch.OutOfMemoryError):
         loss.backward()
+
+
+def test_layers_checkpointed_by_their_user_keep_their_path(model):
+    """Here nothing tells the layer what its first run did."""
+    from torch.utils.checkpoint import checkpoint
+    cos, sin = F.rope_tables(torch.arange(TOKENS), 128, 10000.0)
+    y, _ = checkpoint(model.layers[0], torch.randn(TOKENS, 512).to(torch.bfloat16), None, cos, sin, use_reentrant=False)
+    with _profile():
+        y.sum().backward()
+    assert not model.calls and model.layers[0].input_layernorm.grad is not None
 
 
 def test_replaced_layers_get_four_arguments(model):
