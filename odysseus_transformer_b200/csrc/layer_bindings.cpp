@@ -58,8 +58,8 @@ struct Layer {
     I = w[W_GU].size(0) / 2;
     const int64_t rows[N_WEIGHTS] = {d, n, d, d, 2 * I, d}, cols[N_WEIGHTS] = {0, d, q, 0, d, I};
     for (int i = 0; i < N_WEIGHTS; ++i)
-      req(w[i].is_cuda() && w[i].get_device() == x.get_device() && w[i].scalar_type() == at::kBFloat16 && w[i].is_contiguous() &&
-          w[i].dim() == (cols[i] ? 2 : 1) && w[i].size(0) == rows[i] && (!cols[i] || w[i].size(1) == cols[i]),
+      req(w[i].is_cuda() && w[i].get_device() == x.get_device() && w[i].scalar_type() == at::kBFloat16 && w[i].dim() == (cols[i] ? 2 : 1) &&
+          rows_of(w[i]) && w[i].size(0) == rows[i] && (!cols[i] || w[i].size(1) == cols[i]),
           "a weight has the wrong shape, type, layout or device");
     for (const at::Tensor* t : {&cos_, &sin_})
       req(t->is_cuda() && t->get_device() == x.get_device() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->dim() == 2 &&
@@ -75,18 +75,21 @@ struct Layer {
     err = ody_status_ptr(x);
   }
 
+  // a norm's weight is packed; a projection's rows are, and may lie apart (a slice of a wider matrix)
+  static bool rows_of(const at::Tensor& t) { return t.dim() == 2 ? t.stride(1) == 1 : t.is_contiguous(); }
+
   at::Tensor bytes(int64_t size) const { return at::empty({size}, x.options().dtype(at::kByte)); }
 
   static int64_t gemm_scratch(int64_t M, int64_t N, int64_t K, bool rope = false) {
     int bn, s;
     return ody_gemm_cluster_plan((int)M, (int)N, (int)K, rope, &bn, &s) ? 0 : ody_gemm_split_bytes((int)M, (int)N, (int)K);
   }
-  // C = A B in `layout`, all packed
-  void gemm(const void* A, const void* B, void* C, int64_t M, int64_t N, int64_t K, int layout, bool accumulate, const OdyEpilogue* epi,
-            const ody::OptionalScratch& ws) const {
+  // C = A B in `layout`, rows of B and C ldb and ldc apart, those of A packed
+  void gemm(const void* A, const void* B, void* C, int64_t M, int64_t N, int64_t K, int64_t ldb, int64_t ldc, int layout, bool accumulate,
+            const OdyEpilogue* epi, const ody::OptionalScratch& ws) const {
     const int64_t need = gemm_scratch(M, N, K, epi != nullptr && epi->rope_cos != nullptr);
     const bool split = need > 0 && ws.bytes >= need;
-    check(ody_gemm_bf16_ws(A, B, C, (int)M, (int)N, (int)K, layout == 2 ? M : K, layout == 0 ? K : N, N, layout, accumulate ? 1 : 0, epi,
+    check(ody_gemm_bf16_ws(A, B, C, (int)M, (int)N, (int)K, layout == 2 ? M : K, ldb, ldc, layout, accumulate ? 1 : 0, epi,
                            split ? ws.ptr() : nullptr, split ? ws.bytes : 0, err, st), "gemm");
     ody_count_launches(split ? 2 : 1);
   }
@@ -111,17 +114,20 @@ std::pair<at::Tensor, c10::optional<at::Tensor>> decoder_layer_fwd(const at::Ten
   res.residual_ld = d;
 
   check(ody_rmsnorm_fwd(x.data_ptr(), nullptr, w[W_IN].data_ptr(), nullptr, k + L.h1, (float*)(k + L.rstd1), T, (int)d, (float)eps, L.st), "norm");
-  L.gemm(k + L.h1, w[W_QKV].data_ptr(), k + L.qkv, T, L.n, d, 0, false, &rope, ws);
+  auto project = [&](const void* in, int i, void* dst, const OdyEpilogue* epi) {
+    L.gemm(in, w[i].data_ptr(), dst, T, w[i].size(0), w[i].size(1), w[i].stride(0), w[i].size(0), 0, false, epi, ws);
+  };
+  project(k + L.h1, W_QKV, k + L.qkv, &rope);
   char* q = k + L.qkv;
   check(ody_flash_fwd_parts(q, q + L.q * 2, q + (L.q + hkv * 128) * 2, k + L.o, (float*)(k + L.lse), (int)T, (int)T, (int)hq, (int)hkv, L.n, L.n,
                             L.n, L.q, 1, (float)scale, nullptr, nullptr, 0, 0, 0, parts.ptr(), parts.bytes, L.err, L.st), "attention");
   res.residual = x.data_ptr();
-  L.gemm(k + L.o, w[W_O].data_ptr(), k + L.x2, T, d, L.q, 0, false, &res, ws);
+  project(k + L.o, W_O, k + L.x2, &res);
   check(ody_rmsnorm_fwd(k + L.x2, nullptr, w[W_POST].data_ptr(), nullptr, k + L.h2, (float*)(k + L.rstd2), T, (int)d, (float)eps, L.st), "norm");
-  L.gemm(k + L.h2, w[W_GU].data_ptr(), k + L.gu, T, 2 * L.I, d, 0, false, nullptr, ws);
+  project(k + L.h2, W_GU, k + L.gu, nullptr);
   check(ody_swiglu_fwd(k + L.gu, k + L.act, T, L.I, L.st), "swiglu");
   res.residual = k + L.x2;
-  L.gemm(k + L.act, w[W_DOWN].data_ptr(), y.data_ptr(), T, d, L.I, 0, false, &res, ws);
+  project(k + L.act, W_DOWN, y.data_ptr(), &res);
   ody_count_launches(3 + (parts.bytes > 0 ? 2 : 1));
   if (!keep) return {y, c10::nullopt};
   return {y, kept};
@@ -142,16 +148,19 @@ Tensors decoder_layer_bwd(const at::Tensor& dy, const at::Tensor& x, const Tenso
   req(out.size() == N_WEIGHTS && accumulate.size() == N_WEIGHTS, "six destinations");
   Tensors r(1 + N_WEIGHTS);
   void* dw[N_WEIGHTS];
+  int64_t ld_dw[N_WEIGHTS];
   for (int i = 0; i < N_WEIGHTS; ++i) {
     const bool norm = i == W_IN || i == W_POST;
     if (out[i].has_value()) {
       const at::Tensor& t = out[i].value();
-      req(t.is_cuda() && t.get_device() == x.get_device() && t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.sizes() == w[i].sizes(),
+      req(t.is_cuda() && t.get_device() == x.get_device() && t.scalar_type() == at::kBFloat16 && t.sizes() == w[i].sizes() && Layer::rows_of(t),
           "a gradient's destination has the wrong shape, type, layout or device");
       dw[i] = t.data_ptr();
+      ld_dw[i] = t.stride(0);
     } else {
       r[1 + i] = at::empty(w[i].sizes(), norm ? x.options().dtype(at::kFloat) : x.options());
       dw[i] = r[1 + i].data_ptr();
+      ld_dw[i] = r[1 + i].stride(0);
     }
   }
   r[0] = at::empty_like(x);
@@ -166,9 +175,11 @@ Tensors decoder_layer_bwd(const at::Tensor& dy, const at::Tensor& x, const Tenso
                                           Layer::gemm_scratch(2 * L.I, d, T), Layer::gemm_scratch(T, L.q, d), Layer::gemm_scratch(d, L.q, T),
                                           Layer::gemm_scratch(T, d, L.n), Layer::gemm_scratch(L.n, d, T)}), x);
   const ody::OptionalScratch parts(ody_flash_bwd_split_bytes((int)T, (int)T, (int)hq, (int)hkv, 1), x);
-  auto dgrad = [&](const void* g, int i, void* dst) { L.gemm(g, w[i].data_ptr(), dst, T, w[i].size(1), w[i].size(0), 1, false, nullptr, ws); };
+  auto dgrad = [&](const void* g, int i, void* dst) {
+    L.gemm(g, w[i].data_ptr(), dst, T, w[i].size(1), w[i].size(0), w[i].stride(0), w[i].size(1), 1, false, nullptr, ws);
+  };
   auto wgrad = [&](const void* g, int i, const void* in) {
-    L.gemm(g, in, dw[i], w[i].size(0), w[i].size(1), T, 2, out[i].has_value() && accumulate[i], nullptr, ws);
+    L.gemm(g, in, dw[i], w[i].size(0), w[i].size(1), T, w[i].size(1), ld_dw[i], 2, out[i].has_value() && accumulate[i], nullptr, ws);
   };
   auto norm = [&](int i, const void* g, const void* in, const void* rstd, const void* ds, void* dst) {
     check(ody_rmsnorm_bwd_to(g, in, w[i].data_ptr(), (const float*)rstd, ds, dst, dw[i], out[i].has_value() ? 1 : 0, (float*)(s + o_norm), T,

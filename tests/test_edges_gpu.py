@@ -295,3 +295,35 @@ def test_decoder_layer_with_shared_norm_weight(lib):
     _check_status(lib)
     # the contributions and their sum are each rounded to bf16 (2^-9 of them) on either side
     assert ((first.main_grad.float() - want).norm() / want.norm()).item() < 2.0 ** -7
+
+
+def test_decoder_layer_node_takes_rows_that_lie_apart(lib):
+    """Projections, and where their gradients go, as slices of wider matrices, as the single products take them: the bits of packed
+    ones, written and added, and nothing beside the slices is touched."""
+    from odysseus_transformer_b200.ops import functional as F
+    torch.manual_seed(1)
+    T, d, hq, hkv, inter = 200, 256, 4, 2, 384
+    shapes = [(d,), ((hq + 2 * hkv) * 128, d), (d, hq * 128), (d,), (2 * inter, d), (d, inter)]
+    packed = [torch.nn.Parameter(_rand(*s, scale=0.05) + (1 if len(s) == 1 else 0)) for s in shapes]
+    wide = [_rand(s[0], s[1] + 40) if len(s) == 2 else None for s in shapes]
+    apart = [torch.nn.Parameter(p.detach().clone() if w is None else w[:, 8:8 + p.shape[1]].copy_(p.detach())) for p, w in zip(packed, wide)]
+    x, dy = _rand(T, d), _rand(T, d)
+    cos, sin = lib.rope_tables(torch.arange(T, device="cuda"), 128, 10000.0)
+    grads = [torch.full((*p.shape[:-1], p.shape[-1] + 24), 3.0, device="cuda", dtype=torch.bfloat16) for p in apart]
+    for p, g in zip(apart, grads):
+        p.main_grad = g[:, 16:16 + p.shape[1]] if p.dim() == 2 else g[:p.shape[0]]
+        p._grad_written = False
+    for p in packed:
+        p.main_grad, p._grad_written = torch.empty_like(p), False
+    for _ in range(2):                                       # written, then added to
+        out = []
+        for ws in (packed, apart):
+            xs = x.clone().requires_grad_(True)
+            y = F.decoder_layer(xs, cos, sin, hq, hkv, 1e-5, 128 ** -0.5, ws)
+            y.backward(dy)
+            out.append((y, xs.grad, *[w.main_grad.clone() for w in ws]))
+        _check_status(lib)
+        assert all(torch.equal(a, b) for a, b in zip(*out))
+    assert all((g[:, :16] == 3.0).all() and (g[:, 16 + p.shape[1]:] == 3.0).all() for p, g in zip(apart, grads) if p.dim() == 2)
+    with pytest.raises(RuntimeError):                        # columns that lie apart were never taken
+        F.decoder_layer(x, cos, sin, hq, hkv, 1e-5, 0.1, [*packed[:5], torch.nn.Parameter(_rand(inter, d).t())])
