@@ -105,6 +105,7 @@ class DecoderLayer(nn.Module):
         heads, names = _ATTENTION.get(type(a)), _MLP.get(type(m))
         if (heads is None or names is None or self.pctx.inner_size > 1 or self.pctx.ring_size > 1 or a.head_dim != 128
                 or not getattr(a, "pack_weight", True) or not native.use_native(x) or x.dim() != 2 or x.shape[0] == 0
+                or cos.shape[0] > x.shape[0]      # tables of more positions: the blocks take those they need, or refuse
                 or not F.epilogue_fusion("rope") or not native.has_native_attention_bwd() or not F.plain_call()
                 or not (_unwatched(a) and _unwatched(m))
                 or _module._global_forward_hooks or _module._global_forward_pre_hooks

@@ -327,3 +327,22 @@ def test_decoder_layer_node_takes_rows_that_lie_apart(lib):
     assert all((g[:, :16] == 3.0).all() and (g[:, 16 + p.shape[1]:] == 3.0).all() for p, g in zip(apart, grads) if p.dim() == 2)
     with pytest.raises(RuntimeError):                        # columns that lie apart were never taken
         F.decoder_layer(x, cos, sin, hq, hkv, 1e-5, 0.1, [*packed[:5], torch.nn.Parameter(_rand(inter, d).t())])
+
+
+@pytest.mark.parametrize("mode", ["ulysses", "ring", "dp"])
+def test_evaluation_with_rope_tables_of_more_positions(lib, mode):
+    """The sequence-parallel attention block takes the rows of its own tokens from longer tables; so does its layer."""
+    from odysseus_transformer_b200.config import get_model_config
+    from odysseus_transformer_b200.mesh import ParallelContext, set_context
+    from odysseus_transformer_b200.parallel.apply import build_model
+    ctx = ParallelContext(device=torch.device("cuda", 0), backend="fused")
+    set_context(ctx)
+    cfg = get_model_config("small")
+    layer = build_model(cfg, mode, ctx, dtype=torch.bfloat16, device=ctx.device, seed=0).layers[0]
+    cos, sin = lib.rope_tables(torch.arange(200, device="cuda"), cfg.head_dim, 10000.0)
+    x = _rand(130, cfg.hidden_size)
+    with torch.no_grad():
+        y, _ = layer(x, None, cos, sin)
+        want, _ = layer(x, None, cos[:130], sin[:130])
+    _check_status(lib)
+    assert torch.equal(y, want)

@@ -24,8 +24,8 @@ def layer(request, monkeypatch):
                               kw.get("zero3", True), kw.get("pack", True))
 
 
-def _node(layer, dtype=torch.bfloat16, tokens=TOKENS):
-    cos, sin = F.rope_tables(torch.arange(TOKENS), 128, 10000.0)
+def _node(layer, dtype=torch.bfloat16, tokens=TOKENS, positions=TOKENS):
+    cos, sin = F.rope_tables(torch.arange(positions), 128, 10000.0)
     return layer._one_node(torch.empty(tokens, 512, dtype=dtype), cos, sin)
 
 
@@ -198,6 +198,7 @@ def test_replaced_layers_get_four_arguments(model):
 def test_other_calls_keep_their_path(layer):
     assert _node(layer, dtype=torch.float32) is None
     assert _node(layer, tokens=0) is None
+    assert _node(layer, positions=TOKENS + 1) is None
     assert _node(layer, tokens=llama._ONE_NODE_BYTES // ROW) is not None
     assert _node(layer, tokens=llama._ONE_NODE_BYTES // ROW + 1) is None
     keep = F.fuse_epilogues()
