@@ -71,7 +71,7 @@ template <int LAYOUT, bool ROPE, bool SPLIT = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __nv_bfloat16* __restrict__ c_in, int M, int N, int K,
-                 int64_t ldc, int accumulate, int mn3d, const RopeEpi rp, int* __restrict__ err,
+                 int64_t ldc, int accumulate, int mn3d, RopeEpi rp, int* __restrict__ err,
                  float* __restrict__ part = nullptr, int splits = 1) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -112,7 +112,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  after_previous_kernel(c_in);
+  if constexpr (ROPE) after_previous_kernel(c_in, rp.cos, rp.sin); else after_previous_kernel(c_in);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -311,9 +311,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // C = sum over the shares of a split product, in order, then what the GEMM epilogue does: rotary embedding of the q / k heads,
 // plus what C accumulates onto or the residual, one rounding.  Eight columns per thread; bound by the partials' reads (L2).
 __global__ void __launch_bounds__(256) splitk_sum_kernel(const float* __restrict__ part, int splits, int M, int N,
-                                                         const __nv_bfloat16* c_in, int64_t ld_in, int accumulate, const RopeEpi rp,
+                                                         const __nv_bfloat16* c_in, int64_t ld_in, int accumulate, RopeEpi rp,
                                                          __nv_bfloat16* C, int64_t ldc) {
-  after_previous_kernel(part, c_in);
+  after_previous_kernel(part, c_in, rp.cos, rp.sin);
   const int vpr = N / 8;
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= (int64_t)M * vpr) return;

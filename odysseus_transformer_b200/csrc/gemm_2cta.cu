@@ -141,7 +141,7 @@ template <int LAYOUT, bool ROPE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmC, const __nv_bfloat16* __restrict__ c_in, int M, int N, int K,
-                  int64_t ldc, int accumulate, int mn3d, const RopeEpi rp, int* __restrict__ err) {
+                  int64_t ldc, int accumulate, int mn3d, RopeEpi rp, int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Bars* bars = (Bars*)(smem + SMEM_TILES);
@@ -182,7 +182,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   cluster_sync_all();          // both CTAs' barriers exist before anything may signal them from the other side
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  after_previous_kernel(c_in);
+  if constexpr (ROPE) after_previous_kernel(c_in, rp.cos, rp.sin); else after_previous_kernel(c_in);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (each CTA loads its own halves)

@@ -83,7 +83,7 @@ template <int LAYOUT, int BN, bool ROPE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __nv_bfloat16* c_in,
                     int64_t ld_in, __nv_bfloat16* C, int64_t ldc, int M, int N, int K, int splits, int accumulate, int mn3d,
-                    const RopeEpi rp, int* __restrict__ err) {
+                    RopeEpi rp, int* __restrict__ err) {
   static_assert(!ROPE || BN == 128, "a rotated head needs both of its halves");
   constexpr int ST = stages<BN>(), STAGE = stage_bytes<BN>(), ROW = row_bytes<BN>();
   constexpr bool A_MN = (LAYOUT == 2), B_MN = (LAYOUT != 0);
@@ -115,7 +115,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
-  after_previous_kernel(c_in);
+  if constexpr (ROPE) after_previous_kernel(c_in, rp.cos, rp.sin); else after_previous_kernel(c_in);
 
   bool ok = true;
   if (warp == 0) {

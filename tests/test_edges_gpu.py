@@ -346,3 +346,32 @@ def test_evaluation_with_rope_tables_of_more_positions(lib, mode):
         want, _ = layer(x, None, cos[:130], sin[:130])
     _check_status(lib)
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("kernel", ["one CTA", "pairs", "cluster", "split"])
+def test_rotation_right_behind_its_tables(lib, kernel):
+    """The rope tables' kernel is the direct predecessor of the product that rotates with them: the product's blocks are resident
+    before the tables are written.  The same bits as with the GPU waited for in between."""
+    M, N, K = {"one CTA": (300, 768, 512), "pairs": (600, 768, 512), "cluster": (300, 768, 512), "split": (1, 384, 32000)}[kernel]
+    torch.manual_seed(M + N)
+    a, b, big = _rand(M, K, scale=0.1), _rand(N, K, scale=0.1), _rand(8192, 8192)
+    pos = [torch.randint(0, 9999, (M,), device="cuda") for _ in range(8)]
+
+    def product(p, wait):
+        cos, sin = lib.rope_tables(p, 128, 10000.0)
+        if wait:
+            torch.cuda.synchronize()
+        rope = (cos, sin, 256, 384)
+        return lib.gemm_cluster(a, b, None, 0, False, rope, None, 128, 2) if kernel == "cluster" else lib.gemm(a, b, None, 0, False, rope, None)
+    try:
+        lib.gemm_set_variant({"one CTA": 1, "pairs": 2}.get(kernel, 0))
+        lib.reset_launch_count()
+        want = [product(p, True) for p in pos]
+        assert lib.launch_count() == 8 * (3 if kernel == "split" else 2)
+        for _ in range(4):                                   # about 3 ms of work, so that the calls below queue up behind it
+            lib.gemm(big, big, None, 0, False)
+        got = [product(p, False) for p in pos]
+    finally:
+        lib.gemm_set_variant(0)
+    _check_status(lib)
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
