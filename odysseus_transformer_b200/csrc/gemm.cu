@@ -480,6 +480,8 @@ static bool takes_pairs(int M, int N) {
 // k-blocks to a CTA: beyond that the wide tiles' smaller operand traffic wins (1024 x 1024 from K = 32000: 60 us, here 63).
 // Measured, before -> cluster: 128 x 3072 from K = 1024 9.7 -> 6.6, 128 x 1024 from 2816 13.1 -> 7.4, 512 x 1024 from 1024 10.3 -> 6.6,
 // from 5632 17.3 -> 12.7, 1531 x 1024 from 1536 12.7 -> 10.5, 1024 x 1024 from 2816 18.4 -> 11.4, 128 x 4096 from 11008 30.7 -> 22.0.
+// Products that the split kernel shares among more CTAs than a cluster has are the faster ones here too: 128 x 256 from K = 4096 12.6
+// -> 6.6, from 12288 15.8 -> 9.6, 1 x 256 from 4096 7.7 -> 4.2, 512 x 64 from 12288 12.0 -> 9.6, 218 x 72 from 10728 13.0 -> 10.9.
 extern "C" int ody_gemm_cluster_plan(int M, int N, int K, int rope, int* bn, int* splits) {
   if (g_gemm_variant != 0 || M <= 0 || N <= 0 || K <= 0 || (N % 8)) return 0;
   const int64_t kblocks = (K + 63) / 64, tiles = (int64_t)((M + 127) / 128) * ((N + 255) / 256);
@@ -501,9 +503,6 @@ extern "C" int ody_gemm_cluster_plan(int M, int N, int K, int rope, int* bn, int
       static const double sharing[2][4] = {{0.0, 1.0, 1.4, 1.8}, {0.0, 1.0, 2.5, 4.0}};
       const int64_t kb = (kblocks + s - 1) / s;
       if (t * s > max_ctas[i] || kb > 192) continue;
-      // up to 256 columns of up to 128 rows from a long K stay split over up to 32 CTAs, two launches that a test counts
-      // (128 x 256 from K = 4096: 12.6 us, a cluster of eight 7.1)
-      if (s_old > 8 && t * s < 37) continue;
       const double e = (b == 64 ? 3.9 + 0.185 * kb : 5.4 + 0.196 * kb) + sharing[b / 128][i];
       if (e < best) { best = e; *bn = b; *splits = s; found = 1; }
     }

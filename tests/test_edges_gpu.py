@@ -73,7 +73,8 @@ def test_launches_are_counted(lib):
         fn()
         return lib.launch_count()
     g = lambda m, n, k: (lambda a, b: count(lambda: lib.gemm(a, b, None, 0, False)))(_rand(m, k), _rand(n, k))   # noqa: E731
-    assert g(128, 256, 4096) == 2                        # split, sum of the shares
+    assert g(512, 1024, 32000) == 2                      # split, sum of the shares
+    assert g(128, 256, 4096) == 1                        # shared by the CTAs of a cluster
     assert g(2048, 4096, 1024) == 1
 
     def attention(Tq, Tk, H, Hkv, causal):

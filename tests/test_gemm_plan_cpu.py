@@ -46,6 +46,7 @@ def test_where_the_line_lies(plan):
     assert plan(128, 3072, 1024) and plan(512, 1024, 2816) and plan(2048, 1024, 5632)
     assert plan(8192, 4096, 4096) is None and plan(4096, 1024, 1024) is None          # more tiles than SMs
     assert plan(1024, 1024, 32000) is None                                             # K too long for narrow tiles
-    assert plan(128, 256, 4096) is None                                                # split over more CTAs than a cluster has
+    assert plan(128, 256, 4096) and plan(512, 64, 12288)      # also where a split would take more CTAs than a cluster has
+    assert plan(128, 256, 32000) is None                      # so long a K that 32 CTAs and a sum are expected to be as fast
     for bad in ((0, 8, 8), (8, 0, 8), (8, 8, 0), (128, 1020, 1024)):
         assert plan(*bad) is None
