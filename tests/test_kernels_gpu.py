@@ -603,15 +603,23 @@ def test_embedding_grad(lib, T, V, d):
     assert torch.equal(dw[k.view(-1) == 0], torch.zeros_like(dw[k.view(-1) == 0]))
 
 
-# Few output tiles and a long K (the split of csrc/gemm.cu): one tile, ragged edges, the smallest and largest number of shares
-SPLITK_SHAPES = [(128, 256, 2048), (512, 1024, 32000), (8, 8, 65536), (130, 264, 4104), (1, 4096, 11008), (2000, 72, 8200),
-                 (128, 1024, 2816)]
+# Few output tiles and a long K, as csrc/gemm.cu splits them: one tile, ragged edges over several tiles, the smallest and largest
+# number of shares.  The first of these share K in clusters (csrc/gemm_cluster.cu); K of the others is too long for those.
+SPLITK_SHAPES = [(128, 256, 2048), (130, 264, 4104), (1, 4096, 11008), (2000, 72, 8200), (128, 1024, 2816)]
+SPLIT_KERNEL_SHAPES = [(512, 1024, 32000), (8, 8, 65536), (130, 264, 65544), (1000, 72, 32008), (300, 520, 32776)]
+
+
+def _kernels(lib, call):
+    lib.reset_launch_count()
+    r = call()
+    return r, lib.launch_count()
 
 
 @pytest.mark.parametrize("layout", [0, 1, 2])
-@pytest.mark.parametrize("M,N,K", SPLITK_SHAPES)
+@pytest.mark.parametrize("M,N,K", SPLITK_SHAPES + SPLIT_KERNEL_SHAPES)
 def test_gemm_split_k(lib, splits, layout, M, N, K):
     """Against fp32 and against the unsplit kernel; accumulating onto C, with a residual, into a strided output."""
+    kernels = 2 if (M, N, K) in SPLIT_KERNEL_SHAPES else 1
     torch.manual_seed(M + N + K + layout)
     K = K // 8 * 8
     if layout == 2:
@@ -620,7 +628,8 @@ def test_gemm_split_k(lib, splits, layout, M, N, K):
     a = _rand(M, K) if layout != 2 else _rand(K, M)
     b = _rand(N, K) if layout == 0 else _rand(K, N)
     ref = (a.float() if layout != 2 else a.float().t()) @ (b.float().t() if layout == 0 else b.float())
-    c = lib.gemm(a, b, None, layout, False)
+    c, n = _kernels(lib, lambda: lib.gemm(a, b, None, layout, False))
+    assert n == kernels
     with _unsplit(lib):
         c1 = lib.gemm(a, b, None, layout, False)
     _check_status(lib)
@@ -638,17 +647,19 @@ def test_gemm_split_k(lib, splits, layout, M, N, K):
         assert ((y.float() - (ref + res.float())).norm() / (ref + res.float()).norm()).item() < 5e-3
 
 
-@pytest.mark.parametrize("M", [1, 128, 300])
-def test_gemm_split_k_rope(lib, splits, M):
-    """The rotary epilogue done by the summing kernel equals the one of the unsplit kernel up to the sum's rounding."""
+@pytest.mark.parametrize("M,K", [(1, 4096), (128, 4096), (300, 4096), (130, 65536), (300, 32768)])
+def test_gemm_split_k_rope(lib, splits, M, K):
+    """The rotary epilogue done by the summing kernel (of one row, and where K is too long for clusters) equals the one of the
+    unsplit kernel up to the sum's rounding."""
     from odysseus_transformer_b200.ops import torch_ref as R
     torch.manual_seed(M)
-    N, K = 768, 4096
+    N = 768
     assert splits.ody_gemm_split_bytes(M, N, K) > 0
     a, b = _rand(M, K), _rand(N, K)
     cos, sin = R.rope_tables(torch.randint(0, 9999, (M,), device="cuda"), 128, 10000.0)
     rope = (cos, sin, 256, 384)
-    y = lib.gemm(a, b, None, 0, False, rope, None)
+    y, n = _kernels(lib, lambda: lib.gemm(a, b, None, 0, False, rope, None))
+    assert n == (1 if M > 1 and K == 4096 else 2)
     with _unsplit(lib):
         y1 = lib.gemm(a, b, None, 0, False, rope, None)
     _check_status(lib)
