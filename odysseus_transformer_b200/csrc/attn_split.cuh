@@ -59,6 +59,7 @@ inline double split_cost_us(bool uniform, int64_t work, int top, int len, int ti
     t = even + (ctas > SPLIT_SMS ? 0.15 * longest : 0.0);
     if (t < longest) t = longest;
   }
+  // 4 us for the launch of the sum: measured when a kernel started only after the one before had ended
   return c == 1 ? t : t + 4.0 + ctas * part_bytes * 2.0 / 5.0e6;
 }
 

@@ -638,7 +638,8 @@ extern "C" int ody_flash_fwd_push(const void* q, const void* k, const void* v, v
   return ody_flash_fwd_ex(q, k, v, o, lse, Tq, Tk, H, Hkv, q_row, k_row, v_row, o_row, causal, scale, push, nullptr, 0, 0, 0, err, st);
 }
 
-// Plan of the forward grid when its streamed dimension may be split (attn_split.cuh): 1.9 us per pair of 128 x 128 blocks
+// Plan of the forward grid when its streamed dimension may be split (attn_split.cuh): 1.9 us per pair of 128 x 128 blocks.  That is
+// from before P was announced in two halves; the period of a pair is 3120 cycles since, 1.63 us at 1.92 GHz.
 static ody::SplitPlan fwd_plan(int Tq, int Tk, int H, int causal, ody::SplitUnits* u) {
   using namespace ody;
   using namespace ody::fwd;

@@ -443,7 +443,9 @@ extern "C" int ody_gemm_resolve_epilogue(const OdyEpilogue* epi, const void* C, 
 // others in a long chain (512 x 1024 from K = 32000, the gradient of a small model's last hidden state: 16 tiles of 500
 // k-blocks).  Estimates in us: 0.3 per 64-deep k-block of a 128 x 256 tile, operands at 6 TB/s, and for a split one
 // more launch and its partials written and read in the L2; a split has to promise a sixth.  That product
-// 158 -> 52 us with its sum.  Products that fit one wave of the cluster kernel with a shorter K go there (ody_gemm_cluster_plan).
+// 158 -> 52 us with its sum.  The estimate lacks the operands that every tile fetches again: it puts that product at 26 us (31.6
+// with the constants of ody_gemm_cluster_plan), so that for such a K it says which forms are near each other and no more.
+// Products that fit one wave of the cluster kernel with a shorter K go there (ody_gemm_cluster_plan).
 static int gemm_splits(int M, int N, int K) {
   const int sms = 148;
   if (g_gemm_variant != 0 || (N % 8)) return 1;
@@ -475,7 +477,8 @@ static bool takes_pairs(int M, int N) {
 // Tiles and shares of K for gemm_cluster.cu, or 0 where the kernels above are expected to be as fast.  Estimates in us from
 // back-to-back launches of 90 products: a fixed part, so much per 64-deep k-block of a CTA, and what sharing costs at the end.
 //   128 x 64 tiles 3.9 + 0.185 (two shares 1.0, four 1.4, eight 1.8 more), 128 x 128 5.4 + 0.196 (1.0, 2.5, 4.0)
-//   one-CTA kernel 4.5 + 0.27 a wave, pairs 6.8 + 0.24 a wave, split K 8.5 + 0.3 and its partials written and read
+//   one-CTA kernel 4.5 + 0.27 a wave, pairs 6.8 + 0.24 a wave, split K 8.5 + 0.3 and its partials written and read (too little for
+//   512 x 1024 from K = 32000: 31.6 us against 52, see gemm_splits)
 // At most one wave of CTAs (clusters leave SMs of a GPC unused: 128 CTAs in clusters of eight take two rounds), and at most 192
 // k-blocks to a CTA: beyond that the wide tiles' smaller operand traffic wins (1024 x 1024 from K = 32000: 60 us, here 63).
 // Measured, before -> cluster: 128 x 3072 from K = 1024 9.7 -> 6.6, 128 x 1024 from 2816 13.1 -> 7.4, 512 x 1024 from 1024 10.3 -> 6.6,

@@ -14,8 +14,9 @@ __device__ __forceinline__ void opaque_pointer(P& p) { asm volatile("" : "+l"(p)
 // resident while the kernel before it in the stream drains.  Waits until that kernel has finished and its writes are visible, then
 // lets the next kernel of the stream come in as SMs run empty.  (In this order: when a kernel starts, everything before its direct
 // predecessor is complete.)  What it saves is the gap between two kernels: a chain of products of 2048 x 1024 from K = 1024 took 11.9
-// us each, this way 10.7; of 128 x 1024 from 1024 9.2 and 8.6.  A launch that waits for another GPU is not started like this.  The pointers a kernel reads through are passed along so that no load of read-only data, which the
-// compiler may otherwise move across a fence, is formed before the wait.
+// us each, this way 10.7; of 128 x 1024 from 1024 9.2 and 8.6.  A launch that waits for another GPU is not started like this.
+// The pointers a kernel reads through, those inside its parameter structs among them, are passed along so that no load of read-only
+// data, which the compiler may otherwise move across a fence, is formed before the wait.  (What TMA loads fetch needs none.)
 template <class... P>
 __device__ __forceinline__ void after_previous_kernel(P&... read) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
